@@ -956,7 +956,6 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     host_mailbox mbox(lease.cache, nb_cap * 4 + (nb_cap + 1) * 8 + 1024);
     uint32_t *h_tsz_pin = mbox.take<uint32_t>(nb_cap);
     uint64_t *h_so = mbox.take<uint64_t>(nb_cap + 1);
-    unsigned long long *h_spill_p = mbox.take<unsigned long long>(1);
     // Queue counts: items, root items, conjunctions, screened, prefiltered,
     // then the 7 narrow-phase counters.
     unsigned long long *h_q = mbox.take<unsigned long long>(5 + 7);
@@ -1071,7 +1070,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     dbuf<int32_t> ropes(SL());
     dbuf<walk_node> walks(SL());
     dbuf<dev_status> d_st(SL());
-    dbuf<unsigned long long> visits(SL()); // broad-phase node visits of the call
+    dbuf<unsigned long long> visits(SL()); // broad-phase node visits of the batch
     dbuf<unsigned long long> ctr(SL()), rq_count(SL()), cq_count(SL());
     keys_a.alloc(uint64_t(nb_max) * N, st);
     vals_a.alloc(uint64_t(nb_max) * N, st);
@@ -1091,21 +1090,21 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     const uint64_t aux_step = bvh_aux_words(N, R.cap);
     aux.alloc(uint64_t(nb_max) * aux_step, st);
     counts.alloc(uint64_t(nb_max) * N, st);
-    dbuf<uint32_t> leaf_of(SL()), stage(SL());
-    dbuf<uint64_t> overflow(SL());
-    dbuf<unsigned long long> overflow_count(SL());
+    dbuf<uint32_t> leaf_of(SL()), longer(SL());
+    dbuf<unsigned long long> n_longer(SL());
     leaf_of.alloc(uint64_t(nb_max) * N, st);
-    stage.alloc(uint64_t(nb_max) * N * BROAD_STAGE_K, st);
-    overflow.alloc(uint64_t(nb_max) * N, st);
-    overflow_count.alloc(1, st);
-    // Partners beyond the staged ones; when more spill than this holds, the
-    // overflowing objects are walked again instead.
-    dbuf<ulonglong2> spill(SL());
-    dbuf<unsigned long long> spill_count(SL());
+    longer.alloc(uint64_t(nb_max) * N, st);
+    n_longer.alloc(1, st);
+    // The batch's pair queue: one pair per object and step to begin with
+    // (half of that on the 20,000-object day); a batch with more grows it and
+    // walks again, and later calls keep the larger block.
+    dbuf<uint2> qpair(SL());
+    dbuf<uint32_t> qrank(SL());
+    dbuf<unsigned long long> qcount(SL());
     dbuf<unsigned long long> walk_next(SL());
-    const uint64_t spill_cap = std::max<uint64_t>(1 << 16, uint64_t(nb_max) * N / 8);
-    spill.alloc(spill_cap, st);
-    spill_count.alloc(1, st);
+    qpair.alloc_queue(std::max<uint64_t>(1 << 16, uint64_t(nb_max) * N), st);
+    qrank.alloc_queue(std::max<uint64_t>(1 << 16, uint64_t(nb_max) * N), st);
+    qcount.alloc(1, st);
     walk_next.alloc(1, st);
     offs.alloc(uint64_t(nb_max) * N, st);
     block_sums.alloc((uint64_t(nb_max) * N + 1023) / 1024 + 1, st);
@@ -1120,7 +1119,6 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     cc_cur.alloc(nb_max + 1, st);
     CK(cudaMemsetAsync(d_st.p, 0, sizeof(dev_status), st));
     visits.alloc(1, st);
-    CK(cudaMemsetAsync(visits.p, 0, sizeof(unsigned long long), st));
 
     dbuf<root_item> rq(SL());
     dbuf<np_item> items(SL()), surv(SL()), cand(SL());
@@ -1233,23 +1231,34 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         uint64_t n_mbox = want_trees ? 2 : 1;
         if (!skip_cd) {
             CK(cudaEventRecord(ev[3].a, st));
-            launch_broad_half(R.srt_aabbs.p, R.trees.p, R.cap, ropes.p, walks.p, leaf_of.p, R.srt_idx.p, R.tree_size.p,
-                              d_ot.p, sf, nb, N, counts.p, stage.p, spill.p, spill_cap, spill_count.p, walk_next.p,
-                              broad_walk, visits.p, st);
-            launch_scan(counts.p, uint64_t(nb) * N, offs.p, block_sums.p, total.p, st);
-            launch_step_offsets(offs.p, N, nb, total.p, step_off.p, st);
-            mbox.start()
-                .add(h_so, static_cast<const uint64_t *>(step_off.p), nb + 1)
-                .add(h_spill_p, static_cast<const unsigned long long *>(spill_count.p), 1)
-                .launch(st);
-            ++n_mbox;
-            CK(cudaStreamSynchronize(st));
-            const unsigned long long h_spill = *h_spill_p;
+            uint64_t np_batch = 0;
+            for (bool again = true; again;) {
+                const uint64_t qcap = std::min(qpair.n, qrank.n);
+                CK(cudaMemsetAsync(visits.p, 0, sizeof(unsigned long long), st));
+                launch_broad_half(R.srt_aabbs.p, R.trees.p, R.cap, ropes.p, walks.p, leaf_of.p, R.srt_idx.p,
+                                  R.tree_size.p, d_ot.p, sf, nb, N, counts.p, qpair.p, qrank.p, qcap, qcount.p,
+                                  walk_next.p, broad_walk, visits.p, st);
+                launch_scan(counts.p, uint64_t(nb) * N, offs.p, block_sums.p, total.p, st);
+                launch_step_offsets(offs.p, N, nb, total.p, step_off.p, st);
+                mbox.start()
+                    .add(h_so, static_cast<const uint64_t *>(step_off.p), nb + 1)
+                    .add(h_visits, static_cast<const unsigned long long *>(visits.p), 1)
+                    .launch(st);
+                ++n_mbox;
+                n_broad_launches += 5;
+                CK(cudaStreamSynchronize(st));
+                np_batch = h_so[nb];
+                if (np_batch >= (1ull << 32)) throw std::runtime_error("too many broad-phase pairs in one batch");
+                again = np_batch > qcap;
+                if (again) {
+                    qpair.alloc_queue(np_batch + np_batch / 8, st);
+                    qrank.alloc_queue(np_batch + np_batch / 8, st);
+                }
+            }
+            R.broad_visits += *h_visits;
             tr.mark("broad-phase counts read", "steps " + std::to_string(s0) + "+" + std::to_string(nb));
             stream_trees();
             tr.dev_mark(bname + ": broad phase done", st);
-            const uint64_t np_batch = h_so[nb];
-            if (np_batch >= (1ull << 32)) throw std::runtime_error("too many broad-phase pairs in one batch");
             // The pair and conjunction lists of the call grow batch by batch;
             // each new block is sized for the whole call by extrapolating from
             // the steps screened so far (+15 %), so that a multi-batch call
@@ -1263,10 +1272,9 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             if (R.bp.n < R.n_bp + np_batch)
                 R.bp.grow(std::max(R.n_bp + np_batch, whole_call(R.n_bp + np_batch)), R.n_bp, st);
             uint2 *bp_batch = R.bp.p + R.n_bp;
-            launch_broad_copy(R.aabbs.p, R.trees.p, R.cap, ropes.p, R.srt_idx.p, d_ot.p, sf, nb, N, counts.p, offs.p,
-                              stage.p, bp_batch, overflow.p, overflow_count.p, spill.p, spill_count.p,
-                              h_spill <= spill_cap, st);
-            n_broad_launches = h_spill <= spill_cap ? 8 : 7;
+            launch_broad_lists(nb, N, counts.p, offs.p, qpair.p, qrank.p, np_batch, bp_batch, longer.p, n_longer.p,
+                               st);
+            if (np_batch) n_broad_launches += 3;
             CK(cudaEventRecord(ev[3].b, st));
             for (uint32_t b = 0; b < nb; ++b) {
                 R.bp_off[2 * (s0 + b)] = R.n_bp + h_so[b];
@@ -1396,7 +1404,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             t_bp = ev[3].ms();
         }
         // aabb (2 passes + global box) + morton + sort + bvh; broad half walk, 3 scan kernels,
-        // step offsets, copy + spill scatter + list sort (or the overflow walk),
+        // step offsets, scatter + list sorts,
         // items + narrow, roots (+ retry), 5 conj-order kernels.
         R.n_launches += 6 + n_mbox;
         if (!skip_cd) R.n_launches += n_broad_launches + n_narrow_launches + n_roots_launches + 5;
@@ -1421,12 +1429,6 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         }
     }
     for (int k = 0; k < 7; ++k) R.stage_ms[7] += R.stage_ms[k];
-    {
-        mbox.start().add(h_visits, static_cast<const unsigned long long *>(visits.p), 1).launch(st);
-        R.n_launches += 1;
-        CK(cudaStreamSynchronize(st));
-        R.broad_visits = *h_visits;
-    }
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamSynchronize(cs));
     tr.mark("call done");
