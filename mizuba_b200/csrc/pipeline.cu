@@ -2053,12 +2053,26 @@ int mzb_result_copy_trees(const mzb_result *r, void *dst)
         }
         if (tot == 0) return;
         // Trees live at a fixed per-step capacity: pack them on the device,
-        // then one copy to the caller.
+        // straight into the caller's memory when that is this device's (and
+        // aligned as the nodes' 16-byte moves need), else into a block that
+        // one copy takes to the caller.  On the 20,000-object day the block
+        // is 0.9 GB, written and read once more, and its allocation had the
+        // pool map memory when a polyjectory had taken its place.
         dbuf<uint64_t> d_off;
-        dbuf<bvh_node> packed;
         d_off.alloc(off.size(), 0);
-        packed.alloc(tot, 0);
         CK(cudaMemcpy(d_off.p, off.data(), off.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+        cudaPointerAttributes pa{};
+        const bool known = cudaPointerGetAttributes(&pa, dst) == cudaSuccess;
+        if (!known) cudaGetLastError();
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        if (known && pa.type == cudaMemoryTypeDevice && pa.device == dev && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+            launch_tree_gather(r->trees.p, r->cap, d_off.p, r->tree_size.p, r->n_run, static_cast<bvh_node *>(dst), 0);
+            CK(cudaGetLastError());
+            return;
+        }
+        dbuf<bvh_node> packed;
+        packed.alloc(tot, 0);
         launch_tree_gather(r->trees.p, r->cap, d_off.p, r->tree_size.p, r->n_run, packed.p, 0);
         CK(cudaMemcpy(dst, packed.p, tot * sizeof(bvh_node), cudaMemcpyDefault));
     });
