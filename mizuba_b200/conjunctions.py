@@ -276,8 +276,8 @@ class device_conjunctions:
 
     @property
     def narrow_split(self):
-        """Mixed form: (items past the distance screen, items past the FMA
-        prefilter); zeros for the plain form."""
+        """Mixed form: (items past the distance screen, items whose FMA
+        enclosure reaches below the threshold); zeros for the plain form."""
         out = (ct.c_uint64 * 2)()
         self._L.mzb_result_narrow_split(self._h, ct.addressof(out))
         return tuple(int(x) for x in out)
@@ -305,7 +305,7 @@ class conjunctions:
     """Conjunction screening of a polyjectory (the drop-in for
     ``mizuba.conjunctions``).  ``steps_per_batch``, ``step_range`` (a shard of
     the time axis) and ``form`` ("plain": the reference's FP64 arithmetic;
-    "mixed": enclosing boxes and an FP64 prefilter with the same conjunction
+    "mixed": enclosing boxes and a distance screen with the same conjunction
     records) are extensions."""
 
     bvh_node = BVH_NODE

@@ -4,7 +4,12 @@
 // k_items: one thread per broad-phase pair walks the two objects' segment
 //   boundaries (narrow.cpp:345-418) and appends every overlapping
 //   sub-interval to a device queue of items.
-// k_narrow: one thread per item (persistent grid pulling from that queue)
+// k_narrow_filter: one thread per item (persistent grid pulling from that
+//   queue) settles the items whose outcome a cheap FMA formulation proves:
+//   those whose enclosure clears the threshold, and those with one interior
+//   minimum that clears it.  In the mixed form a distance screen inside the
+//   merge walk drops most items before it.
+// k_narrow: one thread per item that is left
 //   translates both position polynomials to the sub-interval start
 //   (conjunctions_jit.cpp:68-140), evaluates them at the order+1 Chebyshev
 //   nodes, interpolates the squared distance with Bjorck-Pereyra
@@ -20,6 +25,9 @@
 //   threshold test on the interpolant, the trajectory-boundary minima
 //   (narrow.cpp:629-714) and the state vectors at TCA (narrow.cpp:542-575).
 // k_conj_*: per-step ordering by (tca, record) (narrow.cpp:751-757).
+#include <algorithm>
+#include <cmath>
+
 #include "block.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -130,93 +138,255 @@ __global__ void __launch_bounds__(128) k_items(const dev_pj pj, const double2 *_
     warp_add(counters + 0, n_cand);
 }
 
-// One thread per item (persistent grid over the device-side item count).
-// The per-item arithmetic is the reference's, operation for operation.
-template <int OP1>
-__global__ void __launch_bounds__(128, 3) k_narrow(dev_pj pj, cheb_nodes cheb, const double2 *__restrict__ cd_bounds,
-                                                   uint32_t s_first, const np_item *__restrict__ items,
-                                                   const unsigned long long *item_count, uint64_t item_cap,
-                                                   double thresh2, root_item *__restrict__ rq, uint64_t rq_cap,
-                                                   unsigned long long *rq_count, unsigned long long *counters,
-                                                   dev_status *st)
+// The reference formulation of one item, operation for operation.  Persistent
+// grid over the device-side item count: one thread per item, or, for few
+// items, one warp.
+//
+// The filter leaves 1 % of a day's items and 2 % of dense catalogues'.  The
+// 11,000 dependent FP64 operations of an item take one thread 63 us however
+// few the items, which is 6 % of a small call.  With a warp per item (lane I
+// computes translated coefficient I, node I, divided difference I; every
+// value by the same operations in the same order, so bit for bit the same)
+// they take 19 us; the warp keeps 19 of 32 lanes busy at order 18 and repeats
+// the powers, so beyond WARP_ITEMS items, three or four a resident warp, the
+// thread per item is faster (13,000 items: 67 against 105 us; 517,000 of
+// 60,000 objects x 48 steps at 20 km: 0.65 ms).  That path keeps node values and
+// squared distances in a shared-memory column per thread, so that its loops
+// over objects, coordinates, nodes and divided differences stay loops (14,000
+// instructions unrolled, 0.71 ms).
+constexpr int NARROW_T = 64;
+constexpr uint64_t WARP_ITEMS = 6144;
+
+// The sub-interval of an item: false (with the reference's error) when it is
+// not a valid one.
+struct sub_interval {
+    double lb_rf, ub_rf, rf_int, di, dj;
+    uint64_t gsi, gsj;
+    uint32_t flags; // 1 = end of trajectory data, 2 = start
+};
+__device__ __forceinline__ bool item_interval(const dev_pj &pj, const double2 *__restrict__ cd_bounds,
+                                              uint32_t s_first, const np_item &it, sub_interval &v)
 {
+    const double2 cbe = cd_bounds[s_first + it.b];
+    const double cb = cbe.x, ce = cbe.y;
+    const double *ti = pj.time + pj.time_off[it.i];
+    const double *tj = pj.time + pj.time_off[it.j];
+    const double si = ti[it.it_i - 1], sj = tj[it.it_j - 1];
+    const double ti_e = ti[it.it_i], tj_e = tj[it.it_j];
+    const double lb_i = dmax_ref(cb, si), ub_i = dmin_ref(ce, ti_e);
+    const double lb_j = dmax_ref(cb, sj), ub_j = dmin_ref(ce, tj_e);
+    v.lb_rf = dmax_ref(lb_i, lb_j);
+    v.ub_rf = dmin_ref(ub_i, ub_j);
+    v.di = v.lb_rf - si;
+    v.dj = v.lb_rf - sj;
+    v.rf_int = v.ub_rf - v.lb_rf;
+    v.gsi = pj.seg_off[it.i] + it.it_i - 1;
+    v.gsj = pj.seg_off[it.j] + it.it_j - 1;
+    const uint32_t nsi = pj.nseg[it.i], nsj = pj.nseg[it.j];
+    v.flags = 0;
+    if ((it.it_i == nsi && ti_e == v.ub_rf) || (it.it_j == nsj && tj_e == v.ub_rf)) v.flags |= 1u;
+    if ((it.it_i == 1 && v.lb_rf == ti[0]) || (it.it_j == 1 && v.lb_rf == tj[0])) v.flags |= 2u;
+    return isfinite(v.di) && isfinite(v.dj) && isfinite(v.rf_int) && v.di >= 0 && v.dj >= 0 && v.rf_int >= 0;
+}
+
+__device__ __forceinline__ void fill_root_item(root_item &q, const np_item &it, const sub_interval &v)
+{
+    q.i = it.i;
+    q.j = it.j;
+    q.step = it.b;
+    q.flags = v.flags;
+    q.lb_rf = v.lb_rf;
+    q.rf_int = v.rf_int;
+    q.di = v.di;
+    q.dj = v.dj;
+    q.seg_i = v.gsi;
+    q.seg_j = v.gsj;
+}
+
+// One item by one warp (OP1 <= 32); shift[k * OP1 + i] = C(i + k, k).  Returns
+// whether the item goes to root finding, lane k's f then being coefficient k
+// of its squared-distance polynomial.  The pairwise sums run over OP1 terms in
+// every lane: a lane with fewer has -0.0 in the others' places, and x + -0.0
+// is x, so the tree is the reference's.
+template <int OP1>
+__device__ __forceinline__ bool narrow_by_warp(const dev_pj &pj, const double *__restrict__ shift,
+                                               const double *nodes, const np_item &it, const sub_interval &v,
+                                               double thresh2, unsigned long long &n_pruned, double &f,
+                                               dev_status *st)
+{
+    constexpr int n = OP1 - 1;
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31;
+    const bool in = lane < OP1;
+    const double node = in ? nodes[lane] : 0.0;
+    const double x = node * v.rf_int;
+    double vi = 0;
+    f = 0;
+#pragma unroll 1
+    for (int r = 0; r < 6; ++r) {
+        const int c = r >> 1, o = r & 1; // coordinate, object
+        const double delta = o ? v.dj : v.di;
+        double tr = in ? __ldg(coef_row<OP1>(pj, o ? v.gsj : v.gsi, c) + lane) : 0.0;
+        if (delta != 0) {
+            double ap[OP1], t[OP1];
+            powers<OP1>(delta, ap);
+#pragma unroll
+            for (int k = 0; k < OP1; ++k) {
+                const double ck = __shfl_down_sync(ALL, tr, k);
+                t[k] = lane + k <= n ? (ck * __ldg(shift + k * OP1 + lane)) * ap[k] : -0.0;
+            }
+            tr = pw<OP1>::reduce(t, add_op{});
+        }
+        double h = __shfl_sync(ALL, tr, n);
+#pragma unroll
+        for (int k = n - 1; k >= 0; --k) h = __shfl_sync(ALL, tr, k) + h * x;
+        if (o == 0) {
+            vi = h;
+        } else {
+            const double d = vi - h;
+            f = (c == 0) ? d * d : f + d * d;
+        }
+    }
+    // Bjorck-Pereyra on the ascending nodes.
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const double lo = __shfl_up_sync(ALL, f, 1), a_lo = __shfl_up_sync(ALL, x, k + 1);
+        if (in && int(lane) > k) f = (f - lo) / (x - a_lo);
+    }
+#pragma unroll 1
+    for (int k = n - 1; k >= 0; --k) {
+        const double hi = __shfl_down_sync(ALL, f, 1), ck = __shfl_sync(ALL, x, k);
+        if (int(lane) >= k && int(lane) < n) f = f - ck * hi;
+    }
+    // Cargo-Shisha: lane 0 meets b_k at step k.
+    double dp[OP1], t = f;
+    powers<OP1>(v.rf_int, dp);
+#pragma unroll
+    for (int k = 0; k < OP1; ++k)
+        if (int(lane) == k) t = (t * dp[k]) / c_binom[n][k];
+    double emin = t, emax = t;
+#pragma unroll 1
+    for (int k = 1; k < OP1; ++k) {
+        t = t + __shfl_down_sync(ALL, t, 1);
+        emin = hy_min_op{}(emin, t);
+        emax = hy_max_op{}(emax, t);
+    }
+    emin = __shfl_sync(ALL, emin, 0);
+    emax = __shfl_sync(ALL, emax, 0);
+    if (!isfinite(emin) || !isfinite(emax)) {
+        if (lane == 0) set_error(st, ERR_NP_NONFINITE, it.i, it.j, 0, 0);
+        return false;
+    }
+    if (emin < thresh2) return true;
+    n_pruned += lane == 0;
+    return false;
+}
+
+template <int OP1>
+__global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb, const double *__restrict__ shift,
+                                                     const double2 *__restrict__ cd_bounds,
+                                                     uint32_t s_first, const np_item *__restrict__ items,
+                                                     const unsigned long long *item_count, uint64_t item_cap,
+                                                     double thresh2, root_item *__restrict__ rq, uint64_t rq_cap,
+                                                     unsigned long long *rq_count, unsigned long long *counters,
+                                                     dev_status *st)
+{
+    __shared__ double vs[OP1][NARROW_T], fs[OP1][NARROW_T], nodes[OP1];
+    const unsigned tid = threadIdx.x;
+    if (tid < OP1) nodes[tid] = cheb.v[tid];
+    __syncthreads();
     const uint64_t n_items = min(*item_count, (unsigned long long)item_cap);
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    const uint64_t stride = uint64_t(gridDim.x) * NARROW_T;
     unsigned long long n_pruned = 0;
-    for (uint64_t base = blockIdx.x * uint64_t(blockDim.x); base < n_items; base += stride) {
-        const uint64_t q_idx = base + threadIdx.x;
+    if constexpr (OP1 <= 32) {
+        if (n_items <= WARP_ITEMS) {
+            const unsigned lane = tid & 31;
+            const uint64_t nwarps = stride / 32;
+            for (uint64_t w = (blockIdx.x * uint64_t(NARROW_T) + tid) / 32; w < n_items; w += nwarps) {
+                const np_item it = items[w];
+                sub_interval v;
+                if (!item_interval(pj, cd_bounds, s_first, it, v)) {
+                    if (lane == 0) set_error(st, ERR_NP_INTERVAL, it.i, it.j, 0, 0);
+                    continue;
+                }
+                double f;
+                if (!narrow_by_warp<OP1>(pj, shift, nodes, it, v, thresh2, n_pruned, f, st)) continue;
+                unsigned long long slot = 0;
+                if (lane == 0) slot = atomicAdd(rq_count, 1ull);
+                slot = __shfl_sync(0xffffffffu, slot, 0);
+                if (slot < rq_cap) {
+                    if (lane == 0) fill_root_item(rq[slot], it, v);
+                    if (lane < OP1) rq[slot].ptd2[lane] = f;
+                }
+            }
+            warp_add(counters + 1, n_pruned);
+            return;
+        }
+    }
+    for (uint64_t base = blockIdx.x * uint64_t(NARROW_T); base < n_items; base += stride) {
+        const uint64_t q_idx = base + tid;
         const bool active = q_idx < n_items;
         bool push = false;
         np_item it{};
-        double lb_rf = 0, rf_int = 0, di = 0, dj = 0;
-        uint32_t flags = 0;
-        uint64_t gsi = 0, gsj = 0;
-        double f[OP1];
+        sub_interval v{};
         if (active) {
             it = items[q_idx];
-            const double2 cbe = cd_bounds[s_first + it.b];
-            const double cb = cbe.x, ce = cbe.y;
-            const double *ti = pj.time + pj.time_off[it.i];
-            const double *tj = pj.time + pj.time_off[it.j];
-            const double si = ti[it.it_i - 1], sj = tj[it.it_j - 1];
-            const double ti_e = ti[it.it_i], tj_e = tj[it.it_j];
-            const double lb_i = dmax_ref(cb, si), ub_i = dmin_ref(ce, ti_e);
-            const double lb_j = dmax_ref(cb, sj), ub_j = dmin_ref(ce, tj_e);
-            lb_rf = dmax_ref(lb_i, lb_j);
-            const double ub_rf = dmin_ref(ub_i, ub_j);
-            di = lb_rf - si;
-            dj = lb_rf - sj;
-            rf_int = ub_rf - lb_rf;
-            if (!isfinite(di) || !isfinite(dj) || !isfinite(rf_int) || di < 0 || dj < 0 || rf_int < 0) {
+            if (!item_interval(pj, cd_bounds, s_first, it, v)) {
                 set_error(st, ERR_NP_INTERVAL, it.i, it.j, 0, 0);
             } else {
-                gsi = pj.seg_off[it.i] + it.it_i - 1;
-                gsj = pj.seg_off[it.j] + it.it_j - 1;
-                const double *ci_base = coef_row<OP1>(pj, gsi, 0);
-                const double *cj_base = coef_row<OP1>(pj, gsj, 0);
+                const double rf_int = v.rf_int;
 #pragma unroll 1
-                for (int c = 0; c < 3; ++c) {
-                    double cf[OP1], tr[OP1], vi[OP1];
-                    load_row<OP1>(ci_base + c * row_ld(OP1), cf);
-                    if (di != 0) translate<OP1>(cf, di, tr);
+                for (int r = 0; r < 6; ++r) {
+                    const int c = r >> 1, o = r & 1; // coordinate, object
+                    const double delta = o ? v.dj : v.di;
+                    double cf[OP1], tr[OP1];
+                    load_row<OP1>(coef_row<OP1>(pj, o ? v.gsj : v.gsi, c), cf);
+                    if (delta != 0) translate<OP1>(cf, delta, tr);
                     else
 #pragma unroll
                         for (int k = 0; k < OP1; ++k) tr[k] = cf[k];
-#pragma unroll
-                    for (int m = 0; m < OP1; ++m) vi[m] = horner<OP1>(tr, cheb.v[m] * rf_int);
-                    load_row<OP1>(cj_base + c * row_ld(OP1), cf);
-                    if (dj != 0) translate<OP1>(cf, dj, tr);
-                    else
-#pragma unroll
-                        for (int k = 0; k < OP1; ++k) tr[k] = cf[k];
-#pragma unroll
+#pragma unroll 4
                     for (int m = 0; m < OP1; ++m) {
-                        const double d = vi[m] - horner<OP1>(tr, cheb.v[m] * rf_int);
-                        f[m] = (c == 0) ? d * d : f[m] + d * d;
+                        const double h = horner<OP1>(tr, nodes[m] * rf_int);
+                        if (o == 0) {
+                            vs[m][tid] = h;
+                        } else {
+                            const double d = vs[m][tid] - h;
+                            fs[m][tid] = (c == 0) ? d * d : fs[m][tid] + d * d;
+                        }
                     }
                 }
                 // Bjorck-Pereyra on the ascending nodes.
-#pragma unroll
-                for (int k = 0; k < OP1 - 1; ++k)
-#pragma unroll
-                    for (int jj = OP1 - 1; jj > k; --jj)
-                        f[jj] = (f[jj] - f[jj - 1]) / (cheb.v[jj] * rf_int - cheb.v[jj - k - 1] * rf_int);
-#pragma unroll
-                for (int k = OP1 - 2; k >= 0; --k)
-#pragma unroll
-                    for (int jj = k; jj < OP1 - 1; ++jj) f[jj] = f[jj] - (cheb.v[k] * rf_int) * f[jj + 1];
+#pragma unroll 1
+                for (int k = 0; k < OP1 - 1; ++k) {
+                    double hi = fs[OP1 - 1][tid];
+#pragma unroll 4
+                    for (int jj = OP1 - 1; jj > k; --jj) {
+                        const double lo = fs[jj - 1][tid];
+                        fs[jj][tid] = (hi - lo) / (nodes[jj] * rf_int - nodes[jj - k - 1] * rf_int);
+                        hi = lo;
+                    }
+                }
+#pragma unroll 1
+                for (int k = OP1 - 2; k >= 0; --k) {
+                    const double ck = nodes[k] * rf_int;
+                    double lo = fs[k][tid];
+#pragma unroll 4
+                    for (int jj = k; jj < OP1 - 1; ++jj) {
+                        const double hi = fs[jj + 1][tid];
+                        fs[jj][tid] = lo - ck * hi;
+                        lo = hi;
+                    }
+                }
                 double e[OP1];
 #pragma unroll
-                for (int k = 0; k < OP1; ++k) e[k] = f[k];
+                for (int k = 0; k < OP1; ++k) e[k] = fs[k][tid];
                 double emin, emax;
                 cs_from_translated<OP1>(e, rf_int, emin, emax);
                 if (!isfinite(emin) || !isfinite(emax)) {
                     set_error(st, ERR_NP_NONFINITE, it.i, it.j, 0, 0);
                 } else if (emin < thresh2) {
                     push = true;
-                    const uint32_t nsi = pj.nseg[it.i], nsj = pj.nseg[it.j];
-                    if ((it.it_i == nsi && ti_e == ub_rf) || (it.it_j == nsj && tj_e == ub_rf)) flags |= 1u;
-                    if ((it.it_i == 1 && lb_rf == ti[0]) || (it.it_j == 1 && lb_rf == tj[0])) flags |= 2u;
                 } else {
                     ++n_pruned;
                 }
@@ -225,66 +395,133 @@ __global__ void __launch_bounds__(128, 3) k_narrow(dev_pj pj, cheb_nodes cheb, c
         const unsigned long long slot = warp_append(rq_count, push);
         if (push && slot < rq_cap) {
             root_item &q = rq[slot];
-            q.i = it.i;
-            q.j = it.j;
-            q.step = it.b;
-            q.flags = flags;
-            q.lb_rf = lb_rf;
-            q.rf_int = rf_int;
-            q.di = di;
-            q.dj = dj;
-            q.seg_i = gsi;
-            q.seg_j = gsj;
-#pragma unroll
-            for (int k = 0; k < OP1; ++k) q.ptd2[k] = f[k];
+            fill_root_item(q, it, v);
+#pragma unroll 4
+            for (int k = 0; k < OP1; ++k) q.ptd2[k] = fs[k][tid];
         }
     }
     warp_add(counters + 1, n_pruned);
 }
 
-// ------------------------------------------------------------ mixed form
+// ---------------------------------------------------------------- filter
 //
-// A conservative FMA-native prefilter in front of k_narrow.  For each item
-// the dist^2 interpolant is formed cheaply: each object's original segment
-// polynomial is evaluated by FMA Horner at the shifted nodes delta + alpha_m
-// (mathematically the translated polynomial at alpha_m, so the explicit
-// translation is skipped), the squared distances are interpolated in the
-// normalised time s = t / rf_int on the fixed nodes c_m with Bjorck-Pereyra
-// using precomputed reciprocals 1 / (c_j - c_{j-k-1}), and the Cargo-Shisha
-// enclosure over s in [0, 1] needs no powers of rf_int.  An item is dropped
-// only if this enclosure clears threshold^2 by a margin (1e-8 of the largest
-// sampled dist^2 plus 1e-12 of threshold^2) that covers the difference from
-// the reference formulation; the survivors are queued and recomputed by
-// k_narrow with the reference formulation, so every conjunction record comes
-// from the reference arithmetic.  It runs on the items that the distance screen
-// leaves.
+// In front of k_narrow, in both forms.  Of the items of a catalogue day 85 %
+// have an enclosure that clears the threshold and 15 % go to root finding,
+// where all but 1 % turn out to have one minimum, above the threshold.  The
+// reference formulation takes 8,921 FP64 operations and 190 divisions for an
+// item, and root finding as much again; which of the two outcomes it will
+// have can be proven from an FMA-native evaluation of 3,000 operations:
+//
+// * each object's segment polynomial is evaluated by FMA Horner at the nodes
+//   delta + c_m rf_int (mathematically the translated polynomial at
+//   c_m rf_int: the explicit translation is skipped); the squared distances
+//   are interpolated in the normalised time s = t / rf_int on the fixed nodes
+//   c_m by Bjorck-Pereyra with precomputed reciprocals 1 / (c_j - c_{j-k-1}),
+//   and their Bernstein coefficients b_i over [0, 1] come from the difference
+//   table of Cargo-Shisha;
+// * both formulations interpolate the same values on the same nodes.  Their
+//   Bernstein coefficients differ by the rounding of the values (of order
+//   u P sqrt(max f) + u max f, with P = sum |c_k| (delta + rf_int)^k over both
+//   objects and the three coordinates), which interpolation amplifies by at
+//   most the largest Bernstein coefficient of the Chebyshev polynomial,
+//   A_n = C(2n, n) / C(n, n / 2), for a single value.  Over random pairs of
+//   catalogue segments (orders 2 to 32, sub-intervals from 1e-6 of a segment
+//   to a whole one, distances from 1 m to 2,000 km) the largest difference was
+//   1.5 u A_n (P sqrt(max f) + max f) at order 2 and at most 0.5 of that from
+//   order 12 on; the margin M takes 32 (and a P^2 term for vanishing f);
+// * min b >= threshold^2 + M: the reference prunes the item (counter 1);
+// * b_1 - b_0 < -2M, b_n - b_{n-1} > 2M, every second difference > 4M and
+//   min b < threshold^2 - M: the reference keeps the item and finds exactly
+//   one root of the derivative, a minimum.  The polynomial is convex with
+//   p'' / 2 >= kappa = n (n - 1) / 2 min (second difference), so p is at least
+//   p(s) - p'(s)^2 / (4 kappa) for any s; after two Newton steps from the
+//   secant of p' that bound is the minimum itself for all purposes.  If it is
+//   at least threshold^2 + 2M, the minimum is discarded (counters 2, 5 and 6)
+//   and no trajectory boundary in the item can be below the threshold either;
+// * everything else (also values outside the range in which neither
+//   formulation can overflow: see filter_limits) goes to k_narrow.
+//
+// So the records and all counters are those of the reference formulation.
+//
+// Bound by the FP64 pipe, if the coefficients arrive: 960 bytes an item, in
+// rows of 160 (order 18).  Loaded by each thread for itself, a 16-byte load of
+// a warp touched 32 lines and the load pipe was the bound (31 % of the FP64
+// rate).  Here a warp copies its items' rows of one coordinate to shared
+// memory together (cp.async, consecutive lanes on consecutive bytes of a row),
+// reads them back at an odd stride of 16-byte units (conflict-free), and has
+// the next coordinate's copies in flight while it computes.  6.38 M items of
+// the 20,000-object day: 2.6 ms, 49 % of the FP64 rate (three warps a
+// scheduler at 168 registers; the rest is latency of the dependent FMAs).
+// Narrow phase with root finding, plain form, 10.4 -> 3.1 ms; mixed form
+// 3.1 -> 1.2 ms; 60,000 objects x 48 steps at 20 km, mixed, 11.9 -> 4.7 ms.
 //
 // tab layout (doubles): [0, OP1) nodes c_m; [OP1, OP1 + OP1^2) inverse node
-// differences, row k; then OP1 inverse binomials 1 / C(n, i).
+// differences, row k; then OP1 inverse binomials 1 / C(n, i); then the
+// binomials of k_narrow's warp path, row k: C(i + k, k).
+//
+// One warp a CTA: the work is per warp, and its shared memory (rows and f)
+// stays below 48 KB up to order 32.
 template <int OP1>
-__global__ void __launch_bounds__(128, 3) k_narrow_mixed(dev_pj pj, const double *__restrict__ tab,
-                                                         const double2 *__restrict__ cd_bounds, uint32_t s_first,
-                                                         const np_item *__restrict__ items,
-                                                         const unsigned long long *item_count, uint64_t item_cap,
-                                                         double thresh2, np_item *__restrict__ surv,
-                                                         uint64_t surv_cap, unsigned long long *surv_count,
-                                                         unsigned long long *counters, dev_status *st)
+struct filter_shape {
+    static constexpr int UNITS = row_ld(OP1) / 2; // 16-byte units of a row
+    static constexpr int STRIDE = UNITS | 1;      // odd: conflict-free 16-byte reads
+    static constexpr int GROUPS = 32 / UNITS;     // rows copied per instruction
+    static constexpr int CTAS = OP1 <= 22 ? 12 : 8;
+};
+
+template <int OP1>
+__global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
+    k_narrow_filter(dev_pj pj, const double *__restrict__ tab, filter_limits lim,
+                    const double2 *__restrict__ cd_bounds, uint32_t s_first, const np_item *__restrict__ items,
+                    const unsigned long long *item_count, uint64_t item_cap, double thresh2,
+                    np_item *__restrict__ surv, uint64_t surv_cap, unsigned long long *surv_count,
+                    unsigned long long *counters)
 {
+    using F = filter_shape<OP1>;
     constexpr int n = OP1 - 1;
+    __shared__ __align__(16) double2 rows[64 * F::STRIDE];
+    __shared__ double fs[OP1][32];
+    __shared__ const double2 *base[64];
+    const unsigned lane = threadIdx.x;
     const double *cheb = tab;
     const double *inv_dd = tab + OP1;
     const double *inv_binom = tab + OP1 + OP1 * OP1;
     const uint64_t n_items = min(*item_count, (unsigned long long)item_cap);
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    unsigned long long n_pruned = 0;
-    for (uint64_t base = blockIdx.x * uint64_t(blockDim.x); base < n_items; base += stride) {
-        const uint64_t q_idx = base + threadIdx.x;
+    unsigned long long n_pruned = 0, n_single = 0;
+    // The rows of coordinate c of the warp's 32 items (first object: rows
+    // 0..31, second: 32..63), GROUPS rows at a time.
+    const unsigned part = lane % F::UNITS, grp = lane / F::UNITS;
+    const unsigned dst0 = unsigned(__cvta_generic_to_shared(rows + grp * F::STRIDE + part));
+    auto fetch = [&](int c) {
+#pragma unroll
+        for (int k = 0; k < (64 + F::GROUPS - 1) / F::GROUPS; ++k) {
+            const unsigned r = grp + unsigned(k * F::GROUPS);
+            if (grp < F::GROUPS && r < 64) {
+                const double2 *src = base[r] + c * F::UNITS + part;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 dst0 + unsigned(k * F::GROUPS * F::STRIDE * 16)),
+                             "l"(src)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto row_in = [&](const double2 *r, double(&c)[OP1]) {
+#pragma unroll
+        for (int k = 0; k < OP1 / 2; ++k) {
+            const double2 v = r[k];
+            c[2 * k] = v.x;
+            c[2 * k + 1] = v.y;
+        }
+        if (OP1 & 1) c[OP1 - 1] = r[OP1 / 2].x;
+    };
+    for (uint64_t b0 = blockIdx.x * uint64_t(32); b0 < n_items; b0 += uint64_t(gridDim.x) * 32) {
+        const uint64_t q_idx = b0 + lane;
         const bool active = q_idx < n_items;
-        bool push = false;
         np_item it{};
-        double lb_rf = 0, rf_int = 0, di = 0, dj = 0;
+        double rf_int = 0, di = 0, dj = 0;
         uint64_t gsi = 0, gsj = 0;
-        double f[OP1];
+        bool usable = false;
         if (active) {
             it = items[q_idx];
             const double2 cbe = cd_bounds[s_first + it.b];
@@ -292,85 +529,128 @@ __global__ void __launch_bounds__(128, 3) k_narrow_mixed(dev_pj pj, const double
             const double *ti = pj.time + pj.time_off[it.i];
             const double *tj = pj.time + pj.time_off[it.j];
             const double si = ti[it.it_i - 1], sj = tj[it.it_j - 1];
-            const double ti_e = ti[it.it_i], tj_e = tj[it.it_j];
-            const double lb_i = dmax_ref(cb, si), ub_i = dmin_ref(ce, ti_e);
-            const double lb_j = dmax_ref(cb, sj), ub_j = dmin_ref(ce, tj_e);
-            lb_rf = dmax_ref(lb_i, lb_j);
+            const double lb_i = dmax_ref(cb, si), ub_i = dmin_ref(ce, ti[it.it_i]);
+            const double lb_j = dmax_ref(cb, sj), ub_j = dmin_ref(ce, tj[it.it_j]);
+            const double lb_rf = dmax_ref(lb_i, lb_j);
             const double ub_rf = dmin_ref(ub_i, ub_j);
-            (void)ti_e;
-            (void)tj_e;
             di = lb_rf - si;
             dj = lb_rf - sj;
             rf_int = ub_rf - lb_rf;
-            if (!isfinite(di) || !isfinite(dj) || !isfinite(rf_int) || di < 0 || dj < 0 || rf_int < 0) {
-                push = true; // the exact recheck reports the invalid interval
-            } else {
-                gsi = pj.seg_off[it.i] + it.it_i - 1;
-                gsj = pj.seg_off[it.j] + it.it_j - 1;
-                const double *ci_base = coef_row<OP1>(pj, gsi, 0);
-                const double *cj_base = coef_row<OP1>(pj, gsj, 0);
+            usable = di >= 0 && dj >= 0 && rf_int >= lim.rf_lo && rf_int <= lim.rf_hi;
+            gsi = pj.seg_off[it.i] + it.it_i - 1;
+            gsj = pj.seg_off[it.j] + it.it_j - 1;
+        }
+        // Rows of lanes without an item are segment 0's: copied, not used.
+        base[lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsi, 0));
+        base[32 + lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsj, 0));
+        __syncwarp();
+        fetch(0);
+        double P = 0;
+        const double ei = di + rf_int, ej = dj + rf_int;
 #pragma unroll 1
-                for (int c = 0; c < 3; ++c) {
-                    double ci[OP1], cj[OP1];
-                    load_row<OP1>(ci_base + c * row_ld(OP1), ci);
-                    load_row<OP1>(cj_base + c * row_ld(OP1), cj);
+        for (int c = 0; c < 3; ++c) {
+            double ci[OP1], cj[OP1];
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+            row_in(rows + lane * F::STRIDE, ci);
+            row_in(rows + (32 + lane) * F::STRIDE, cj);
+            __syncwarp(); // every row is in registers: the next ones may land
+            if (c < 2) fetch(c + 1);
+            double pi = fabs(ci[n]), pj_ = fabs(cj[n]);
 #pragma unroll
-                    for (int m = 0; m < OP1; ++m) {
-                        const double am = __ldg(cheb + m) * rf_int;
-                        const double tii = di + am, tjj = dj + am;
-                        double xi = ci[n], xj = cj[n];
-#pragma unroll
-                        for (int k = n - 1; k >= 0; --k) {
-                            xi = fma(xi, tii, ci[k]);
-                            xj = fma(xj, tjj, cj[k]);
-                        }
-                        const double d = xi - xj;
-                        f[m] = (c == 0) ? d * d : fma(d, d, f[m]);
-                    }
-                }
-                double fmax_s = f[0];
-#pragma unroll
-                for (int m = 1; m < OP1; ++m) fmax_s = fmax(fmax_s, f[m]);
-                // Bjorck-Pereyra on the normalised nodes.
-#pragma unroll
-                for (int k = 0; k < n; ++k)
-#pragma unroll
-                    for (int jj = n; jj > k; --jj) f[jj] = (f[jj] - f[jj - 1]) * __ldg(inv_dd + k * OP1 + jj);
+            for (int k = n - 1; k >= 0; --k) {
+                pi = fma(pi, ei, fabs(ci[k]));
+                pj_ = fma(pj_, ej, fabs(cj[k]));
+            }
+            P += pi + pj_;
+            // The sums of squares stay in shared memory between coordinates:
+            // in registers they made this loop spill, and unrolled whole it
+            // was 10,000 instructions, whose fetch was most of a small call.
+#pragma unroll 4
+            for (int m = 0; m < OP1; ++m) {
+                const double am = __ldg(cheb + m) * rf_int;
+                const double tii = di + am, tjj = dj + am;
+                double xi = ci[n], xj = cj[n];
 #pragma unroll
                 for (int k = n - 1; k >= 0; --k) {
-                    const double ck = __ldg(cheb + k);
-#pragma unroll
-                    for (int jj = k; jj < n; ++jj) f[jj] = fma(-ck, f[jj + 1], f[jj]);
+                    xi = fma(xi, tii, ci[k]);
+                    xj = fma(xj, tjj, cj[k]);
                 }
-                // Cargo-Shisha over s in [0, 1].
-                double e[OP1];
-#pragma unroll
-                for (int k = 0; k < OP1; ++k) e[k] = f[k] * __ldg(inv_binom + k);
-                double emin = e[0], emax = e[0];
-#pragma unroll
-                for (int k = 1; k < OP1; ++k) {
-#pragma unroll
-                    for (int jj = 0; jj + k < OP1; ++jj) e[jj] = e[jj] + e[jj + 1];
-                    emin = fmin(emin, e[0]);
-                    emax = fmax(emax, e[0]);
-                }
-                const double margin = 1e-8 * fmax_s + 1e-12 * thresh2;
-                if (!(emin >= thresh2 + margin)) {
-                    // kept (non-finite values are left to the exact recheck,
-                    // which reports them as the reference does)
-                    push = true;
-                } else {
-                    ++n_pruned;
-                }
+                const double d = xi - xj;
+                fs[m][lane] = (c == 0) ? d * d : fma(d, d, fs[m][lane]);
             }
         }
+        double f[OP1];
+#pragma unroll
+        for (int m = 0; m < OP1; ++m) f[m] = fs[m][lane];
+        double fmax_s = f[0];
+#pragma unroll
+        for (int m = 1; m < OP1; ++m) fmax_s = fmax(fmax_s, f[m]);
+        // Bjorck-Pereyra on the normalised nodes.
+#pragma unroll
+        for (int k = 0; k < n; ++k)
+#pragma unroll
+            for (int jj = n; jj > k; --jj) f[jj] = (f[jj] - f[jj - 1]) * __ldg(inv_dd + k * OP1 + jj);
+#pragma unroll
+        for (int k = n - 1; k >= 0; --k) {
+            const double ck = __ldg(cheb + k);
+#pragma unroll
+            for (int jj = k; jj < n; ++jj) f[jj] = fma(-ck, f[jj + 1], f[jj]);
+        }
+        // Bernstein coefficients over s in [0, 1], each one's first and
+        // second differences as it appears.
+        double e[OP1];
+#pragma unroll
+        for (int k = 0; k < OP1; ++k) e[k] = f[k] * __ldg(inv_binom + k);
+        double emin = e[0], b1 = e[0], d_first = 0, d_prev = 0, dd_min = INFINITY;
+#pragma unroll
+        for (int k = 1; k < OP1; ++k) {
+#pragma unroll
+            for (int jj = 0; jj + k < OP1; ++jj) e[jj] = e[jj] + e[jj + 1];
+            emin = fmin(emin, e[0]);
+            const double d = e[0] - b1;
+            if (k == 1) d_first = d;
+            else dd_min = fmin(dd_min, d - d_prev);
+            d_prev = d;
+            b1 = e[0];
+        }
+        const double root_f = double(__fsqrt_ru(__double2float_ru(fmax_s)));
+        const double M = lim.margin * (root_f * P + fmax_s + 1e-14 * P * P);
+        usable = usable && fmax_s <= 1e30 && P <= 1e15; // false for non-finite values
+        const bool pruned = usable && emin >= thresh2 + M;
+        bool single = false;
+        if (usable && !pruned && emin < thresh2 - M && d_first < -2 * M && d_prev > 2 * M && dd_min > 4 * M) {
+            const double kappa = 0.5 * (double(n) * (n - 1)) * dd_min;
+            double s = d_first / (d_first - d_prev);
+            double p = 0, p1 = 0;
+#pragma unroll 1
+            for (int r = 0; r < 3; ++r) {
+                double p2 = 0;
+                p = f[n], p1 = 0;
+#pragma unroll
+                for (int k = n - 1; k >= 0; --k) {
+                    p2 = fma(p2, s, p1);
+                    p1 = fma(p1, s, p);
+                    p = fma(p, s, f[k]);
+                }
+                if (r < 2) s = fmin(fmax(s - p1 / (2 * p2), 0.0), 1.0);
+            }
+            single = p - p1 * p1 / (4 * kappa) >= thresh2 + 2 * M;
+        }
+        n_pruned += pruned;
+        n_single += single;
+        const bool push = active && !pruned && !single;
         const unsigned long long slot = warp_append(surv_count, push);
         if (push && slot < surv_cap) surv[slot] = it;
     }
     warp_add(counters + 1, n_pruned);
+    warp_add(counters + 2, n_single);
+    warp_add(counters + 5, n_single);
+    warp_add(counters + 6, n_single);
+    warp_add(counters + 7, n_single);
 }
 
-// Screen ahead of the mixed prefilter: a rigorous lower bound on the
+// Screen ahead of the filter (mixed form): a rigorous lower bound on the
 // distance over the item's sub-interval from linear models of both objects.
 // For each object, on the portion of its segment inside the step, Taylor's
 // theorem gives x(tm + s) = x(tm) + x'(tm) s + R(s) with |R(s)| <= |A| s^2 / 2,
@@ -382,7 +662,7 @@ __global__ void __launch_bounds__(128, 3) k_narrow_mixed(dev_pj pj, const double
 // term is the closest approach of a straight line, in closed form.  Items
 // whose bound clears the threshold (relative slack 1e-6) cannot hold a
 // conjunction: they are dropped and counted as pruned by the distance
-// check; the rest go on to k_narrow_mixed, compacted so its warps stay full.
+// check; the rest go on to k_narrow_filter, compacted so its warps stay full.
 //
 // The models come from the mixed AABB pass (32 bytes each, FP32: position,
 // velocity at the portion midpoint, |A| rounded up) for the first and second
@@ -498,7 +778,7 @@ __device__ __forceinline__ bool screen_keeps(const dev_pj &pj, const double2 *__
 
 // The mixed form's merge walk (k_items) with the distance screen inside: each item of the
 // merge walk is screened as it is found and only the items the screen keeps
-// are appended (to the prefilter's queue), so the day's 6.4 M items are
+// are appended (to the filter's queue), so the day's 6.4 M items are
 // never written out and read back.  Counters: every item (counter 0, and
 // *item_count), the pruned ones (counter 1).
 template <int OP1>
@@ -1226,16 +1506,17 @@ void launch_items(const dev_pj &pj, const double2 *cdb, uint32_t s_first, uint32
 }
 
 template <int OP1>
-static void narrow_t(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items,
+static void narrow_t(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first, const np_item *items,
                      const unsigned long long *item_count, uint64_t item_cap, double thresh2, root_item *rq,
                      uint64_t rq_cap, unsigned long long *rq_count, unsigned long long *counters, dev_status *st,
                      unsigned grid, cudaStream_t stream)
 {
-    k_narrow<OP1><<<grid, 128, 0, stream>>>(pj, make_cheb_nodes(OP1), cdb, s_first, items, item_count, item_cap,
-                                             thresh2, rq, rq_cap, rq_count, counters, st);
+    k_narrow<OP1><<<grid, NARROW_T, 0, stream>>>(pj, make_cheb_nodes(OP1), tab + OP1 * (OP1 + 2), cdb, s_first, items,
+                                                  item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st);
 }
 
-void launch_narrow(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items,
+// tab: the tables of launch_narrow_filter.
+void launch_narrow(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first, const np_item *items,
                    const unsigned long long *item_count, uint64_t item_cap, double thresh2, root_item *rq,
                    uint64_t rq_cap, unsigned long long *rq_count, unsigned long long *counters, dev_status *st,
                    unsigned grid, cudaStream_t stream)
@@ -1243,7 +1524,7 @@ void launch_narrow(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        narrow_t<K>(pj, cdb, s_first, items, item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st, grid, \
+        narrow_t<K>(pj, tab, cdb, s_first, items, item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st, grid, \
                     stream);                                                                                           \
         break;
         MZB_FOR_EACH_OP1(X)
@@ -1254,31 +1535,59 @@ void launch_narrow(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const
 }
 
 template <int OP1>
-static void prefilter_t(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first,
-                        const np_item *items, const unsigned long long *item_count, uint64_t item_cap, double thresh2,
-                        np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
-                        unsigned long long *counters, dev_status *st, unsigned grid, cudaStream_t stream)
+static void filter_t(const dev_pj &pj, const double *tab, const filter_limits &lim, const double2 *cdb,
+                     uint32_t s_first, const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
+                     double thresh2, np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
+                     unsigned long long *counters, cudaStream_t stream)
 {
-    k_narrow_mixed<OP1><<<grid, 128, 0, stream>>>(pj, tab, cdb, s_first, items, item_count, item_cap, thresh2, surv,
-                                                   surv_cap, surv_count, counters, st);
+    using F = filter_shape<OP1>;
+    k_narrow_filter<OP1><<<148 * F::CTAS, 32, 0, stream>>>(pj, tab, lim, cdb, s_first, items, item_count, item_cap,
+                                                             thresh2, surv, surv_cap, surv_count, counters);
 }
 
-void launch_narrow_prefilter(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first,
-                             const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
-                             double thresh2, np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
-                             unsigned long long *counters, dev_status *st, unsigned grid, cudaStream_t stream)
+void launch_narrow_filter(const dev_pj &pj, const double *tab, const filter_limits &lim, const double2 *cdb,
+                          uint32_t s_first, const np_item *items, const unsigned long long *item_count,
+                          uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
+                          unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream)
 {
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        prefilter_t<K>(pj, tab, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,       \
-                       counters, st, grid, stream);                                                                    \
+        filter_t<K>(pj, tab, lim, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,     \
+                    counters, stream);                                                                                 \
         break;
         MZB_FOR_EACH_OP1(X)
 #undef X
     default:
         break;
     }
+}
+
+// Where the filter's argument holds for order op1 - 1: the reference
+// formulation divides differences of f by node distances c rf_int, so its
+// k-th divided differences are at most 2^k max f / (G_k rf_int^k), G_k the
+// product of the smallest node distances at lags 1 to k; with max f <= 1e30
+// they stay below 1e280 for rf_int >= rf_lo, and neither rf_int^n nor its
+// inverse leaves the exponent range for rf_int in [rf_lo, rf_hi].
+filter_limits make_filter_limits(int op1)
+{
+    const int n = op1 - 1;
+    const cheb_nodes c = make_cheb_nodes(op1);
+    filter_limits lim{};
+    lim.rf_lo = std::pow(10.0, -250.0 / n);
+    lim.rf_hi = std::pow(10.0, 200.0 / n);
+    double log_g = 0;
+    for (int k = 1; k <= n; ++k) {
+        double gap = 1.0;
+        for (int j = k; j <= n; ++j) gap = std::min(gap, c.v[j] - c.v[j - k]);
+        log_g += std::log10(gap);
+        lim.rf_lo = std::max(lim.rf_lo, std::pow(10.0, (k * std::log10(2.0) + 30.0 - log_g - 280.0) / k));
+    }
+    double a = 1.0; // C(2n, n) / C(n, n / 2)
+    for (int k = 1; k <= n; ++k) a = a * (n + k) / k;
+    for (int k = 1; k <= n / 2; ++k) a = a * k / (n - n / 2 + k);
+    lim.margin = 32.0 * 1.1102230246251565e-16 * a;
+    return lim;
 }
 
 template <int OP1>

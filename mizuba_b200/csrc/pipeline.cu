@@ -616,7 +616,7 @@ struct mzb_result {
     dbuf<conj_rec> conj;
     uint64_t n_conj = 0;
     uint64_t np[7] = {};
-    uint64_t narrow_split[2] = {}; // mixed form: items past the screen, past the prefilter
+    uint64_t narrow_split[2] = {}; // mixed form: items past the screen, past the filter's enclosure
     double stage_ms[8] = {};
     uint64_t broad_visits = 0; // node visits of the default broad-phase walk
     mzb_result() = default;
@@ -956,9 +956,10 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     host_mailbox mbox(lease.cache, nb_cap * 4 + (nb_cap + 1) * 8 + 1024);
     uint32_t *h_tsz_pin = mbox.take<uint32_t>(nb_cap);
     uint64_t *h_so = mbox.take<uint64_t>(nb_cap + 1);
-    // Queue counts: items, root items, conjunctions, screened, prefiltered,
-    // then the 7 narrow-phase counters.
-    unsigned long long *h_q = mbox.take<unsigned long long>(5 + 7);
+    // Queue counts: items, root items, conjunctions, screened, left by the
+    // filter, then the 7 narrow-phase counters and the items that the filter
+    // settled as single minima.
+    unsigned long long *h_q = mbox.take<unsigned long long>(5 + 8);
     dev_status *h_status = mbox.take<dev_status>(1);
     unsigned long long *h_bad = mbox.take<unsigned long long>(1);
     unsigned long long *h_visits = mbox.take<unsigned long long>(1);
@@ -997,13 +998,14 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     }
     dbuf<double2> d_cdb(SL());
     d_cdb.alloc(S, st);
-    // Mixed-form tables: nodes, inverse node differences, inverse binomials.
+    // Tables of the narrow phase: nodes, inverse node differences, inverse
+    // binomials, binomials of the translation.
     dbuf<double> d_mixed(SL());
     std::vector<double> h_mixed;
-    if (mixed) {
+    {
         const int op1 = pj.order + 1, n = pj.order;
         const cheb_nodes cn = make_cheb_nodes(op1);
-        h_mixed.assign(size_t(op1) + size_t(op1) * op1 + op1, 0.0);
+        h_mixed.assign(size_t(op1) * (2 * op1 + 2), 0.0);
         for (int m = 0; m < op1; ++m) h_mixed[m] = cn.v[m];
         for (int k = 0; k < n; ++k)
             for (int j = k + 1; j < op1; ++j) h_mixed[op1 + size_t(k) * op1 + j] = 1.0 / (cn.v[j] - cn.v[j - k - 1]);
@@ -1012,10 +1014,16 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             h_mixed[op1 + size_t(op1) * op1 + i] = 1.0 / c;
             c = c * (n - i) / (i + 1);
         }
+        // C(i + k, k), exact: Pascal's rule along row k.
+        double *sh = h_mixed.data() + size_t(op1) * (op1 + 2);
+        for (int k = 0; k < op1; ++k)
+            for (int i = 0; i + k < op1; ++i)
+                sh[size_t(k) * op1 + i] = (k == 0 || i == 0) ? 1.0 : sh[size_t(k) * op1 + i - 1] + sh[size_t(k - 1) * op1 + i];
         d_mixed.alloc(h_mixed.size(), st);
         CK(cudaMemcpyAsync(d_mixed.p, h_mixed.data(), h_mixed.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     }
-    const double *mixed_tab = mixed ? d_mixed.p : nullptr;
+    const double *filter_tab = d_mixed.p;
+    const filter_limits filter_lim = make_filter_limits(pj.order + 1);
     const double *mixed_inv_binom = mixed ? d_mixed.p + (pj.order + 1) + size_t(pj.order + 1) * (pj.order + 1) : nullptr;
     CK(cudaMemcpyAsync(d_cdb.p, cdb.data(), S * sizeof(double2), cudaMemcpyHostToDevice, st));
     dbuf<int32_t> d_ot(SL());
@@ -1111,7 +1119,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     step_off.alloc(nb_max + 1, st);
     total.alloc(1, st);
     d_st.alloc(1, st);
-    ctr.alloc(7, st);
+    ctr.alloc(8, st);
     rq_count.alloc(1, st);
     cq_count.alloc(1, st);
     cc_cnt.alloc(nb_max + 1, st);
@@ -1126,7 +1134,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     item_count.alloc(1, st);
     surv_count.alloc(1, st);
     cand_count.alloc(1, st);
-    const unsigned narrow_grid = 148 * 3;
+    const unsigned narrow_grid = 148 * 6;
     dbuf<conj_out> cq(SL()), cgrp(SL());
     dbuf<double> wl(SL()), wl_full(SL());
     dbuf<uint32_t> retry(SL());
@@ -1283,7 +1291,8 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             R.n_bp += np_batch;
 
             // Narrow phase and minimum search: k_items appends sub-interval
-            // items, the persistent k_narrow consumes them and appends
+            // items, the persistent k_narrow_filter settles most of them, the
+            // persistent k_narrow consumes the rest and appends
             // surviving items to the root queue, the persistent k_roots
             // consumes that (items whose working list outgrows the short one
             // are retried with the full list).  Queue sizes are read on the
@@ -1291,45 +1300,44 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             // stage reruns with grown queues on overflow.
             auto sized = [np_batch](double per_pair) { return uint64_t(double(np_batch) * per_pair * 1.1) + 1024; };
             // The mixed form screens items as they are found: no item queue,
-            // the screen's queue (cand) and the prefilter's (surv) are sized
-            // for every item instead.
+            // the screen's queue (cand) is sized for every item instead, as
+            // is the queue of the items that the filter leaves (surv).
             const uint64_t item_cap0 = std::max<uint64_t>(mixed ? cand.n : items.n, sized(items_per_pair));
             if (!mixed && items.n < item_cap0) items.alloc_queue(item_cap0, st);
             if (mixed && cand.n < item_cap0) cand.alloc_queue(item_cap0, st);
-            if (mixed && surv.n < cand.n) surv.alloc_queue(cand.n, st);
+            if (surv.n < (mixed ? cand.n : items.n)) surv.alloc_queue(mixed ? cand.n : items.n, st);
             const uint64_t rq_cap0 = std::max<uint64_t>(rq.n, sized(roots_per_pair));
             if (rq.n < rq_cap0) rq.alloc_queue(rq_cap0, st);
             if (retry.n < rq.n) retry.alloc_queue(rq.n, st);
             const uint64_t cq_cap0 = std::max<uint64_t>(cq.n, sized(conj_per_pair));
             if (cq.n < cq_cap0) cq.alloc_queue(cq_cap0, st);
             tr.mark("pair list and queues allocated", std::to_string(np_batch) + " pairs");
-            unsigned long long h_rq = 0, h_items = 0, h_cq = 0, h_ctr[7] = {}, h_cand = 0, h_surv = 0;
+            unsigned long long h_rq = 0, h_items = 0, h_cq = 0, h_ctr[8] = {}, h_cand = 0, h_surv = 0;
             for (;;) {
-                CK(cudaMemsetAsync(ctr.p, 0, 7 * sizeof(unsigned long long), st));
+                CK(cudaMemsetAsync(ctr.p, 0, 8 * sizeof(unsigned long long), st));
                 CK(cudaMemsetAsync(rq_count.p, 0, sizeof(unsigned long long), st));
                 CK(cudaMemsetAsync(item_count.p, 0, sizeof(unsigned long long), st));
                 CK(cudaMemsetAsync(cq_count.p, 0, sizeof(unsigned long long), st));
                 CK(cudaMemsetAsync(retry_count.p, 0, sizeof(unsigned long long), st));
                 CK(cudaEventRecord(ev[4].a, st));
+                CK(cudaMemsetAsync(surv_count.p, 0, sizeof(unsigned long long), st));
                 if (mixed) {
-                    // Items screened as the merge walk finds them, the
-                    // FMA-native prefilter, then the reference formulation on
-                    // the survivors only.
-                    CK(cudaMemsetAsync(surv_count.p, 0, sizeof(unsigned long long), st));
+                    // Items screened as the merge walk finds them.
                     CK(cudaMemsetAsync(cand_count.p, 0, sizeof(unsigned long long), st));
                     launch_items_screen(P, d_cdb.p, sf, nb, bp_batch, step_off.p, srange.p, np_batch, thresh, scr.p,
                                         cand.p, cand.n, cand_count.p, item_count.p, ctr.p, d_st.p, st);
-                    launch_narrow_prefilter(P, mixed_tab, d_cdb.p, sf, cand.p, cand_count.p, cand.n, thresh2,
-                                            surv.p, surv.n, surv_count.p, ctr.p, d_st.p, narrow_grid, st);
-                    launch_narrow(P, d_cdb.p, sf, surv.p, surv_count.p, surv.n, thresh2, rq.p, rq.n, rq_count.p,
-                                  ctr.p, d_st.p, narrow_grid, st);
-                    n_narrow_launches += 1;
                 } else {
                     launch_items(P, d_cdb.p, sf, nb, bp_batch, step_off.p, srange.p, np_batch, items.p, items.n,
                                  item_count.p, ctr.p, d_st.p, st);
-                    launch_narrow(P, d_cdb.p, sf, items.p, item_count.p, items.n, thresh2, rq.p, rq.n, rq_count.p,
-                                  ctr.p, d_st.p, narrow_grid, st);
                 }
+                // The FMA filter, then the reference formulation on the items
+                // it leaves.
+                const dbuf<np_item> &src = mixed ? cand : items;
+                launch_narrow_filter(P, filter_tab, filter_lim, d_cdb.p, sf, src.p,
+                                     mixed ? cand_count.p : item_count.p, src.n, thresh2, surv.p, surv.n,
+                                     surv_count.p, ctr.p, st);
+                launch_narrow(P, filter_tab, d_cdb.p, sf, surv.p, surv_count.p, surv.n, thresh2, rq.p, rq.n, rq_count.p, ctr.p,
+                              d_st.p, narrow_grid, st);
                 CK(cudaEventRecord(ev[4].b, st));
                 CK(cudaEventRecord(ev[5].a, st));
                 launch_roots(P, rq.p, rq_count.p, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL, roots_grid,
@@ -1337,17 +1345,16 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 launch_roots(P, rq.p, rq_count.p, rq.n, retry.p, retry_count.p, thresh2, wl_full.p, ROOTS_WL_FULL,
                              roots_grid_full, nullptr, nullptr, cq.p, cq.n, cq_count.p, ctr.p, d_st.p, st);
                 CK(cudaEventRecord(ev[5].b, st));
-                n_narrow_launches += 2;
+                n_narrow_launches += 3;
                 n_roots_launches += 2;
                 {
                     auto job = mbox.start();
                     job.add(h_q + 0, static_cast<const unsigned long long *>(item_count.p), 1)
                         .add(h_q + 1, static_cast<const unsigned long long *>(rq_count.p), 1)
                         .add(h_q + 2, static_cast<const unsigned long long *>(cq_count.p), 1)
-                        .add(h_q + 5, static_cast<const unsigned long long *>(ctr.p), 7);
-                    if (mixed)
-                        job.add(h_q + 3, static_cast<const unsigned long long *>(cand_count.p), 1)
-                            .add(h_q + 4, static_cast<const unsigned long long *>(surv_count.p), 1);
+                        .add(h_q + 4, static_cast<const unsigned long long *>(surv_count.p), 1)
+                        .add(h_q + 5, static_cast<const unsigned long long *>(ctr.p), 8);
+                    if (mixed) job.add(h_q + 3, static_cast<const unsigned long long *>(cand_count.p), 1);
                     job.launch(st);
                     ++n_mbox;
                 }
@@ -1356,8 +1363,8 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 h_rq = h_q[1];
                 h_cq = h_q[2];
                 h_cand = mixed ? h_q[3] : 0;
-                h_surv = mixed ? h_q[4] : 0;
-                for (int k = 0; k < 7; ++k) h_ctr[k] = h_q[5 + k];
+                h_surv = h_q[4];
+                for (int k = 0; k < 8; ++k) h_ctr[k] = h_q[5 + k];
                 tr.mark("narrow phase and root finding run",
                         std::to_string(h_items) + " items, " + std::to_string(h_rq) + " root items, "
                             + std::to_string(h_cq) + " conjunctions");
@@ -1366,12 +1373,9 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 t_rt += ev[5].ms();
                 bool again = false;
                 if (h_items > (mixed ? cand.n : items.n)) {
-                    if (mixed) {
-                        cand.alloc_queue(h_items + h_items / 4, st);
-                        surv.alloc_queue(cand.n, st);
-                    } else {
-                        items.alloc_queue(h_items + h_items / 4, st);
-                    }
+                    dbuf<np_item> &q = mixed ? cand : items;
+                    q.alloc_queue(h_items + h_items / 4, st);
+                    surv.alloc_queue(q.n, st);
                     again = true;
                 }
                 if (h_rq > rq.n) {
@@ -1391,8 +1395,12 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 conj_per_pair = std::max(conj_per_pair, double(h_cq) / double(np_batch));
             }
             for (int k = 0; k < 7; ++k) R.np[k] += h_ctr[k];
-            R.narrow_split[0] += h_cand;
-            R.narrow_split[1] += h_surv;
+            if (mixed) {
+                // Past the filter's enclosure: left to the reference
+                // formulation or settled as a single minimum.
+                R.narrow_split[0] += h_cand;
+                R.narrow_split[1] += h_surv + h_ctr[7];
+            }
             // Per-step ordering, appended to the result.
             if (cgrp.n < h_cq) cgrp.alloc(h_cq, st);
             if (R.conj.n < R.n_conj + h_cq)
