@@ -10,14 +10,15 @@
 // bisects the step while the error is 1e-7 km or more (steps under 5 s are
 // accepted as they are; more than 20 polynomials in one step is an error).
 //
-// Near-Earth and deep-space element sets alike (sgp4.cuh).  Here one warp
-// runs one (satellite, element set) span: lanes 0..18 evaluate
-// SGP4 at the 19 nodes (and then at the 19 midpoints) of a step in parallel,
-// lanes 0..6 interpolate one state variable each, and the bisection stack
-// lives in the warp's shared memory.  Accepted polynomials are appended to a
-// pool (one atomic per polynomial) with their (span, sequence) tags; a
-// gather pass lays the pool out as the polyjectory's trajectory and time
-// arrays.
+// Near-Earth and deep-space element sets alike (sgp4.cuh).  The steps of a span
+// do not depend on its polynomials, so the work is laid out by what is
+// independent: one thread per span finds its steps (k_sgp4_steps); then every
+// step of every span is interpolated and checked at once, one thread per node
+// and midpoint, packed without idle lanes (k_sgp4_interp); the few steps that
+// need bisection or end in an error go through the reference's procedure one
+// warp per step (k_sgp4_bisect), which also yields its exact status.  A pass
+// over each span's steps numbers its polynomials up to the first failure, and
+// a gather lays them out as the polyjectory's trajectory and time arrays.
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -25,6 +26,7 @@
 #include <string>
 #include <vector>
 
+#include "block.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "sgp4pj.cuh"
@@ -39,9 +41,18 @@ constexpr int STACK = 40;
 constexpr int MAX_POLYS = 20;                  // make_sgp4_polyjectory.cpp:495-502
 constexpr double MIN_STEP = 5.0 / 86400.0;     // days, make_sgp4_polyjectory.cpp:487
 constexpr double ERR_THRESH = 1e-7;            // km, make_sgp4_polyjectory.cpp:490
+constexpr uint32_t NOT_KEPT = 0xffffffffu;
 
+// One step of a span: [b, e) in days from the polyjectory epoch, [bs, es) the
+// same instants from the element set's epoch; the k-th of its job.
+struct step_rec {
+    double b, e, bs, es;
+    uint32_t job, k;
+};
+
+// One accepted polynomial: number `seq` of step `step`, over [t0, t1).
 struct seg_rec {
-    uint32_t job, seq;
+    uint32_t step, seq;
     double t0, t1;
 };
 
@@ -204,110 +215,298 @@ __device__ int interpolate_step(const sgp4::sat &sat, const nodes_t &nd, double 
     return 0;
 }
 
-// Each warp takes the next job of `order` (the jobs by decreasing expected
-// work: mean motion times span) from the counter *next until none is left,
-// so that the long low-orbit spans start first and the short ones fill in
-// at the end, and warps of one SM tend to run the same propagator branch.
-__global__ void __launch_bounds__(32 * WARPS, 4) k_sgp4_pj(const job *__restrict__ jobs, uint32_t n_jobs,
-                                                        const uint32_t *__restrict__ order, uint32_t *next,
-                                                        dfl pj_epoch, double reentry, double exit_r, nodes_t nd,
-                                                        double *__restrict__ pool, seg_rec *__restrict__ recs,
-                                                        uint64_t cap, unsigned long long *pool_count, int *overflow,
-                                                        int *__restrict__ job_status,
-                                                        uint32_t *__restrict__ job_committed, uint64_t max_steps)
+// Set-up of every element set, once (its coefficients are read by all of its
+// propagations); init[j] is the set-up's error code.
+__global__ void __launch_bounds__(64) k_sgp4_setup(const job *__restrict__ jobs, uint32_t n, sgp4::sat *sats,
+                                                   int *__restrict__ init)
+{
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const job J = jobs[j];
+    init[j] = sgp4::setup(J.n0, J.e0, J.i0, J.node0, J.omega0, J.m0, J.bstar, J.epoch1950, sats[j]);
+}
+
+// The steps of every span, one thread per span in the sequence `order` (the
+// jobs by decreasing expected work, so that the lanes of a warp take about as
+// many steps).  A serial chain of one propagation and one Taylor step size
+// per step: bound by its latency, and short against the interpolation
+// (MEASURED_S).  n_steps[j] steps are appended to `out` in any order, end[j]
+// is the status that ended them (0: the span's end).
+__global__ void __launch_bounds__(32) k_sgp4_steps(const job *__restrict__ jobs, uint32_t n_jobs,
+                                                   const uint32_t *__restrict__ order, const sgp4::sat *sats,
+                                                   const int *__restrict__ init, dfl pj_epoch, double reentry,
+                                                   double exit_r, uint64_t max_steps, step_rec *__restrict__ out,
+                                                   uint64_t cap, unsigned long long *count,
+                                                   uint32_t *__restrict__ n_steps, int *__restrict__ end)
+{
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n_jobs) return;
+    const uint32_t jb = order[q];
+    const job J = jobs[jb];
+    const sgp4::sat &sat = sats[jb];
+    int st = init[jb];
+    uint32_t k = 0;
+    dfl cur = J.begin_tai;
+    // Every step but the last is at least 1 s long, so max_steps bounds the
+    // loop; reaching it reports the small-step status.
+    for (uint64_t it = 0; st == 0; ++it) {
+        if (it >= max_steps) {
+            st = ST_SMALL_STEP;
+            break;
+        }
+        const double step_begin = dfl_sub(cur, pj_epoch).hi;
+        const dfl sb_s = dfl_sub(cur, J.epoch_tai);
+        double r[3], v[3];
+        const int e = sgp4::propagate(sat, sb_s.hi * 1440., r, v);
+        if (e) {
+            st = e;
+            break;
+        }
+        const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        if (r2 < reentry * reentry) {
+            st = ST_REENTRY;
+            break;
+        }
+        if (r2 >= exit_r * exit_r) {
+            st = ST_EXIT;
+            break;
+        }
+        const double hmax = dfl_sub(J.end_tai, cur).hi * 86400.;
+        double h = kepler_step(r, v);
+        bool last = false;
+        if (!isfinite(h)) {
+            st = ST_NONFINITE;
+            break;
+        }
+        if (h >= hmax) {
+            h = hmax;
+            last = true;
+        } else if (h < 1.) {
+            st = ST_SMALL_STEP;
+            break;
+        }
+        const unsigned long long slot = atomicAdd(count, 1ull);
+        if (slot < cap)
+            out[slot] = step_rec{step_begin, step_begin + h / 86400., sb_s.hi, dfl_add(sb_s, h / 86400.).hi, jb, k};
+        ++k;
+        if (last) break;
+        cur = dfl_add(cur, h / 86400.);
+    }
+    n_steps[jb] = k;
+    end[jb] = st;
+}
+
+// First step of every job when the steps stand job by job in the sequence
+// `order` (one block).
+__global__ void __launch_bounds__(1024) k_sgp4_bases(const uint32_t *__restrict__ order, uint32_t n_jobs,
+                                                     const uint32_t *__restrict__ n_steps, uint32_t *__restrict__ base)
+{
+    __shared__ uint32_t sm[33];
+    uint32_t carry = 0;
+    for (uint32_t q0 = 0; q0 < n_jobs; q0 += blockDim.x) {
+        const uint32_t q = q0 + threadIdx.x;
+        const uint32_t jb = q < n_jobs ? order[q] : 0;
+        uint32_t tot;
+        const uint32_t ex = block_excl_scan(q < n_jobs ? n_steps[jb] : 0, sm, &tot);
+        if (q < n_jobs) base[jb] = carry + ex;
+        carry += tot;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sgp4_place(const step_rec *__restrict__ in, uint64_t n,
+                                                    const uint32_t *__restrict__ base, step_rec *__restrict__ out)
+{
+    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    if (g >= n) return;
+    const step_rec r = in[g];
+    out[base[r.job] + r.k] = r;
+}
+
+// Interpolation and error check of INTERP_STEPS steps by one CTA
+// (make_sgp4_polyjectory.cpp:478-700 without the bisection): thread (s, m)
+// propagates step s to node m, thread (s, v) interpolates variable v of step
+// s, thread (s, m) compares the interpolant with SGP4 halfway to node m.
+// An accepted step's polynomial goes to the pool slot of its own number; the
+// others are listed for k_sgp4_bisect.
+//
+// Bound by instruction issue and fetch of the propagator (FP64 and the
+// transcendental functions around it).  With 8 steps a CTA 152 of 160 lanes
+// propagate; a warp per step had 19 of 32, computed the step size in all of
+// them and interpolated with 7 (23.7 ms for 6,000 element sets over 6 hours,
+// MEASURED_I).
+constexpr int INTERP_STEPS = 8;
+constexpr int INTERP_T = 160;
+static_assert(INTERP_STEPS * OP1 <= INTERP_T, "one thread per node");
+
+__global__ void __launch_bounds__(INTERP_T) k_sgp4_interp(const step_rec *__restrict__ steps, uint64_t n_steps,
+                                                          const sgp4::sat *sats, nodes_t nd,
+                                                          double *__restrict__ pool, seg_rec *__restrict__ recs,
+                                                          uint32_t *__restrict__ n_polys,
+                                                          uint32_t *__restrict__ redo, unsigned long long *n_redo)
+{
+    __shared__ double f[INTERP_STEPS][OP1][7]; // node values, then coefficients
+    __shared__ double al[INTERP_STEPS][OP1], cn[OP1];
+    __shared__ step_rec sr[INTERP_STEPS];
+    __shared__ int bad[INTERP_STEPS];
+    const unsigned tid = threadIdx.x;
+    const uint64_t first = blockIdx.x * uint64_t(INTERP_STEPS);
+    const unsigned n = unsigned(n_steps - first < INTERP_STEPS ? n_steps - first : INTERP_STEPS);
+    if (tid < OP1) cn[tid] = nd.c[tid];
+    if (tid < n) {
+        const step_rec r = steps[first + tid];
+        sr[tid] = r;
+        bad[tid] = !isfinite(r.e - r.b) || !isfinite(r.es - r.bs);
+    }
+    __syncthreads();
+    const unsigned s = tid / OP1, m = tid % OP1;
+    const bool mine = s < n && !bad[s < n ? s : 0];
+    double b = 0, bs = 0, dur = 0, dur_s = 0;
+    const sgp4::sat *sat = sats;
+    if (mine) {
+        b = sr[s].b;
+        bs = sr[s].bs;
+        dur = sr[s].e - b;
+        dur_s = sr[s].es - bs;
+        sat = sats + sr[s].job;
+        al[s][m] = (cn[m] + 1) / 2 * dur;
+        double st[7];
+        if (state7(*sat, (cn[m] + 1) / 2 * (dur_s * 1440.) + bs * 1440., st)) bad[s] = 1;
+        for (int v = 0; v < 7; ++v) f[s][m][v] = st[v];
+    }
+    __syncthreads();
+    // Bjorck-Pereyra on the nodes of [0, dur], one variable per thread
+    // (vm_interp, mizuba/detail/poly_utils.cpp:467-535).
+    if (tid < n * 7) {
+        const unsigned u = tid / 7, v = tid % 7;
+        if (!bad[u]) {
+#pragma unroll 1
+            for (int k = 0; k < ORDER; ++k) {
+                double hi = f[u][ORDER][v];
+#pragma unroll 6
+                for (int j = ORDER; j > k; --j) {
+                    const double lo = f[u][j - 1][v];
+                    f[u][j][v] = (hi - lo) / (al[u][j] - al[u][j - k - 1]);
+                    hi = lo;
+                }
+            }
+#pragma unroll 1
+            for (int k = ORDER - 1; k >= 0; --k) {
+                const double ck = al[u][k];
+                double lo = f[u][k][v];
+#pragma unroll 6
+                for (int j = k; j < ORDER; ++j) {
+                    const double hi = f[u][j + 1][v];
+                    f[u][j][v] = lo - ck * hi;
+                    lo = hi;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // Position error halfway between the nodes (eval_interp_error2,
+    // make_sgp4_polyjectory.cpp:325-410).
+    if (mine && !bad[s] && !(dur < MIN_STEP)) {
+        const double a_cur = (cn[m] + 1) / 2 * dur;
+        const double a_prev = m == 0 ? 0. : (cn[m - 1] + 1) / 2 * dur;
+        const double ev = a_prev / 2 + a_cur / 2;
+        double xyz[3];
+        for (int v = 0; v < 3; ++v) {
+            double r = f[s][ORDER][v];
+            for (int o = 1; o <= ORDER; ++o) r = f[s][ORDER - o][v] + r * ev;
+            xyz[v] = r;
+        }
+        const double s_cur = (cn[m] + 1) / 2 * (dur_s * 1440.) + bs * 1440.;
+        const double s_prev = m == 0 ? bs * 1440. : (cn[m - 1] + 1) / 2 * (dur_s * 1440.) + bs * 1440.;
+        double st[7];
+        const int code = state7(*sat, s_prev / 2 + s_cur / 2, st);
+        const double dx = xyz[0] - st[0], dy = xyz[1] - st[1], dz = xyz[2] - st[2];
+        const double err2 = dx * dx + dy * dy + dz * dz;
+        if (code || !isfinite(err2) || !(err2 < ERR_THRESH * ERR_THRESH)) bad[s] = 1;
+    }
+    __syncthreads();
+    for (unsigned e = tid; e < n * (OP1 * 7); e += INTERP_T)
+        if (!bad[e / (OP1 * 7)]) pool[first * (OP1 * 7) + e] = (&f[0][0][0])[e];
+    if (tid < n) {
+        const uint32_t idx = uint32_t(first + tid);
+        recs[idx] = seg_rec{bad[tid] ? NOT_KEPT : idx, 0, sr[tid].b, sr[tid].e};
+        n_polys[idx] = bad[tid] ? 0 : 1;
+        if (bad[tid]) redo[atomicAdd(n_redo, 1ull)] = idx;
+    }
+}
+
+// The steps that k_sgp4_interp left, one warp per step: interpolation with
+// bisection as the reference does it, polynomials appended to the pool from
+// slot n_steps on.
+__global__ void __launch_bounds__(32 * WARPS, 4) k_sgp4_bisect(const step_rec *__restrict__ steps,
+                                                            const sgp4::sat *sats, nodes_t nd,
+                                                            const uint32_t *__restrict__ redo,
+                                                            const unsigned long long *n_redo,
+                                                            double *__restrict__ pool, seg_rec *__restrict__ recs,
+                                                            uint64_t cap, unsigned long long *pool_count,
+                                                            int *overflow, uint32_t *__restrict__ n_polys,
+                                                            int *__restrict__ status)
 {
     __shared__ warp_smem smem[WARPS];
     const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     warp_smem &S = smem[w];
-    for (;;) {
-        uint32_t kq = 0;
-        if (lane == 0) kq = atomicAdd(next, 1u);
-        kq = __shfl_sync(0xffffffffu, kq, 0);
-        if (kq >= n_jobs) break;
-        const uint32_t jb = order[kq];
-        const job J = jobs[jb];
-        int st = 0;
-        uint32_t committed = 0;
-        sgp4::sat sat;
-        st = sgp4::setup(J.n0, J.e0, J.i0, J.node0, J.omega0, J.m0, J.bstar, J.epoch1950, sat);
-        dfl cur = J.begin_tai;
-        // Every step but the last is at least 1 s long, so max_steps bounds
-        // the loop; reaching it reports the small-step status.
-        for (uint64_t it = 0; st == 0; ++it) {
-            if (it >= max_steps) {
-                st = ST_SMALL_STEP;
-                break;
-            }
-            const double step_begin = dfl_sub(cur, pj_epoch).hi;
-            const dfl sb_s = dfl_sub(cur, J.epoch_tai);
-            double r[3], v[3];
-            int e = sgp4::propagate(sat, sb_s.hi * 1440., r, v);
-            if (e) {
-                st = e;
-                break;
-            }
-            const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-            if (r2 < reentry * reentry) {
-                st = ST_REENTRY;
-                break;
-            }
-            if (r2 >= exit_r * exit_r) {
-                st = ST_EXIT;
-                break;
-            }
-            const double hmax = dfl_sub(J.end_tai, cur).hi * 86400.;
-            double h = kepler_step(r, v);
-            bool last = false;
-            if (!isfinite(h)) {
-                st = ST_NONFINITE;
-                break;
-            }
-            if (h >= hmax) {
-                h = hmax;
-                last = true;
-            } else if (h < 1.) {
-                st = ST_SMALL_STEP;
-                break;
-            }
-            const double step_end = step_begin + h / 86400.;
-            const double se_s = dfl_add(sb_s, h / 86400.).hi;
-            int n_acc = 0;
-            st = interpolate_step(sat, nd, step_begin, step_end, sb_s.hi, se_s, S, n_acc, pool, cap, pool_count,
-                                  overflow);
-            if (st) break;
-            // The step's polynomials in time order, tagged (span, sequence).
-            if (lane == 0) {
-                for (int a = 1; a < n_acc; ++a)
-                    for (int c = a; c > 0 && S.acc_t0[c] < S.acc_t0[c - 1]; --c) {
-                        const double t0 = S.acc_t0[c], t1 = S.acc_t1[c];
-                        const unsigned long long sl = S.acc_slot[c];
-                        S.acc_t0[c] = S.acc_t0[c - 1];
-                        S.acc_t1[c] = S.acc_t1[c - 1];
-                        S.acc_slot[c] = S.acc_slot[c - 1];
-                        S.acc_t0[c - 1] = t0;
-                        S.acc_t1[c - 1] = t1;
-                        S.acc_slot[c - 1] = sl;
-                    }
-                for (int a = 0; a < n_acc; ++a)
-                    if (S.acc_slot[a] < cap) recs[S.acc_slot[a]] = seg_rec{jb, committed + a, S.acc_t0[a], S.acc_t1[a]};
-            }
-            __syncwarp();
-            committed += uint32_t(n_acc);
-            if (last) break;
-            cur = dfl_add(cur, h / 86400.);
-        }
+    const uint64_t n = *n_redo;
+    for (uint64_t k = blockIdx.x * uint64_t(WARPS) + w; k < n; k += uint64_t(gridDim.x) * WARPS) {
+        const uint32_t idx = redo[k];
+        const step_rec r = steps[idx];
+        int n_acc = 0;
+        const int st = interpolate_step(sats[r.job], nd, r.b, r.e, r.bs, r.es, S, n_acc, pool, cap, pool_count,
+                                        overflow);
+        // The step's polynomials in time order.
         if (lane == 0) {
-            job_status[jb] = st;
-            job_committed[jb] = committed;
+            for (int a = 1; a < n_acc; ++a)
+                for (int c = a; c > 0 && S.acc_t0[c] < S.acc_t0[c - 1]; --c) {
+                    const double t0 = S.acc_t0[c], t1 = S.acc_t1[c];
+                    const unsigned long long sl = S.acc_slot[c];
+                    S.acc_t0[c] = S.acc_t0[c - 1];
+                    S.acc_t1[c] = S.acc_t1[c - 1];
+                    S.acc_slot[c] = S.acc_slot[c - 1];
+                    S.acc_t0[c - 1] = t0;
+                    S.acc_t1[c - 1] = t1;
+                    S.acc_slot[c - 1] = sl;
+                }
+            for (int a = 0; a < n_acc; ++a)
+                if (S.acc_slot[a] < cap)
+                    recs[S.acc_slot[a]] = seg_rec{idx, uint32_t(a), S.acc_t0[a], S.acc_t1[a]};
+            n_polys[idx] = uint32_t(n_acc);
+            status[idx] = st;
         }
         __syncwarp();
     }
 }
 
-// Lays the pool out as the polyjectory: segment dest = seg_base[job] + seq,
+// Numbers each span's polynomials up to its first failing step: step_seq[s]
+// is the number of step s's first polynomial, NOT_KEPT from the failure on.
+__global__ void __launch_bounds__(64) k_sgp4_number(uint32_t n_jobs, const uint32_t *__restrict__ base,
+                                                    const uint32_t *__restrict__ n_steps,
+                                                    const uint32_t *__restrict__ n_polys,
+                                                    const int *__restrict__ status, const int *__restrict__ end,
+                                                    uint32_t *__restrict__ step_seq, int *__restrict__ job_status,
+                                                    uint32_t *__restrict__ job_committed)
+{
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n_jobs) return;
+    const uint32_t b = base[j], e = b + n_steps[j];
+    uint32_t committed = 0;
+    int st = 0;
+    for (uint32_t s = b; s < e; ++s) {
+        if (st == 0) st = status[s];
+        step_seq[s] = st ? NOT_KEPT : committed;
+        if (st == 0) committed += n_polys[s];
+    }
+    job_status[j] = st ? st : end[j];
+    job_committed[j] = committed;
+}
+
+// Lays the pool out as the polyjectory: segment dest = seg_base[job] + number,
 // its coefficients (mizuba layout [order + 1][7]) and its end time; the
 // first segment of each satellite also writes the start time.
 __global__ void k_sgp4_gather(const double *__restrict__ pool, const seg_rec *__restrict__ recs, uint64_t n_slots,
+                              const step_rec *__restrict__ steps, const uint32_t *__restrict__ step_seq,
                               const uint64_t *__restrict__ seg_base, const uint32_t *__restrict__ keep,
                               const uint32_t *__restrict__ job_sat, const uint64_t *__restrict__ sat_seg_off,
                               const uint64_t *__restrict__ sat_time_off, double *__restrict__ traj,
@@ -318,15 +517,17 @@ __global__ void k_sgp4_gather(const double *__restrict__ pool, const seg_rec *__
          g += uint64_t(gridDim.x) * blockDim.x) {
         const uint64_t slot = g / per, k = g % per;
         const seg_rec rc = recs[slot];
-        if (rc.job == 0xffffffffu || rc.seq >= keep[rc.job]) continue;
-        const uint64_t dest = seg_base[rc.job] + rc.seq;
+        if (rc.step == NOT_KEPT) continue;
+        const uint32_t s0 = step_seq[rc.step], jb = steps[rc.step].job;
+        if (s0 == NOT_KEPT || s0 + rc.seq >= keep[jb]) continue;
+        const uint64_t dest = seg_base[jb] + s0 + rc.seq;
         const double v = pool[slot * per + k];
         // The polyjectory constructor's finiteness check (polyjectory.cpp:
         // 558-569), on the coefficients as they are laid out.
         if (!isfinite(v)) atomicMin(bad_seg, (unsigned long long)dest);
         traj[dest * per + k] = v;
         if (k == 0) {
-            const uint32_t sat = job_sat[rc.job];
+            const uint32_t sat = job_sat[jb];
             const uint64_t local = dest - sat_seg_off[sat];
             time[sat_time_off[sat] + local + 1] = rc.t1;
             if (local == 0) time[sat_time_off[sat]] = rc.t0;
@@ -334,19 +535,30 @@ __global__ void k_sgp4_gather(const double *__restrict__ pool, const seg_rec *__
     }
 }
 
-__global__ void k_sgp4_propagate(const job *__restrict__ jobs, uint64_t n, const double *__restrict__ tsince,
-                                 uint64_t n_t, double *__restrict__ out, int *__restrict__ err)
+// Every element set at every time, one thread per propagation; consecutive
+// threads take consecutive times of one set and so read its coefficients
+// together.
+__global__ void __launch_bounds__(128) k_sgp4_propagate(const sgp4::sat *sats, const int *__restrict__ init,
+                                                        uint64_t n, const double *__restrict__ tsince, uint64_t n_t,
+                                                        double *__restrict__ out, int *__restrict__ err)
 {
-    for (uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; g < n * n_t;
-         g += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t i = g / n_t, t = g % n_t;
-        const job J = jobs[i];
-        double *o = out + g * 6;
-        sgp4::sat sat;
-        int e = sgp4::setup(J.n0, J.e0, J.i0, J.node0, J.omega0, J.m0, J.bstar, J.epoch1950, sat);
-        if (e == 0) e = sgp4::propagate(sat, tsince[t], o, o + 3);
-        err[g] = e;
+    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    if (g >= n * n_t) return;
+    const uint64_t i = g / n_t, t = g % n_t;
+    int e = init[i];
+    if (e == 0) {
+        double r[3], v[3];
+        e = sgp4::propagate(sats[i], tsince[t], r, v);
+        // Decay (6) has a state; the other errors come before there is one.
+        if (e == 0 || e == 6) {
+            double *o = out + g * 6;
+            for (int k = 0; k < 3; ++k) {
+                o[k] = r[k];
+                o[3 + k] = v[k];
+            }
+        }
     }
+    err[g] = e;
 }
 
 } // namespace sgp4pj
@@ -366,6 +578,8 @@ namespace
         if (e_ != cudaSuccess) sgp4_cuda_fail(e_, #x);                                                                 \
     } while (0)
 
+// A device buffer from the stream-ordered pool, on the legacy default stream
+// (all of this file's work is on it).
 template <typename T>
 struct devbuf {
     T *p = nullptr;
@@ -374,16 +588,19 @@ struct devbuf {
     explicit devbuf(size_t count) { alloc(count); }
     devbuf(const devbuf &) = delete;
     devbuf &operator=(const devbuf &) = delete;
-    ~devbuf()
+    ~devbuf() { release(); }
+    void release()
     {
-        if (p) cudaFree(p);
+        if (p) cudaFreeAsync(p, 0);
+        p = nullptr;
+        n = 0;
     }
     void alloc(size_t count)
     {
-        if (p) cudaFree(p);
-        p = nullptr;
+        release();
+        ensure_device_pool();
+        if (count) SK(cudaMallocAsync(reinterpret_cast<void **>(&p), count * sizeof(T), 0));
         n = count;
-        if (count) SK(cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T)));
     }
 };
 
@@ -557,19 +774,23 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
         const double wb = jobs[b].n0 * dfl_sub(jobs[b].end_tai, jobs[b].begin_tai).hi;
         return wa > wb;
     });
-    devbuf<uint32_t> d_order(n_jobs), d_next(1);
+    devbuf<uint32_t> d_order(n_jobs);
     SK(cudaMemcpy(d_order.p, order.data(), n_jobs * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    devbuf<int> d_status(n_jobs), d_overflow(1);
-    devbuf<uint32_t> d_committed(n_jobs);
-    devbuf<unsigned long long> d_count(1);
+    devbuf<sgp4::sat> d_sats(n_jobs);
+    devbuf<int> d_init(n_jobs), d_end(n_jobs), d_status(n_jobs), d_overflow(1);
+    devbuf<uint32_t> d_nsteps(n_jobs), d_base(n_jobs), d_committed(n_jobs);
+    devbuf<unsigned long long> d_count(1), d_nredo(1);
     const double span_s = (jd_end - jd_begin) * 86400.0;
     const uint64_t max_steps = uint64_t(span_s) + 16;
-    // Pool capacity: about 150 steps a day per span for low orbits, grown
-    // and rerun on overflow.
+    // Room for about 150 steps a day per span for low orbits, grown and run
+    // again when it is not enough.
     uint64_t cap = uint64_t(n_jobs) * 64 + uint64_t(std::ceil(std::max(1.0, jd_end - jd_begin)) * 160.0) * n_sats;
+    devbuf<step_rec> found, steps;
     devbuf<double> pool;
     devbuf<seg_rec> recs;
-    unsigned long long count = 0;
+    devbuf<uint32_t> n_polys, redo, step_seq;
+    devbuf<int> step_status;
+    unsigned long long n_steps = 0, count = 0;
     int dev = 0, n_sm = 148;
     SK(cudaGetDevice(&dev));
     SK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
@@ -592,29 +813,62 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
             return t;
         }
     } ev_k, ev_g;
+    SK(cudaEventRecord(ev_k.a));
+    k_sgp4_setup<<<(n_jobs + 63) / 64, 64>>>(d_jobs.p, n_jobs, d_sats.p, d_init.p);
+    ++out->n_launches;
     for (;;) {
+        found.alloc(cap);
+        SK(cudaMemsetAsync(d_count.p, 0, sizeof(unsigned long long)));
+        k_sgp4_steps<<<(n_jobs + 31) / 32, 32>>>(d_jobs.p, n_jobs, d_order.p, d_sats.p, d_init.p, out->epoch,
+                                                 reentry, exit_r, max_steps, found.p, cap, d_count.p, d_nsteps.p,
+                                                 d_end.p);
+        ++out->n_launches;
+        SK(cudaGetLastError());
+        SK(cudaMemcpy(&n_steps, d_count.p, sizeof(n_steps), cudaMemcpyDeviceToHost));
+        if (n_steps <= cap) break;
+        cap = n_steps;
+    }
+    if (n_steps >= NOT_KEPT) throw std::runtime_error("too many interpolation steps in make_sgp4_polyjectory()");
+    steps.alloc(n_steps);
+    n_polys.alloc(n_steps);
+    redo.alloc(n_steps);
+    step_seq.alloc(n_steps);
+    step_status.alloc(n_steps);
+    k_sgp4_bases<<<1, 1024>>>(d_order.p, n_jobs, d_nsteps.p, d_base.p);
+    if (n_steps) k_sgp4_place<<<unsigned((n_steps + 255) / 256), 256>>>(found.p, n_steps, d_base.p, steps.p);
+    out->n_launches += 2;
+    found.release();
+    // Pool: a slot per step, and room for the polynomials of bisected ones
+    // behind them.
+    cap = n_steps + n_steps / 8 + 4096;
+    for (; n_steps;) {
         pool.alloc(cap * OP1 * 7);
         recs.alloc(cap);
-        SK(cudaMemset(recs.p, 0xff, cap * sizeof(seg_rec)));
-        SK(cudaMemset(d_count.p, 0, sizeof(unsigned long long)));
-        SK(cudaMemset(d_overflow.p, 0, sizeof(int)));
-        SK(cudaMemset(d_next.p, 0, sizeof(uint32_t)));
-        const unsigned grid = unsigned(std::min<uint64_t>((n_jobs + WARPS - 1) / WARPS, uint64_t(n_sm) * 16));
-        SK(cudaEventRecord(ev_k.a));
-        k_sgp4_pj<<<grid, 32 * WARPS>>>(d_jobs.p, n_jobs, d_order.p, d_next.p, out->epoch, reentry, exit_r, nd, pool.p,
-                                          recs.p, cap,
-                                          d_count.p, d_overflow.p, d_status.p, d_committed.p, max_steps);
-        SK(cudaEventRecord(ev_k.b));
-        ++out->n_launches;
+        SK(cudaMemcpyAsync(d_count.p, &n_steps, sizeof(n_steps), cudaMemcpyHostToDevice, 0));
+        SK(cudaMemsetAsync(d_overflow.p, 0, sizeof(int)));
+        SK(cudaMemsetAsync(d_nredo.p, 0, sizeof(unsigned long long)));
+        SK(cudaMemsetAsync(step_status.p, 0, n_steps * sizeof(int)));
+        k_sgp4_interp<<<unsigned((n_steps + INTERP_STEPS - 1) / INTERP_STEPS), INTERP_T>>>(
+            steps.p, n_steps, d_sats.p, nd, pool.p, recs.p, n_polys.p, redo.p, d_nredo.p);
+        // Every polynomial of a step, the ones of a step that fails in the
+        // end included, takes a slot.
+        k_sgp4_bisect<<<n_sm * 4, 32 * WARPS>>>(steps.p, d_sats.p, nd, redo.p, d_nredo.p, pool.p, recs.p, cap,
+                                                 d_count.p, d_overflow.p, n_polys.p, step_status.p);
+        out->n_launches += 2;
         SK(cudaGetLastError());
         SK(cudaMemcpy(&count, d_count.p, sizeof(count), cudaMemcpyDeviceToHost));
         if (count <= cap) break;
         cap = count + count / 8 + 1024;
     }
-    out->kernel_ms = ev_k.ms();
+    k_sgp4_number<<<(n_jobs + 63) / 64, 64>>>(n_jobs, d_base.p, d_nsteps.p, n_polys.p, step_status.p, d_end.p,
+                                              step_seq.p, d_status.p, d_committed.p);
+    ++out->n_launches;
+    SK(cudaEventRecord(ev_k.b));
+    SK(cudaGetLastError());
     std::vector<int> status(n_jobs);
     std::vector<uint32_t> committed(n_jobs);
     SK(cudaMemcpy(status.data(), d_status.p, n_jobs * sizeof(int), cudaMemcpyDeviceToHost));
+    out->kernel_ms = ev_k.ms();
     SK(cudaMemcpy(committed.data(), d_committed.p, n_jobs * sizeof(uint32_t), cudaMemcpyDeviceToHost));
     // Per satellite: its spans in order up to the first that failed (the
     // failing span keeps the steps completed before the error).
@@ -653,14 +907,17 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
     SK(cudaMemcpy(d_sat_seg_off.p, sat_seg_off.data(), n_sats * 8, cudaMemcpyHostToDevice));
     SK(cudaMemcpy(d_sat_time_off.p, sat_time_off.data(), n_sats * 8, cudaMemcpyHostToDevice));
     out->n_traj = seg_cursor * OP1 * 7;
-    if (out->n_traj) SK(cudaMalloc(reinterpret_cast<void **>(&out->d_traj), out->n_traj * sizeof(double)));
+    out->dev = dev;
+    if (out->n_traj)
+        SK(cudaMallocAsync(reinterpret_cast<void **>(&out->d_traj), out->n_traj * sizeof(double), 0));
     devbuf<double> d_time(time_cursor);
     devbuf<unsigned long long> d_bad(1);
     SK(cudaMemset(d_bad.p, 0xff, sizeof(unsigned long long)));
     if (seg_cursor) {
         SK(cudaEventRecord(ev_g.a));
-        k_sgp4_gather<<<n_sm * 8, 256>>>(pool.p, recs.p, count, d_seg_base.p, d_keep.p, d_job_sat.p,
-                                          d_sat_seg_off.p, d_sat_time_off.p, out->d_traj, d_time.p, d_bad.p);
+        k_sgp4_gather<<<n_sm * 8, 256>>>(pool.p, recs.p, count, steps.p, step_seq.p, d_seg_base.p, d_keep.p,
+                                          d_job_sat.p, d_sat_seg_off.p, d_sat_time_off.p, out->d_traj, d_time.p,
+                                          d_bad.p);
         SK(cudaEventRecord(ev_g.b));
         ++out->n_launches;
         SK(cudaGetLastError());
@@ -716,15 +973,31 @@ void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_
         J.bstar = g[i].bstar;
         J.epoch1950 = dfl_sub(dfl_norm(g[i].epoch_jd1, g[i].epoch_jd2), dfl{2433281.5, 0.0}).hi;
     }
+    // Outputs in this device's memory are written in place; others through a
+    // buffer.
+    int dev = 0;
+    SK(cudaGetDevice(&dev));
+    auto here = [dev](const void *p) {
+        cudaPointerAttributes pa{};
+        const bool ok = cudaPointerGetAttributes(&pa, p) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok && pa.type == cudaMemoryTypeDevice && pa.device == dev;
+    };
+    const bool out_here = here(out), err_here = here(err);
     devbuf<job> d_jobs(n);
-    devbuf<double> d_t(n_t), d_out(n * n_t * 6);
-    devbuf<int> d_err(n * n_t);
-    SK(cudaMemcpy(d_jobs.p, jobs.data(), n * sizeof(job), cudaMemcpyHostToDevice));
-    SK(cudaMemcpy(d_t.p, tsince, n_t * 8, cudaMemcpyDefault));
-    k_sgp4_propagate<<<148 * 8, 128>>>(d_jobs.p, n, d_t.p, n_t, d_out.p, d_err.p);
+    devbuf<sgp4::sat> d_sats(n);
+    devbuf<double> d_t(n_t), d_out(out_here ? 0 : n * n_t * 6);
+    devbuf<int> d_init(n), d_err(err_here ? 0 : n * n_t);
+    double *po = out_here ? out : d_out.p;
+    int *pe = err_here ? err : d_err.p;
+    SK(cudaMemcpyAsync(d_jobs.p, jobs.data(), n * sizeof(job), cudaMemcpyHostToDevice, 0));
+    SK(cudaMemcpyAsync(d_t.p, tsince, n_t * 8, cudaMemcpyDefault, 0));
+    k_sgp4_setup<<<unsigned((n + 63) / 64), 64>>>(d_jobs.p, uint32_t(n), d_sats.p, d_init.p);
+    k_sgp4_propagate<<<unsigned((n * n_t + 127) / 128), 128>>>(d_sats.p, d_init.p, n, d_t.p, n_t, po, pe);
     SK(cudaGetLastError());
-    SK(cudaMemcpy(out, d_out.p, n * n_t * 6 * 8, cudaMemcpyDefault));
-    SK(cudaMemcpy(err, d_err.p, n * n_t * 4, cudaMemcpyDefault));
+    if (!out_here) SK(cudaMemcpy(out, po, n * n_t * 6 * 8, cudaMemcpyDefault));
+    if (!err_here) SK(cudaMemcpy(err, pe, n * n_t * 4, cudaMemcpyDefault));
+    SK(cudaStreamSynchronize(0));
 }
 
 } // namespace sgp4pj

@@ -34,6 +34,9 @@ struct conj_out {
     uint32_t pad;
 };
 
+// Raises the release threshold of the current device's default memory pool
+// once (pipeline.cu).
+void ensure_device_pool();
 cudaError_t init_aabb_consts();
 cudaError_t measure_dfma_rate(double *per_second);
 cudaError_t init_narrow_consts();
@@ -135,9 +138,15 @@ struct sgp4_pj_out {
     sgp4_pj_out() = default;
     sgp4_pj_out(const sgp4_pj_out &) = delete;
     sgp4_pj_out &operator=(const sgp4_pj_out &) = delete;
+    int dev = 0; // the device of d_traj
     ~sgp4_pj_out()
     {
-        if (d_traj) cudaFree(d_traj);
+        if (!d_traj) return;
+        int cur = 0;
+        cudaGetDevice(&cur);
+        cudaSetDevice(dev);
+        cudaFreeAsync(d_traj, 0);
+        cudaSetDevice(cur);
     }
 };
 dfl utc_to_tai(dfl utc);

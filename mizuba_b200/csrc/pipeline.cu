@@ -75,6 +75,16 @@ void ensure_pool()
     });
 }
 
+} // namespace
+
+namespace mzb
+{
+void ensure_device_pool() { ensure_pool(); }
+} // namespace mzb
+
+namespace
+{
+
 // Batch scratch kept between screening calls, one set of blocks per device.
 // Every call allocates the same few dozen scratch buffers of a few GB in
 // total; drawn from the stream-ordered pool afresh each time, their changing
