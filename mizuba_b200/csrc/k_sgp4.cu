@@ -226,11 +226,22 @@ __global__ void __launch_bounds__(64) k_sgp4_setup(const job *__restrict__ jobs,
     init[j] = sgp4::setup(J.n0, J.e0, J.i0, J.node0, J.omega0, J.m0, J.bstar, J.epoch1950, sats[j]);
 }
 
+__global__ void __launch_bounds__(64) k_sgp4_setup_gpes(const gpe_host *__restrict__ gpes, uint64_t n,
+                                                        sgp4::sat *sats, int *__restrict__ init)
+{
+    const uint64_t j = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    if (j >= n) return;
+    const gpe_host g = gpes[j];
+    const double epoch1950 = dfl_sub(dfl_norm(g.epoch_jd1, g.epoch_jd2), dfl{2433281.5, 0.0}).hi;
+    init[j] = sgp4::setup(g.n0, g.e0, g.i0, g.node0, g.omega0, g.m0, g.bstar, epoch1950, sats[j]);
+}
+
 // The steps of every span, one thread per span in the sequence `order` (the
 // jobs by decreasing expected work, so that the lanes of a warp take about as
 // many steps).  A serial chain of one propagation and one Taylor step size
 // per step: bound by its latency, and short against the interpolation
-// (MEASURED_S).  n_steps[j] steps are appended to `out` in any order, end[j]
+// (1.2 of 4.1 ms of kernels for 6,000 element sets over 6 hours; 2.7 ms with
+// the step size's Taylor coefficients in local memory instead of registers).  n_steps[j] steps are appended to `out` in any order, end[j]
 // is the status that ended them (0: the span's end).
 __global__ void __launch_bounds__(32) k_sgp4_steps(const job *__restrict__ jobs, uint32_t n_jobs,
                                                    const uint32_t *__restrict__ order, const sgp4::sat *sats,
@@ -329,16 +340,18 @@ __global__ void __launch_bounds__(256) k_sgp4_place(const step_rec *__restrict__
 // An accepted step's polynomial goes to the pool slot of its own number; the
 // others are listed for k_sgp4_bisect.
 //
-// Bound by instruction issue and fetch of the propagator (FP64 and the
-// transcendental functions around it).  With 8 steps a CTA 152 of 160 lanes
-// propagate; a warp per step had 19 of 32, computed the step size in all of
-// them and interpolated with 7 (23.7 ms for 6,000 element sets over 6 hours,
-// MEASURED_I).
+// Bound by the latency of the propagator (FP64 and the transcendental
+// functions around it), so residency counts more than registers: 3.3 ms at two
+// CTAs an SM (154 registers), 1.8 at four, 1.7 at five (72), for 6,000
+// element sets over 6 hours.  With 8 steps a CTA 152 of 160 lanes propagate; a
+// warp per step had 19 of 32, computed the step size in all of them and
+// interpolated with 7 (23.7 ms, step sizes included; the day of every third of
+// the 26,389 sets of a catalogue 155 -> 35 ms).
 constexpr int INTERP_STEPS = 8;
 constexpr int INTERP_T = 160;
 static_assert(INTERP_STEPS * OP1 <= INTERP_T, "one thread per node");
 
-__global__ void __launch_bounds__(INTERP_T) k_sgp4_interp(const step_rec *__restrict__ steps, uint64_t n_steps,
+__global__ void __launch_bounds__(INTERP_T, 5) k_sgp4_interp(const step_rec *__restrict__ steps, uint64_t n_steps,
                                                           const sgp4::sat *sats, nodes_t nd,
                                                           double *__restrict__ pool, seg_rec *__restrict__ recs,
                                                           uint32_t *__restrict__ n_polys,
@@ -502,8 +515,8 @@ __global__ void __launch_bounds__(64) k_sgp4_number(uint32_t n_jobs, const uint3
     job_committed[j] = committed;
 }
 
-// Lays the pool out as the polyjectory: segment dest = seg_base[job] + number,
-// its coefficients (mizuba layout [order + 1][7]) and its end time; the
+// Lays the pool out as the polyjectory, one warp per polynomial: segment
+// dest = seg_base[job] + number, its coefficients (mizuba layout [order + 1][7]) and its end time; the
 // first segment of each satellite also writes the start time.
 __global__ void k_sgp4_gather(const double *__restrict__ pool, const seg_rec *__restrict__ recs, uint64_t n_slots,
                               const step_rec *__restrict__ steps, const uint32_t *__restrict__ step_seq,
@@ -512,21 +525,25 @@ __global__ void k_sgp4_gather(const double *__restrict__ pool, const seg_rec *__
                               const uint64_t *__restrict__ sat_time_off, double *__restrict__ traj,
                               double *__restrict__ time, unsigned long long *bad_seg)
 {
-    const uint64_t per = uint64_t(OP1) * 7;
-    for (uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; g < n_slots * per;
-         g += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t slot = g / per, k = g % per;
+    constexpr unsigned per = OP1 * 7;
+    const unsigned lane = threadIdx.x & 31;
+    for (uint64_t slot = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; slot < n_slots;
+         slot += (uint64_t(gridDim.x) * blockDim.x) >> 5) {
         const seg_rec rc = recs[slot];
         if (rc.step == NOT_KEPT) continue;
         const uint32_t s0 = step_seq[rc.step], jb = steps[rc.step].job;
         if (s0 == NOT_KEPT || s0 + rc.seq >= keep[jb]) continue;
         const uint64_t dest = seg_base[jb] + s0 + rc.seq;
-        const double v = pool[slot * per + k];
         // The polyjectory constructor's finiteness check (polyjectory.cpp:
         // 558-569), on the coefficients as they are laid out.
-        if (!isfinite(v)) atomicMin(bad_seg, (unsigned long long)dest);
-        traj[dest * per + k] = v;
-        if (k == 0) {
+        bool finite = true;
+        for (unsigned k = lane; k < per; k += 32) {
+            const double v = pool[slot * per + k];
+            finite = finite && isfinite(v);
+            traj[dest * per + k] = v;
+        }
+        if (!finite) atomicMin(bad_seg, (unsigned long long)dest);
+        if (lane == 0) {
             const uint32_t sat = job_sat[jb];
             const uint64_t local = dest - sat_seg_off[sat];
             time[sat_time_off[sat] + local + 1] = rc.t1;
@@ -961,20 +978,8 @@ void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_
     for (uint64_t k = 0; k < n_t; ++k)
         if (!std::isfinite(ht[k]))
             throw std::invalid_argument("A non-finite propagation time was passed to mzb_sgp4_propagate()");
-    std::vector<job> jobs(n);
-    for (uint64_t i = 0; i < n; ++i) {
-        job &J = jobs[i];
-        J.n0 = g[i].n0;
-        J.e0 = g[i].e0;
-        J.i0 = g[i].i0;
-        J.node0 = g[i].node0;
-        J.omega0 = g[i].omega0;
-        J.m0 = g[i].m0;
-        J.bstar = g[i].bstar;
-        J.epoch1950 = dfl_sub(dfl_norm(g[i].epoch_jd1, g[i].epoch_jd2), dfl{2433281.5, 0.0}).hi;
-    }
-    // Outputs in this device's memory are written in place; others through a
-    // buffer.
+    // Arrays in this device's memory are read and written in place; others
+    // through buffers.
     int dev = 0;
     SK(cudaGetDevice(&dev));
     auto here = [dev](const void *p) {
@@ -983,17 +988,18 @@ void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_
         if (!ok) cudaGetLastError();
         return ok && pa.type == cudaMemoryTypeDevice && pa.device == dev;
     };
-    const bool out_here = here(out), err_here = here(err);
-    devbuf<job> d_jobs(n);
+    const bool g_here = here(g), t_here = here(tsince), out_here = here(out), err_here = here(err);
+    devbuf<gpe_host> d_g(g_here ? 0 : n);
     devbuf<sgp4::sat> d_sats(n);
-    devbuf<double> d_t(n_t), d_out(out_here ? 0 : n * n_t * 6);
+    devbuf<double> d_t(t_here ? 0 : n_t), d_out(out_here ? 0 : n * n_t * 6);
     devbuf<int> d_init(n), d_err(err_here ? 0 : n * n_t);
     double *po = out_here ? out : d_out.p;
     int *pe = err_here ? err : d_err.p;
-    SK(cudaMemcpyAsync(d_jobs.p, jobs.data(), n * sizeof(job), cudaMemcpyHostToDevice, 0));
-    SK(cudaMemcpyAsync(d_t.p, tsince, n_t * 8, cudaMemcpyDefault, 0));
-    k_sgp4_setup<<<unsigned((n + 63) / 64), 64>>>(d_jobs.p, uint32_t(n), d_sats.p, d_init.p);
-    k_sgp4_propagate<<<unsigned((n * n_t + 127) / 128), 128>>>(d_sats.p, d_init.p, n, d_t.p, n_t, po, pe);
+    if (!g_here) SK(cudaMemcpyAsync(d_g.p, g, n * sizeof(gpe_host), cudaMemcpyDefault, 0));
+    if (!t_here) SK(cudaMemcpyAsync(d_t.p, tsince, n_t * 8, cudaMemcpyDefault, 0));
+    k_sgp4_setup_gpes<<<unsigned((n + 63) / 64), 64>>>(g_here ? g : d_g.p, n, d_sats.p, d_init.p);
+    k_sgp4_propagate<<<unsigned((n * n_t + 127) / 128), 128>>>(d_sats.p, d_init.p, n, t_here ? tsince : d_t.p, n_t,
+                                                                po, pe);
     SK(cudaGetLastError());
     if (!out_here) SK(cudaMemcpy(out, po, n * n_t * 6 * 8, cudaMemcpyDefault));
     if (!err_here) SK(cudaMemcpy(err, pe, n * n_t * 4, cudaMemcpyDefault));

@@ -2224,11 +2224,7 @@ void mzb_sgp4_pj_timing(const mzb_sgp4_pj *p, double out[2])
 int mzb_sgp4_propagate(const mzb_gpe *gpes, uint64_t n_gpes, const double *tsince, uint64_t n_times, double *out,
                        int32_t *err)
 {
-    return guarded([&]() {
-        std::vector<mzb_gpe> keep;
-        const mzb_gpe *g = host_view(gpes, n_gpes, keep);
-        sgp4pj::sgp4_propagate(g, n_gpes, tsince, n_times, out, err);
-    });
+    return guarded([&]() { sgp4pj::sgp4_propagate(gpes, n_gpes, tsince, n_times, out, err); });
 }
 
 int mzb_sort_step_noalloc(const float *aabbs, const uint64_t *mcodes, uint64_t n_objs, uint32_t *srt_idx,

@@ -64,6 +64,18 @@ MZB_HD inline double xke() { return 60.0 / std::sqrt(RE * RE * RE / MU); }
 
 // One element set after set-up: the mean elements at epoch (un-Kozai mean
 // motion no) and the secular and drag terms SGP4 derives from them.
+// Sine and cosine of one argument: one call on the device, where the two
+// share the argument reduction (the same values as apart).
+MZB_HD inline void sc(double x, double &s, double &c)
+{
+#ifdef __CUDA_ARCH__
+    sincos(x, &s, &c);
+#else
+    s = std::sin(x);
+    c = std::cos(x);
+#endif
+}
+
 struct sat {
     double no, ecco, inclo, nodeo, argpo, mo, bstar;
     double mdot, argpdot, nodedot, nodecf, omgcof, xmcof, xlcof, aycof;
@@ -671,7 +683,8 @@ MZB_HD MZB_OUTLINE inline int propagate(const sat &s, double t, double r[3], dou
     mm = std::fmod(xlm - argpm - nodem, TWO_PI);
     // Long-period periodics (plus the lunar-solar ones in deep space).
     double ep = em, xincp = inclm, argpp = argpm, nodep = nodem, mp = mm;
-    double sinip = std::sin(inclm), cosip = std::cos(inclm);
+    double sinip, cosip;
+    sc(inclm, sinip, cosip);
     double aycof = s.aycof, xlcof = s.xlcof, con41 = s.con41, x1mth2 = s.x1mth2, x7thm1 = s.x7thm1;
     if (s.deep) {
         deep_periodics(s, t, ep, xincp, nodep, argpp, mp);
@@ -681,22 +694,22 @@ MZB_HD MZB_OUTLINE inline int propagate(const sat &s, double t, double r[3], dou
             argpp = argpp - TWO_PI / 2.0;
         }
         if (ep < 0.0 || ep > 1.0) return 3;
-        sinip = std::sin(xincp);
-        cosip = std::cos(xincp);
+        sc(xincp, sinip, cosip);
         aycof = -0.5 * (J3 / J2) * sinip;
         const double opc = (std::fabs(cosip + 1.0) > 1.5e-12) ? (1.0 + cosip) : 1.5e-12;
         xlcof = -0.25 * (J3 / J2) * sinip * (3.0 + 5.0 * cosip) / opc;
     }
-    const double axnl = ep * std::cos(argpp);
+    double sarg, carg;
+    sc(argpp, sarg, carg);
+    const double axnl = ep * carg;
     double temp = 1.0 / (am * (1.0 - ep * ep));
-    const double aynl = ep * std::sin(argpp) + temp * aycof;
+    const double aynl = ep * sarg + temp * aycof;
     const double xl = mp + argpp + nodep + temp * xlcof * axnl;
     // Kepler's equation for the modified eccentric anomaly.
     const double u = std::fmod(xl - nodep, TWO_PI);
     double eo1 = u, tem5 = 9999.9, sineo1 = 0.0, coseo1 = 0.0;
     for (int ktr = 1; std::fabs(tem5) >= 1.0e-12 && ktr <= 10; ++ktr) {
-        sineo1 = std::sin(eo1);
-        coseo1 = std::cos(eo1);
+        sc(eo1, sineo1, coseo1);
         tem5 = 1.0 - coseo1 * axnl - sineo1 * aynl;
         tem5 = (u - aynl * coseo1 + axnl * sineo1 - eo1) / tem5;
         if (std::fabs(tem5) >= 0.95) tem5 = tem5 > 0.0 ? 0.95 : -0.95;
@@ -734,9 +747,10 @@ MZB_HD MZB_OUTLINE inline int propagate(const sat &s, double t, double r[3], dou
     const double mvt = rdotl - nm * temp1 * x1mth2 * sin2u / k;
     const double rvdot = rvdotl + nm * temp1 * (x1mth2 * cos2u + 1.5 * con41) / k;
     // Orientation vectors.
-    const double sinsu = std::sin(su), cossu = std::cos(su);
-    const double snod = std::sin(xnode), cnod = std::cos(xnode);
-    const double sini = std::sin(xinc), cosi = std::cos(xinc);
+    double sinsu, cossu, snod, cnod, sini, cosi;
+    sc(su, sinsu, cossu);
+    sc(xnode, snod, cnod);
+    sc(xinc, sini, cosi);
     const double xmx = -snod * cosi, xmy = cnod * cosi;
     const double ux = xmx * sinsu + cnod * cossu;
     const double uy = xmy * sinsu + snod * cossu;

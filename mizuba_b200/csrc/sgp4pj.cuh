@@ -23,6 +23,13 @@
 
 #include "sgp4.cuh"
 
+// Loops whose arrays are to stay in registers on the device.
+#ifdef __CUDA_ARCH__
+#define MZB_UNROLL _Pragma("unroll")
+#else
+#define MZB_UNROLL
+#endif
+
 namespace mzb
 {
 namespace sgp4pj
@@ -80,28 +87,35 @@ MZB_HD MZB_OUTLINE inline double kepler_step(const double r[3], const double v[3
         V[i][0] = v[i];
     }
     const double alpha = -1.5;
+MZB_UNROLL
     for (int k = 0; k < ORDER; ++k) {
         // U = x.x and W = U^alpha, order k.
         double u = 0.0;
+MZB_UNROLL
         for (int i = 0; i < 3; ++i)
+MZB_UNROLL
             for (int j = 0; j <= k; ++j) u += X[i][j] * X[i][k - j];
         U[k] = u;
         if (k == 0) {
             W[0] = std::pow(U[0], alpha);
         } else {
             double w = 0.0;
+MZB_UNROLL
             for (int j = 0; j < k; ++j) w += (alpha * double(k - j) - double(j)) * U[k - j] * W[j];
             W[k] = w / (double(k) * U[0]);
         }
         // x' = v, v' = -mu x W.
+MZB_UNROLL
         for (int i = 0; i < 3; ++i) {
             double xw = 0.0;
+MZB_UNROLL
             for (int j = 0; j <= k; ++j) xw += X[i][j] * W[k - j];
             X[i][k + 1] = V[i][k] / double(k + 1);
             V[i][k + 1] = -MU_KEPLER * xw / double(k + 1);
         }
     }
     double s = 0.0, np = 0.0, npm1 = 0.0;
+MZB_UNROLL
     for (int i = 0; i < 3; ++i) {
         s = std::fmax(s, std::fmax(std::fabs(X[i][0]), std::fabs(V[i][0])));
         np = std::fmax(np, std::fmax(std::fabs(X[i][ORDER]), std::fabs(V[i][ORDER])));
