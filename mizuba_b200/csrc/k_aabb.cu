@@ -5,6 +5,7 @@
 // Reference: mizuba/detect_conjunctions_aabbs.cpp:64-398 and
 // mizuba/detect_conjunctions_morton.cpp:70-175.
 #include <algorithm>
+#include <cmath>
 #include <utility>
 
 #include "common.cuh"
@@ -169,9 +170,49 @@ void launch_relayout_runs(const char *piece, uint64_t n_runs, double *coef, int 
     k_relayout_runs<<<unsigned(blocks), 256, 0, stream>>>(piece, coef, op1, bad_seg);
 }
 
-// Cargo-Shisha box of one segment over [h_lb, h_ub] for x, y, z and r, widened
-// by the conjunction radius and rounded outward to float (aabbs.cpp:146-231),
-// folded into (lb, ub) with std::min / std::max semantics.
+// ------------------------------------------------------------------ boxes
+//
+// Two passes over the (step, object) pairs of the batch: the first overlapping
+// segment of every object (k_aabb), then the further segments of the objects
+// that have some in the step, from a queue (k_aabb_more), so that warps do
+// uniform work.  Both forms compute the enclosure with FMA-native
+// formulations: Taylor shift by synthetic division (n(n+1)/2 FMAs), scaling by
+// powers of delta, the binomial division replaced by a multiplication with
+// 1/C(n, i), and the Bernstein difference table.  The result differs from the
+// reference formulation's (binomial sums of products with powers, divisions:
+// segment_box) by rounding only; both are within (8n + 16) u P of the exact
+// Cargo-Shisha bounds, where P = sum_k |c_k| (a + delta)^k bounds every
+// intermediate magnitude (measured: at most 0.11 of that, at order 2; 0.06
+// from order 12 on).  With E = 2 (8n + 16) u P:
+//
+// * plain form: the reference's bound lies within E of the computed one (and
+//   the rounding of the subtraction of the radius), so when both ends of that
+//   interval round to the same float, that float is the reference's, bit for
+//   bit.  E is 1e-10 km against a float spacing of 5e-4 km: one bound in a
+//   million is not decided by it, and its object is recomputed with the
+//   reference formulation (as is any with a non-finite bound, so that the
+//   reference's errors are reported from the reference's values);
+// * mixed form: the bounds are widened by E before the outward float rounding,
+//   so that its boxes contain the plain form's, and the broad phase of the
+//   mixed form finds a superset of the plain form's overlapping pairs.
+//
+// Bound by the FP64 pipe once the coefficients arrive (four rows of 160 bytes
+// per object at order 18): loaded by each thread for itself, a 16-byte load of
+// a warp touched 32 lines and the load pipe was as busy as the FP64 pipe.  A
+// warp copies its objects' rows of one variable to shared memory together
+// (cp.async, consecutive lanes on consecutive bytes of a row), reads them back
+// at an odd stride of 16-byte units (conflict-free), and has the next
+// variable's copies in flight while it computes.
+// 20,000-object day (11.4 M boxes of four variables at order 18): plain form
+// 3.8 -> 2.1 ms (the reference formulation for every box took 1,018 FP64
+// operations a variable, this one 455), mixed form 2.5 -> 2.0 ms; 60 % of the
+// FP64 rate, the rest is latency at the start of a warp's work (segment
+// search, first rows).
+
+// Reference formulation: Cargo-Shisha box of one segment over [h_lb, h_ub] for
+// x, y, z and r, widened by the conjunction radius and rounded outward to
+// float (aabbs.cpp:146-231), folded into (lb, ub) with std::min / std::max
+// semantics.
 template <int OP1>
 __device__ __forceinline__ void segment_box(const double *__restrict__ cf, double h_lb, double h_ub, double radius,
                                             uint32_t obj, float *lb, float *ub, dev_status *st)
@@ -195,130 +236,113 @@ __device__ __forceinline__ void segment_box(const double *__restrict__ cf, doubl
     }
 }
 
-// Pass 1, one thread per (step, object): the first overlapping segment
-// (aabbs.cpp:64-252).  Objects with further overlapping segments in the step
-// are queued for pass 2, so that warps here do uniform work.
+// Reference box of object i over all its segments [tb, te) in the step.
 template <int OP1>
-__global__ void __launch_bounds__(128) k_aabb(dev_pj pj, const double2 *__restrict__ cd_bounds, uint32_t s_first,
-                                              uint32_t n_batch, double radius, float *__restrict__ aabbs,
-                                              uint2 *__restrict__ more, unsigned long long *more_count,
-                                              uint2 *__restrict__ srange, dev_status *st)
+__device__ __noinline__ void object_box(const dev_pj &pj, uint32_t i, double cb, double ce, uint32_t tb, uint32_t te,
+                                        double radius, float *lb, float *ub, dev_status *st)
 {
-    const uint64_t N = pj.n_objs;
-    const uint64_t gid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    const bool active = gid < N * n_batch;
-    const uint32_t b = active ? uint32_t(gid / N) : 0;
-    const uint64_t i = active ? gid % N : 0;
-    float lb[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-    float ub[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    bool queue = false;
-    if (active) {
-        const double2 cbe = cd_bounds[s_first + b];
-        const double cb = cbe.x, ce = cbe.y;
-        const uint32_t ns = pj.nseg[i];
-        uint2 rng = make_uint2(0, 0); // empty: no segment overlaps the step
-        if (ns > 0) {
-            const double *t = pj.time + pj.time_off[i];
-            if (!(t[0] >= ce || t[ns] <= cb)) {
-                uint32_t tb, te;
-                step_range(t, ns, cb, ce, tb, te);
-                rng = make_uint2(tb, te);
-                if (tb != te) {
-                    const uint32_t it = tb;
-                    const double s0 = t[it - 1];
-                    const double ev_lb = (cb < s0) ? s0 : cb;       // std::max(cb, s0)
-                    const double ev_ub = (t[it] < ce) ? t[it] : ce; // std::min(ce, t[it])
-                    segment_box<OP1>(coef_row<OP1>(pj, pj.seg_off[i] + it - 1, 0), ev_lb - s0, ev_ub - s0,
-                                     radius, uint32_t(i), lb, ub, st);
-                    queue = te - tb > 1;
-                }
+    const double *t = pj.time + pj.time_off[i];
+    for (int d = 0; d < 4; ++d) lb[d] = INFINITY, ub[d] = -INFINITY;
+    for (uint32_t it = tb; it != te; ++it) {
+        const double s0 = t[it - 1];
+        const double ev_lb = (cb < s0) ? s0 : cb;       // std::max(cb, s0)
+        const double ev_ub = (t[it] < ce) ? t[it] : ce; // std::min(ce, t[it])
+        segment_box<OP1>(coef_row<OP1>(pj, pj.seg_off[i] + it - 1, 0), ev_lb - s0, ev_ub - s0, radius, i, lb, ub,
+                         st);
+    }
+}
+
+// 1 / C(n, i), passed by value: constant operands of the scaling.
+struct inv_binoms {
+    double v[MAX_OP1];
+};
+static inv_binoms make_inv_binoms(int n)
+{
+    inv_binoms r{};
+    double c = 1.0;
+    for (int i = 0; i <= n; ++i) {
+        r.v[i] = 1.0 / c;
+        c = c * (n - i) / (i + 1);
+    }
+    return r;
+}
+
+constexpr int AABB_T = 128;
+constexpr int AABB_W = AABB_T / 32;
+
+template <int OP1>
+struct aabb_shape {
+    static constexpr int UNITS = row_ld(OP1) / 2; // 16-byte units of a row
+    static constexpr int STRIDE = UNITS | 1;      // odd: conflict-free 16-byte reads
+    static constexpr int GROUPS = 32 / UNITS;     // rows copied per instruction
+    // CTAs an SM: 80 registers a thread hold an order-18 table without
+    // spilling (day 2.12 ms; 2.18 at four CTAs, 118 registers).
+    static constexpr int CTAS = OP1 <= 20 ? 6 : OP1 <= 26 ? 4 : 3;
+};
+template <int OP1>
+struct aabb_smem {
+    double2 rows[32 * aabb_shape<OP1>::STRIDE];
+    const double2 *base[32];
+};
+
+// The boxes of one segment per lane, folded into (lb, ub), by the whole warp:
+// `first` is lane's segment (its first coefficient row), lanes with !act do no
+// folding.  SHIFT false: every h_lb is zero, the shift is the identity.
+// `unsure` (plain form) is set where the float bounds are not proven.
+//
+// With scr != nullptr (mixed form) the pass also writes the distance screen's
+// model of the portion (see screen_keeps): position and velocity at the
+// portion midpoint tm = (h_lb + h_ub) / 2 (FP32, rounded to nearest), and |A|
+// rounded up, where A_c = sum_k k (k - 1) |c_k| h_ub^(k-2) bounds |x_c''| on
+// [0, h_ub].
+template <int OP1, bool MIXED, bool SHIFT>
+__device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_binoms inv,
+                                                 const double *first, bool act, double h_lb, double h_ub,
+                                                 double radius, uint32_t obj, float4 &lb, float4 &ub, bool &unsure,
+                                                 dev_status *st, float4 *__restrict__ scr)
+{
+    using F = aabb_shape<OP1>;
+    constexpr int n = OP1 - 1;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned part = lane % F::UNITS, grp = lane / F::UNITS;
+    const unsigned dst0 = unsigned(__cvta_generic_to_shared(S.rows + grp * F::STRIDE + part));
+    auto fetch = [&](int v) {
+#pragma unroll
+        for (int k = 0; k < (32 + F::GROUPS - 1) / F::GROUPS; ++k) {
+            const unsigned r = grp + unsigned(k * F::GROUPS);
+            if (grp < F::GROUPS && r < 32) {
+                const double2 *src = S.base[r] + v * F::UNITS + part;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 dst0 + unsigned(k * F::GROUPS * F::STRIDE * 16)),
+                             "l"(src)
+                             : "memory");
             }
         }
-        float4 *o = reinterpret_cast<float4 *>(aabbs + ((uint64_t(s_first) + b) * (N + 1) + i) * 8);
-        o[0] = make_float4(lb[0], lb[1], lb[2], lb[3]);
-        o[1] = make_float4(ub[0], ub[1], ub[2], ub[3]);
-        srange[uint64_t(b) * N + i] = rng;
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, queue);
-    if (queue) {
-        const unsigned lane = threadIdx.x & 31;
-        const int leader = __ffs(mask) - 1;
-        unsigned long long base = 0;
-        if (int(lane) == leader) base = atomicAdd(more_count, (unsigned long long)__popc(mask));
-        base = __shfl_sync(mask, base, leader);
-        unsigned lt;
-        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        more[base + __popc(mask & lt)] = make_uint2(b, uint32_t(i));
-    }
-}
-
-// Pass 2: the remaining overlapping segments of the queued objects, in time
-// order, folded into the boxes written by pass 1 (persistent grid).
-template <int OP1>
-__global__ void __launch_bounds__(128) k_aabb_more(dev_pj pj, const double2 *__restrict__ cd_bounds,
-                                                   uint32_t s_first, double radius, float *__restrict__ aabbs,
-                                                   const uint2 *__restrict__ more,
-                                                   const unsigned long long *more_count, dev_status *st)
-{
-    const uint64_t N = pj.n_objs;
-    const uint64_t n = *more_count;
-    for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
-        const uint2 e = more[k];
-        const uint32_t b = e.x, i = e.y;
-        const double2 cbe = cd_bounds[s_first + b];
-        const double cb = cbe.x, ce = cbe.y;
-        const uint32_t ns = pj.nseg[i];
-        const double *t = pj.time + pj.time_off[i];
-        uint32_t tb, te;
-        step_range(t, ns, cb, ce, tb, te);
-        float4 *o = reinterpret_cast<float4 *>(aabbs + ((uint64_t(s_first) + b) * (N + 1) + i) * 8);
-        const float4 l0 = o[0], u0 = o[1];
-        float lb[4] = {l0.x, l0.y, l0.z, l0.w}, ub[4] = {u0.x, u0.y, u0.z, u0.w};
-        for (uint32_t it = tb + 1; it != te; ++it) {
-            const double s0 = t[it - 1];
-            const double ev_lb = (cb < s0) ? s0 : cb;
-            const double ev_ub = (t[it] < ce) ? t[it] : ce;
-            segment_box<OP1>(coef_row<OP1>(pj, pj.seg_off[i] + it - 1, 0), ev_lb - s0, ev_ub - s0, radius, i, lb,
-                             ub, st);
-        }
-        o[0] = make_float4(lb[0], lb[1], lb[2], lb[3]);
-        o[1] = make_float4(ub[0], ub[1], ub[2], ub[3]);
-    }
-}
-
-// ---------------------------------------------------------------- mixed form
-//
-// The same enclosure, computed with FMA-native formulations: Taylor shift by
-// synthetic division (n(n+1)/2 FMAs), scaling by powers of delta, the
-// binomial division replaced by a multiplication with 1/C(n, i), and the
-// Bernstein difference table.  The result differs from the plain form's by
-// rounding only; both are within E = (8n + 16) u P of the exact Cargo-Shisha
-// bounds, where P = sum_k |c_k| (a + delta)^k bounds every intermediate
-// magnitude.  Widening by 2E before the outward float rounding therefore
-// yields boxes that contain the plain form's boxes, so the broad phase of the
-// mixed form finds a superset of the plain form's overlapping pairs.
-//
-// With scr != nullptr the same pass also writes the distance screen's model
-// of the portion (see screen_keeps): position and velocity at the portion
-// midpoint tm = (h_lb + h_ub) / 2 (FP32, rounded to nearest), and |A| rounded
-// up, where A_c = sum_k k (k - 1) |c_k| h_ub^(k-2) bounds |x_c''| on [0, h_ub].
-template <int OP1>
-__device__ __forceinline__ void segment_box_mixed(const double *__restrict__ cf, const double *__restrict__ inv_binom,
-                                                  double h_lb, double h_ub, double radius, uint32_t obj, float *lb,
-                                                  float *ub, dev_status *st, float4 *__restrict__ scr)
-{
-    constexpr int n = OP1 - 1;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    S.base[lane] = reinterpret_cast<const double2 *>(first);
+    __syncwarp();
+    fetch(0);
     const double delta = h_ub - h_lb;
     const double span = h_lb + delta;
     const double tmr = (h_lb + h_ub) / 2;
-    float sp[3], sv[3];
+    float sp[3] = {0, 0, 0}, sv[3] = {0, 0, 0};
     double a2 = 0;
 #pragma unroll 1
     for (int d = 0; d < 4; ++d) {
-        const int v = (d == 3) ? 6 : d;
         double t[OP1];
-        load_row<OP1>(cf + v * row_ld(OP1), t);
-        if (scr && d < 3) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < OP1 / 2; ++k) {
+            const double2 v = S.rows[lane * F::STRIDE + k];
+            t[2 * k] = v.x;
+            t[2 * k + 1] = v.y;
+        }
+        if (OP1 & 1) t[OP1 - 1] = S.rows[lane * F::STRIDE + OP1 / 2].x;
+        __syncwarp(); // every row is in registers: the next ones may land
+        if (d < 3) fetch(d == 2 ? 6 : d + 1);
+        if (MIXED && scr && d < 3) {
             double p = t[n], dp = 0, acc = double(n) * (n - 1) * fabs(t[n]);
 #pragma unroll
             for (int k = n - 1; k >= 0; --k) {
@@ -326,23 +350,26 @@ __device__ __forceinline__ void segment_box_mixed(const double *__restrict__ cf,
                 p = fma(p, tmr, t[k]);
                 if (k >= 2) acc = fma(acc, h_ub, double(k) * (k - 1) * fabs(t[k]));
             }
-            sp[d] = __double2float_rn(p);
-            sv[d] = __double2float_rn(dp);
+            const float fp = __double2float_rn(p), fv = __double2float_rn(dp);
+            if (d == 0) sp[0] = fp, sv[0] = fv;
+            else if (d == 1) sp[1] = fp, sv[1] = fv;
+            else sp[2] = fp, sv[2] = fv;
             a2 = fma(acc, acc, a2);
         }
         // P = sum |c_k| span^k (Horner on absolute values).
         double P = fabs(t[n]);
 #pragma unroll
         for (int k = n - 1; k >= 0; --k) P = fma(P, span, fabs(t[k]));
-        // Taylor shift by h_lb.
+        if (SHIFT) { // Taylor shift by h_lb
 #pragma unroll
-        for (int i = 0; i < n; ++i)
+            for (int i = 0; i < n; ++i)
 #pragma unroll
-            for (int k = n - 1; k >= i; --k) t[k] = fma(h_lb, t[k + 1], t[k]);
+                for (int k = n - 1; k >= i; --k) t[k] = fma(h_lb, t[k + 1], t[k]);
+        }
         double dp = 1.0;
 #pragma unroll
         for (int i = 0; i < OP1; ++i) {
-            t[i] = (t[i] * dp) * __ldg(inv_binom + i);
+            t[i] = (t[i] * dp) * inv.v[i];
             dp *= delta;
         }
         double mn = t[0], mx = t[0];
@@ -350,20 +377,36 @@ __device__ __forceinline__ void segment_box_mixed(const double *__restrict__ cf,
         for (int k = 1; k < OP1; ++k) {
 #pragma unroll
             for (int j = 0; j + k < OP1; ++j) t[j] = t[j] + t[j + 1];
-            mn = fmin(mn, t[0]);
-            mx = fmax(mx, t[0]);
+            mn = t[0] < mn ? t[0] : mn;
+            mx = t[0] > mx ? t[0] : mx;
         }
         const double E = 2.0 * (8.0 * n + 16.0) * 1.1102230246251565e-16 * P * 1.0001;
-        mn = (mn - E) - radius;
-        mx = (mx + E) + radius;
-        const float fl = next_down(__double2float_rd(mn));
-        const float fu = next_up(__double2float_ru(mx));
-        if (!isfinite(fl)) set_error(st, ERR_AABB_LB, obj, 0, fl, 0);
-        if (!isfinite(fu)) set_error(st, ERR_AABB_UB, obj, 0, fu, 0);
-        lb[d] = fmin_ref(lb[d], fl);
-        ub[d] = fmax_ref(ub[d], fu);
+        float fl, fu;
+        if constexpr (MIXED) {
+            mn = (mn - E) - radius;
+            mx = (mx + E) + radius;
+            fl = next_down(__double2float_rd(mn));
+            fu = next_up(__double2float_ru(mx));
+            if (act && !isfinite(fl)) set_error(st, ERR_AABB_LB, obj, 0, fl, 0);
+            if (act && !isfinite(fu)) set_error(st, ERR_AABB_UB, obj, 0, fu, 0);
+        } else {
+            // A NaN anywhere in the table stays in t[0] (the comparisons drop
+            // it); 1e-250 covers values that underflow.
+            const double R = E + 8.9e-16 * (fmax(fabs(mn), fabs(mx)) + radius) + 1e-250;
+            const float l0 = __double2float_rn((mn - R) - radius), l1 = __double2float_rn((mn + R) - radius);
+            const float u0 = __double2float_rn((mx - R) + radius), u1 = __double2float_rn((mx + R) + radius);
+            fl = next_down(l0);
+            fu = next_up(u0);
+            if (!(l0 == l1 && u0 == u1 && isfinite(fl) && isfinite(fu) && t[0] == t[0])) unsure = true;
+        }
+        if (act) {
+            if (d == 0) lb.x = fmin_ref(lb.x, fl), ub.x = fmax_ref(ub.x, fu);
+            else if (d == 1) lb.y = fmin_ref(lb.y, fl), ub.y = fmax_ref(ub.y, fu);
+            else if (d == 2) lb.z = fmin_ref(lb.z, fl), ub.z = fmax_ref(ub.z, fu);
+            else lb.w = fmin_ref(lb.w, fl), ub.w = fmax_ref(ub.w, fu);
+        }
     }
-    if (scr) {
+    if (MIXED && scr && act) {
         // sqrt is correctly rounded; the factor covers its half ulp and the
         // accumulation before the upward conversion.
         const float a = __double2float_ru(sqrt(a2) * (1.0 + 1e-12));
@@ -372,96 +415,167 @@ __device__ __forceinline__ void segment_box_mixed(const double *__restrict__ cf,
     }
 }
 
-template <int OP1>
-__global__ void __launch_bounds__(128) k_aabb_mixed(dev_pj pj, const double2 *__restrict__ cd_bounds,
-                                                    const double *__restrict__ inv_binom, uint32_t s_first,
-                                                    uint32_t n_batch, double radius, float *__restrict__ aabbs,
-                                                    uint2 *__restrict__ more, unsigned long long *more_count,
-                                                    float4 *__restrict__ scr, uint2 *__restrict__ srange,
-                                                    dev_status *st)
+// step_range for an object whose data overlap [cb, ce): the first segment end
+// after cb is looked for around the place it would have if the segments were
+// equally long (most objects' are), so that it usually takes two dependent
+// loads instead of a binary search's seven.
+__device__ __forceinline__ void step_range_near(const double *t, uint32_t ns, double t0, double tn, double cb,
+                                                double ce, uint32_t &tb, uint32_t &te)
 {
+    const double x = (cb - t0) / (tn - t0) * double(ns);
+    uint32_t lo = 1, hi = ns; // t[ns] > cb: the answer is in [lo, hi]
+    const uint32_t g = 1 + uint32_t(fmin(fmax(x, 0.0), double(ns - 1)));
+    if (t[g] > cb) {
+        hi = g;
+        if (g > 1 && t[g - 1] > cb) {
+            hi = g - 1;
+        } else {
+            lo = g;
+        }
+    } else {
+        lo = g + 1;
+        if (t[g + 1] > cb) hi = g + 1; // g < ns, since t[ns] > cb
+        else lo = g + 2;
+    }
+    tb = upper_bound_t(t, lo, hi, cb);
+    uint32_t e = tb;
+    for (int k = 0; k < 2 && e < ns + 1 && t[e] < ce; ++k) ++e;
+    te = (e < ns + 1 && t[e] < ce) ? lower_bound_t(t, e + 1, ns + 1, ce) : e;
+    te += (te != ns + 1);
+}
+
+// Pass 1, one lane per (step, object): the first overlapping segment
+// (aabbs.cpp:64-252).  Queued for pass 2 (more: (step | AABB_EXACT, object)):
+// objects with further overlapping segments in the step, and objects whose
+// bounds are not proven.
+constexpr uint32_t AABB_EXACT = 0x80000000u;
+
+template <int OP1, bool MIXED>
+__global__ void __launch_bounds__(AABB_T, aabb_shape<OP1>::CTAS)
+    k_aabb(dev_pj pj, const double2 *__restrict__ cd_bounds,
+                                                 const inv_binoms inv, uint32_t s_first,
+                                                 uint32_t n_batch, double radius, float *__restrict__ aabbs,
+                                                 uint2 *__restrict__ more, unsigned long long *more_count,
+                                                 float4 *__restrict__ scr, uint2 *__restrict__ srange,
+                                                 dev_status *st)
+{
+    __shared__ __align__(16) aabb_smem<OP1> S[AABB_W];
     const uint64_t N = pj.n_objs;
-    const uint64_t gid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    const uint64_t gid = blockIdx.x * uint64_t(AABB_T) + threadIdx.x;
     const bool active = gid < N * n_batch;
     const uint32_t b = active ? uint32_t(gid / N) : 0;
-    const uint64_t i = active ? gid % N : 0;
-    float lb[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-    float ub[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    bool queue = false;
-    if (active) {
+    const uint32_t i = active ? uint32_t(gid % N) : 0;
+    bool seg = false, queue = false;
+    double h_lb = 0, h_ub = 0;
+    const double *first = pj.coef; // lanes without a segment copy the first one's rows
+    uint2 rng = make_uint2(0, 0);  // empty: no segment overlaps the step
+    const uint32_t ns = active ? pj.nseg[i] : 0;
+    if (ns > 0) {
         const double2 cbe = cd_bounds[s_first + b];
         const double cb = cbe.x, ce = cbe.y;
-        const uint32_t ns = pj.nseg[i];
-        uint2 rng = make_uint2(0, 0); // empty: no segment overlaps the step
-        if (ns > 0) {
-            const double *t = pj.time + pj.time_off[i];
-            if (!(t[0] >= ce || t[ns] <= cb)) {
-                uint32_t tb, te;
-                step_range(t, ns, cb, ce, tb, te);
-                rng = make_uint2(tb, te);
-                if (tb != te) {
-                    const uint32_t it = tb;
-                    const double s0 = t[it - 1];
-                    const double ev_lb = (cb < s0) ? s0 : cb;
-                    const double ev_ub = (t[it] < ce) ? t[it] : ce;
-                    segment_box_mixed<OP1>(coef_row<OP1>(pj, pj.seg_off[i] + it - 1, 0), inv_binom, ev_lb - s0,
-                                           ev_ub - s0, radius, uint32_t(i), lb, ub, st,
-                                           scr ? scr + (uint64_t(b) * N + i) * 4 : nullptr);
-                    queue = te - tb > 1;
-                }
+        const double *t = pj.time + pj.time_off[i];
+        const double t0 = t[0], tn = t[ns];
+        if (!(t0 >= ce || tn <= cb)) {
+            uint32_t tb, te;
+            step_range_near(t, ns, t0, tn, cb, ce, tb, te);
+            rng = make_uint2(tb, te);
+            if (tb != te) {
+                seg = true;
+                const double s0 = t[tb - 1], s1 = t[tb];
+                const double ev_lb = (cb < s0) ? s0 : cb; // std::max(cb, s0)
+                const double ev_ub = (s1 < ce) ? s1 : ce; // std::min(ce, t[it])
+                h_lb = ev_lb - s0;
+                h_ub = ev_ub - s0;
+                first = coef_row<OP1>(pj, pj.seg_off[i] + tb - 1, 0);
+                queue = te - tb > 1;
             }
         }
+    }
+    float4 lb = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+    float4 ub = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    bool unsure = false;
+    if (__any_sync(0xffffffffu, seg))
+        warp_segment_box<OP1, MIXED, true>(S[threadIdx.x >> 5], inv, first, seg, h_lb, h_ub, radius, i, lb, ub,
+                                           unsure, st, MIXED && scr ? scr + (uint64_t(b) * N + i) * 4 : nullptr);
+    if (active) {
         float4 *o = reinterpret_cast<float4 *>(aabbs + ((uint64_t(s_first) + b) * (N + 1) + i) * 8);
-        o[0] = make_float4(lb[0], lb[1], lb[2], lb[3]);
-        o[1] = make_float4(ub[0], ub[1], ub[2], ub[3]);
+        o[0] = lb;
+        o[1] = ub;
         srange[uint64_t(b) * N + i] = rng;
     }
+    const bool redo = !MIXED && seg && unsure;
+    queue = queue || redo;
     const unsigned mask = __ballot_sync(0xffffffffu, queue);
     if (queue) {
         const unsigned lane = threadIdx.x & 31;
         const int leader = __ffs(mask) - 1;
-        unsigned long long base = 0;
-        if (int(lane) == leader) base = atomicAdd(more_count, (unsigned long long)__popc(mask));
-        base = __shfl_sync(mask, base, leader);
+        unsigned long long at = 0;
+        if (int(lane) == leader) at = atomicAdd(more_count, (unsigned long long)__popc(mask));
+        at = __shfl_sync(mask, at, leader);
         unsigned lt;
         asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        more[base + __popc(mask & lt)] = make_uint2(b, uint32_t(i));
+        more[at + __popc(mask & lt)] = make_uint2(b | (redo ? AABB_EXACT : 0u), i);
     }
 }
 
-template <int OP1>
-__global__ void __launch_bounds__(128) k_aabb_mixed_more(dev_pj pj, const double2 *__restrict__ cd_bounds,
-                                                         const double *__restrict__ inv_binom, uint32_t s_first,
-                                                         double radius, float *__restrict__ aabbs,
-                                                         const uint2 *__restrict__ more,
-                                                         const unsigned long long *more_count,
-                                                         float4 *__restrict__ scr, dev_status *st)
+// Pass 2: the remaining overlapping segments of the queued objects, in time
+// order, folded into the boxes written by pass 1 (persistent grid).  They all
+// start inside the step: no shift.
+template <int OP1, bool MIXED>
+__global__ void __launch_bounds__(AABB_T, OP1 <= 20 ? 4 : 3)
+    k_aabb_more(dev_pj pj, const double2 *__restrict__ cd_bounds,
+                                                      const inv_binoms inv, uint32_t s_first,
+                                                      double radius, float *__restrict__ aabbs,
+                                                      const uint2 *__restrict__ more,
+                                                      const unsigned long long *more_count,
+                                                      float4 *__restrict__ scr, const uint2 *__restrict__ srange,
+                                                      dev_status *st)
 {
+    __shared__ __align__(16) aabb_smem<OP1> S[AABB_W];
     const uint64_t N = pj.n_objs;
     const uint64_t n = *more_count;
-    for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
-        const uint2 e = more[k];
-        const uint32_t b = e.x, i = e.y;
+    const unsigned lane = threadIdx.x & 31;
+    for (uint64_t k0 = (blockIdx.x * uint64_t(AABB_T) + threadIdx.x) & ~uint64_t(31); k0 < n;
+         k0 += uint64_t(gridDim.x) * AABB_T) {
+        const bool active = k0 + lane < n;
+        const uint2 e = active ? more[k0 + lane] : make_uint2(0, 0);
+        const uint32_t b = e.x & ~AABB_EXACT, i = e.y;
         const double2 cbe = cd_bounds[s_first + b];
         const double cb = cbe.x, ce = cbe.y;
         const double *t = pj.time + pj.time_off[i];
-        uint32_t tb, te;
-        step_range(t, pj.nseg[i], cb, ce, tb, te);
+        const uint2 rng = active ? srange[uint64_t(b) * N + i] : make_uint2(0, 0);
+        const uint64_t seg0 = pj.seg_off[i];
         float4 *o = reinterpret_cast<float4 *>(aabbs + ((uint64_t(s_first) + b) * (N + 1) + i) * 8);
-        const float4 l0 = o[0], u0 = o[1];
-        float lb[4] = {l0.x, l0.y, l0.z, l0.w}, ub[4] = {u0.x, u0.y, u0.z, u0.w};
-        for (uint32_t it = tb + 1; it != te; ++it) {
-            const double s0 = t[it - 1];
-            const double ev_lb = (cb < s0) ? s0 : cb;
-            const double ev_ub = (t[it] < ce) ? t[it] : ce;
+        float4 lb = o[0], ub = o[1];
+        bool unsure = (e.x & AABB_EXACT) != 0;
+        for (uint32_t it = rng.x + 1;; ++it) {
+            const bool act = active && it < rng.y && !unsure;
+            if (!__any_sync(0xffffffffu, act)) break;
+            double h_ub = 0;
+            const double *first = pj.coef;
+            if (act) {
+                const double s0 = t[it - 1], s1 = t[it];
+                const double ev_ub = (s1 < ce) ? s1 : ce;
+                h_ub = ev_ub - s0;
+                first = coef_row<OP1>(pj, seg0 + it - 1, 0);
+            }
             // The step's second segment has the second model slot; later
             // ones (short segments) are screened from their coefficients.
-            segment_box_mixed<OP1>(coef_row<OP1>(pj, pj.seg_off[i] + it - 1, 0), inv_binom, ev_lb - s0,
-                                   ev_ub - s0, radius, i, lb, ub, st,
-                                   (it == tb + 1 && scr) ? scr + (uint64_t(b) * N + i) * 4 + 2 : nullptr);
+            bool u = false;
+            warp_segment_box<OP1, MIXED, false>(
+                S[threadIdx.x >> 5], inv, first, act, 0.0, h_ub, radius, i, lb, ub, u, st,
+                (MIXED && scr && it == rng.x + 1) ? scr + (uint64_t(b) * N + i) * 4 + 2 : nullptr);
+            unsure = unsure || (act && u);
         }
-        o[0] = make_float4(lb[0], lb[1], lb[2], lb[3]);
-        o[1] = make_float4(ub[0], ub[1], ub[2], ub[3]);
+        if (!active) continue;
+        if (!MIXED && unsure) {
+            float l[4], u[4];
+            object_box<OP1>(pj, i, cb, ce, rng.x, rng.y, radius, l, u, st);
+            lb = make_float4(l[0], l[1], l[2], l[3]);
+            ub = make_float4(u[0], u[1], u[2], u[3]);
+        }
+        o[0] = lb;
+        o[1] = ub;
     }
 }
 
@@ -569,31 +683,30 @@ void launch_relayout(const double *src, double *dst, uint64_t n_seg, int op1, un
 }
 
 template <int OP1>
-static void aabb_t(const dev_pj &pj, const double2 *cdb, const double *inv_binom, uint32_t s_first, uint32_t nb,
+static void aabb_t(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_first, uint32_t nb,
                    double radius, float *aabbs, uint2 *more, unsigned long long *more_count, float4 *scr,
                    uint2 *srange, dev_status *st, cudaStream_t stream)
 {
-    const uint64_t n = pj.n_objs * nb;
-    const unsigned bs = 128;
-    if (inv_binom) {
-        k_aabb_mixed<OP1><<<unsigned((n + bs - 1) / bs), bs, 0, stream>>>(pj, cdb, inv_binom, s_first, nb, radius,
-                                                                          aabbs, more, more_count, scr, srange, st);
-        k_aabb_mixed_more<OP1><<<148 * 5, bs, 0, stream>>>(pj, cdb, inv_binom, s_first, radius, aabbs, more,
-                                                            more_count, scr, st);
+    const inv_binoms inv = make_inv_binoms(OP1 - 1);
+    const unsigned g = unsigned((pj.n_objs * nb + AABB_T - 1) / AABB_T);
+    if (mixed) {
+        k_aabb<OP1, true><<<g, AABB_T, 0, stream>>>(pj, cdb, inv, s_first, nb, radius, aabbs, more, more_count,
+                                                    scr, srange, st);
+        k_aabb_more<OP1, true><<<148 * 5, AABB_T, 0, stream>>>(pj, cdb, inv, s_first, radius, aabbs, more,
+                                                               more_count, scr, srange, st);
     } else {
-        k_aabb<OP1><<<unsigned((n + bs - 1) / bs), bs, 0, stream>>>(pj, cdb, s_first, nb, radius, aabbs, more,
-                                                                    more_count, srange, st);
-        k_aabb_more<OP1><<<148 * 4, bs, 0, stream>>>(pj, cdb, s_first, radius, aabbs, more, more_count, st);
+        k_aabb<OP1, false><<<g, AABB_T, 0, stream>>>(pj, cdb, inv, s_first, nb, radius, aabbs, more, more_count,
+                                                     nullptr, srange, st);
+        k_aabb_more<OP1, false><<<148 * 4, AABB_T, 0, stream>>>(pj, cdb, inv, s_first, radius, aabbs, more,
+                                                                more_count, nullptr, srange, st);
     }
 }
 
-// inv_binom == nullptr selects the plain form; otherwise it points to
-// 1 / C(order, i), i = 0..order, and selects the mixed form.
 // scr (mixed form only): two 32-byte screen models per (step, object) of the
 // batch, for the first and second segment overlapping the step.
 // srange[b * N + i]: the segments of object i overlapping the batch's step b,
 // as step_range gives them (time-point indices [tb, te); (0, 0) if none).
-void launch_aabb(const dev_pj &pj, const double2 *cdb, const double *inv_binom, uint32_t s_first, uint32_t nb,
+void launch_aabb(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_first, uint32_t nb,
                  double radius, float *aabbs, uint2 *more, unsigned long long *more_count, float4 *scr,
                  uint2 *srange, dev_status *st, cudaStream_t stream)
 {
@@ -601,7 +714,7 @@ void launch_aabb(const dev_pj &pj, const double2 *cdb, const double *inv_binom, 
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        aabb_t<K>(pj, cdb, inv_binom, s_first, nb, radius, aabbs, more, more_count, scr, srange, st, stream);         \
+        aabb_t<K>(pj, cdb, mixed, s_first, nb, radius, aabbs, more, more_count, scr, srange, st, stream);         \
         break;
         MZB_FOR_EACH_OP1(X)
 #undef X

@@ -58,7 +58,7 @@ struct stage_run {
 static_assert(sizeof(stage_run) == 16, "stage_run layout");
 void launch_relayout_runs(const char *piece, uint64_t n_runs, double *coef, int op1, unsigned long long *bad_seg,
                           cudaStream_t stream);
-void launch_aabb(const dev_pj &pj, const double2 *cdb, const double *inv_binom, uint32_t s_first, uint32_t nb,
+void launch_aabb(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_first, uint32_t nb,
                  double radius, float *aabbs, uint2 *more, unsigned long long *more_count, float4 *scr,
                  uint2 *srange, dev_status *st, cudaStream_t stream);
 void launch_morton(const float *aabbs, uint32_t s_first, uint32_t nb, uint64_t N, uint64_t *mcodes,

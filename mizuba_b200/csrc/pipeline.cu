@@ -1010,31 +1010,30 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     d_cdb.alloc(S, st);
     // Tables of the narrow phase: nodes, inverse node differences, inverse
     // binomials, binomials of the translation.
-    dbuf<double> d_mixed(SL());
-    std::vector<double> h_mixed;
+    dbuf<double> d_tab(SL());
+    std::vector<double> h_tab;
     {
         const int op1 = pj.order + 1, n = pj.order;
         const cheb_nodes cn = make_cheb_nodes(op1);
-        h_mixed.assign(size_t(op1) * (2 * op1 + 2), 0.0);
-        for (int m = 0; m < op1; ++m) h_mixed[m] = cn.v[m];
+        h_tab.assign(size_t(op1) * (2 * op1 + 2), 0.0);
+        for (int m = 0; m < op1; ++m) h_tab[m] = cn.v[m];
         for (int k = 0; k < n; ++k)
-            for (int j = k + 1; j < op1; ++j) h_mixed[op1 + size_t(k) * op1 + j] = 1.0 / (cn.v[j] - cn.v[j - k - 1]);
+            for (int j = k + 1; j < op1; ++j) h_tab[op1 + size_t(k) * op1 + j] = 1.0 / (cn.v[j] - cn.v[j - k - 1]);
         double c = 1.0;
         for (int i = 0; i <= n; ++i) {
-            h_mixed[op1 + size_t(op1) * op1 + i] = 1.0 / c;
+            h_tab[op1 + size_t(op1) * op1 + i] = 1.0 / c;
             c = c * (n - i) / (i + 1);
         }
         // C(i + k, k), exact: Pascal's rule along row k.
-        double *sh = h_mixed.data() + size_t(op1) * (op1 + 2);
+        double *sh = h_tab.data() + size_t(op1) * (op1 + 2);
         for (int k = 0; k < op1; ++k)
             for (int i = 0; i + k < op1; ++i)
                 sh[size_t(k) * op1 + i] = (k == 0 || i == 0) ? 1.0 : sh[size_t(k) * op1 + i - 1] + sh[size_t(k - 1) * op1 + i];
-        d_mixed.alloc(h_mixed.size(), st);
-        CK(cudaMemcpyAsync(d_mixed.p, h_mixed.data(), h_mixed.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        d_tab.alloc(h_tab.size(), st);
+        CK(cudaMemcpyAsync(d_tab.p, h_tab.data(), h_tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     }
-    const double *filter_tab = d_mixed.p;
+    const double *filter_tab = d_tab.p;
     const filter_limits filter_lim = make_filter_limits(pj.order + 1);
-    const double *mixed_inv_binom = mixed ? d_mixed.p + (pj.order + 1) + size_t(pj.order + 1) * (pj.order + 1) : nullptr;
     CK(cudaMemcpyAsync(d_cdb.p, cdb.data(), S * sizeof(double2), cudaMemcpyHostToDevice, st));
     dbuf<int32_t> d_ot(SL());
     d_ot.alloc(N, st);
@@ -1194,7 +1193,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         const std::string bname = "batch " + std::to_string(s0) + "+" + std::to_string(nb);
         tr.dev_mark(bname + ": its upload chunks in", st);
         CK(cudaEventRecord(ev[0].a, st));
-        launch_aabb(P, d_cdb.p, mixed_inv_binom, sf, nb, radius, R.aabbs.p, more.p, more_count.p,
+        launch_aabb(P, d_cdb.p, mixed, sf, nb, radius, R.aabbs.p, more.p, more_count.p,
                     mixed ? scr.p : nullptr, srange.p, d_st.p, st);
         CK(cudaEventRecord(ev[0].b, st));
         CK(cudaEventRecord(ev[1].a, st));
