@@ -1374,44 +1374,23 @@ __device__ __forceinline__ bool conj_less(const conj_rec &a, const conj_rec &b)
     return false;
 }
 
-__global__ void k_conj_count(const conj_out *cq, uint64_t n, uint32_t *cnt)
-{
-    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    if (g < n) atomicAdd(cnt + cq[g].step, 1u);
-}
-
-// One block: exclusive scan of the per-step counts (also resets cursors).
-__global__ void k_conj_offsets(const uint32_t *cnt, uint32_t nb, uint32_t *off, uint32_t *cursor)
-{
-    __shared__ uint32_t sm[33];
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < nb; base += blockDim.x) {
-        const uint32_t k = base + threadIdx.x;
-        const uint32_t v = k < nb ? cnt[k] : 0;
-        uint32_t tot;
-        const uint32_t ex = block_excl_scan(v, sm, &tot);
-        if (k < nb) {
-            off[k] = carry + ex;
-            cursor[k] = 0;
-        }
-        carry += tot;
-    }
-    if (threadIdx.x == 0) off[nb] = carry;
-}
-
-__global__ void k_conj_group(const conj_out *cq, uint64_t n, const uint32_t *off, uint32_t *cursor, conj_out *grp)
-{
-    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    if (g >= n) return;
-    const uint32_t s = cq[g].step;
-    const uint32_t pos = atomicAdd(cursor + s, 1u);
-    grp[off[s] + pos] = cq[g];
-}
-
-// Steps with at most CONJ_SORT_MAX conjunctions are ordered by one block
-// each (k_conj_sort_step); larger groups by k_conj_rank.
-constexpr uint32_t CONJ_SORT_MAX = 16384;
-constexpr size_t CONJ_SORT_SMEM = size_t(CONJ_SORT_MAX) * (sizeof(uint64_t) + sizeof(uint32_t));
+// The batch's conjunctions ordered by (step, tca, record)
+// (detect_conjunctions_narrow_phase.cpp:751-757: by tca within a step, ties by
+// the record's three-way comparison).
+//
+// Up to CONJ_SMALL of them: one CTA sorts them all (k_conj_small).  More: they
+// are grouped by step as (tca key, queue index) pairs, every step's group is
+// cut into chunks of CONJ_CHUNK that one CTA each sorts in shared memory, and
+// every conjunction's place is its place in its chunk plus, by binary search,
+// the numbers of smaller ones in the step's other chunks; the records move
+// once, to their places.  Counting and grouping take one global atomic per
+// CTA and step.  With one CTA a step, a counter hit by every record and the
+// runs of equal TCAs sorted by one thread each, the 507,000 conjunctions of
+// 60,000 objects x 48 steps at 20 km took 2.8 ms; 0.24 ms now.  A handful of
+// them takes one launch instead of five (22 -> 10 us).
+constexpr uint32_t CONJ_SMALL = 512;
+constexpr uint32_t CONJ_CHUNK = 2048;
+constexpr uint32_t CONJ_HIST = 8192; // steps counted in shared memory
 
 // Order-preserving integer image of a double (the TCAs are finite).
 __device__ __forceinline__ uint64_t tca_key(double x)
@@ -1420,50 +1399,62 @@ __device__ __forceinline__ uint64_t tca_key(double x)
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-// One block per step: bitonic sort of the step's (TCA, slot) keys in shared
-// memory, then each run of equal TCAs ordered by the whole record
-// (detect_conjunctions_narrow_phase.cpp:751-757: by tca, ties by the
-// record's three-way comparison), then the records written in order.
-__global__ void __launch_bounds__(1024) k_conj_sort_step(const conj_out *__restrict__ grp,
-                                                         const uint32_t *__restrict__ off, conj_rec *__restrict__ out)
+// The pair of a record as the second key: (i, j) follow tca in its order.
+__device__ __forceinline__ uint64_t pair_key(const conj_rec &r) { return (uint64_t(r.i) << 32) | r.j; }
+
+constexpr int CONJ_T = 512;
+
+// Sorts n entries (n at most the arrays' power-of-two size) of shared memory
+// by (step, tca key, pair), and each run of equal entries by the whole record.
+// Many conjunctions share a TCA exactly (every close pair at the start of the
+// data has one there), so the pair is a key and not left to the runs.  step
+// may be null (one step).  Whole CTA of CONJ_T threads.
+__device__ __forceinline__ void conj_sort_smem(uint64_t *key, uint64_t *pair, uint32_t *idx, uint32_t *step,
+                                               uint32_t n, const conj_out *__restrict__ cq)
 {
-    extern __shared__ __align__(16) unsigned char conj_smem[];
-    uint64_t *key = reinterpret_cast<uint64_t *>(conj_smem);
-    uint32_t *idx = reinterpret_cast<uint32_t *>(key + CONJ_SORT_MAX);
-    const uint32_t s = blockIdx.x;
-    const uint32_t b0 = off[s], n = off[s + 1] - b0;
-    if (n == 0 || n > CONJ_SORT_MAX) return;
     uint32_t P = 1;
     while (P < n) P <<= 1;
-    for (uint32_t k = threadIdx.x; k < P; k += blockDim.x) {
-        key[k] = k < n ? tca_key(grp[b0 + k].c.tca) : ~0ull;
-        idx[k] = k < n ? k : 0xffffffffu;
+    for (uint32_t k = n + threadIdx.x; k < P; k += CONJ_T) {
+        key[k] = pair[k] = ~0ull;
+        idx[k] = 0xffffffffu;
+        if (step) step[k] = 0xffffffffu;
     }
     __syncthreads();
     for (uint32_t size = 2; size <= P; size <<= 1)
         for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t t = threadIdx.x; t < P / 2; t += blockDim.x) {
+            for (uint32_t t = threadIdx.x; t < P / 2; t += CONJ_T) {
                 const uint32_t i = 2 * t - (t & (stride - 1)), j = i + stride;
                 const bool asc = (i & size) == 0;
                 const uint64_t ki = key[i], kj = key[j];
+                const uint32_t si = step ? step[i] : 0, sj = step ? step[j] : 0;
+                const uint64_t pi = pair[i], pj = pair[j];
                 const uint32_t ii = idx[i], ij = idx[j];
-                const bool gt = ki > kj || (ki == kj && ii > ij);
+                const bool gt = si != sj ? si > sj : ki != kj ? ki > kj : pi != pj ? pi > pj : ii > ij;
                 if (gt == asc) {
                     key[i] = kj;
                     key[j] = ki;
+                    pair[i] = pj;
+                    pair[j] = pi;
                     idx[i] = ij;
                     idx[j] = ii;
+                    if (step) {
+                        step[i] = sj;
+                        step[j] = si;
+                    }
                 }
             }
             __syncthreads();
         }
-    // Runs of equal TCA (rare, short): insertion sort by the whole record.
-    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
-        if ((k == 0 || key[k - 1] != key[k]) && k + 1 < n && key[k + 1] == key[k]) {
+    // One pair twice at one TCA: insertion sort by the whole record.
+    auto same = [&](uint32_t a, uint32_t b) {
+        return key[a] == key[b] && pair[a] == pair[b] && (!step || step[a] == step[b]);
+    };
+    for (uint32_t k = threadIdx.x; k < n; k += CONJ_T) {
+        if ((k == 0 || !same(k - 1, k)) && k + 1 < n && same(k + 1, k)) {
             uint32_t e = k + 1;
-            while (e < n && key[e] == key[k]) ++e;
+            while (e < n && same(e, k)) ++e;
             for (uint32_t a = k + 1; a < e; ++a)
-                for (uint32_t c = a; c > k && conj_less(grp[b0 + idx[c]].c, grp[b0 + idx[c - 1]].c); --c) {
+                for (uint32_t c = a; c > k && conj_less(cq[idx[c]].c, cq[idx[c - 1]].c); --c) {
                     const uint32_t t2 = idx[c];
                     idx[c] = idx[c - 1];
                     idx[c - 1] = t2;
@@ -1471,25 +1462,160 @@ __global__ void __launch_bounds__(1024) k_conj_sort_step(const conj_out *__restr
         }
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) out[b0 + k] = grp[b0 + idx[k]].c;
 }
 
-// Rank within the step's group (groups larger than CONJ_SORT_MAX); equal
-// records are ordered by group slot.
-__global__ void k_conj_rank(const conj_out *grp, uint64_t n, const uint32_t *off, conj_rec *out)
+__global__ void __launch_bounds__(CONJ_T) k_conj_small(const conj_out *__restrict__ cq, uint32_t n,
+                                                       conj_rec *__restrict__ out)
 {
-    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    if (g >= n) return;
-    const conj_out me = grp[g];
-    const uint32_t b0 = off[me.step], b1 = off[me.step + 1];
-    if (b1 - b0 <= CONJ_SORT_MAX) return;
-    uint32_t rank = 0;
-    for (uint32_t k = b0; k < b1; ++k) {
-        if (k == g) continue;
-        const conj_rec &o = grp[k].c;
-        if (conj_less(o, me.c) || (k < g && !conj_less(me.c, o))) ++rank;
+    __shared__ uint64_t key[CONJ_SMALL], pair[CONJ_SMALL];
+    __shared__ uint32_t idx[CONJ_SMALL], step[CONJ_SMALL];
+    for (uint32_t k = threadIdx.x; k < n; k += CONJ_T) {
+        key[k] = tca_key(cq[k].c.tca);
+        pair[k] = pair_key(cq[k].c);
+        idx[k] = k;
+        step[k] = cq[k].step;
     }
-    out[b0 + rank] = me.c;
+    conj_sort_smem(key, pair, idx, step, n, cq);
+    for (uint32_t k = threadIdx.x; k < n; k += CONJ_T) out[k] = cq[idx[k]].c;
+}
+
+// Conjunctions per step: one global atomic per CTA and step it meets.
+__global__ void __launch_bounds__(1024) k_conj_count(const conj_out *__restrict__ cq, uint64_t n, uint32_t nb,
+                                                     uint32_t *__restrict__ cnt)
+{
+    __shared__ uint32_t hist[CONJ_HIST];
+    for (uint32_t s = threadIdx.x; s < min(nb, CONJ_HIST); s += blockDim.x) hist[s] = 0;
+    __syncthreads();
+    for (uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; g < n; g += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t s = cq[g].step;
+        if (s < CONJ_HIST) atomicAdd(&hist[s], 1u);
+        else atomicAdd(cnt + s, 1u);
+    }
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < min(nb, CONJ_HIST); s += blockDim.x)
+        if (hist[s]) atomicAdd(cnt + s, hist[s]);
+}
+
+// One block: exclusive scans of the per-step counts and chunk numbers (also
+// resets cursors).
+__global__ void k_conj_offsets(const uint32_t *cnt, uint32_t nb, uint32_t *off, uint32_t *choff, uint32_t *cursor)
+{
+    __shared__ uint32_t sm[33];
+    uint32_t carry = 0, ccarry = 0;
+    for (uint32_t base = 0; base < nb; base += blockDim.x) {
+        const uint32_t k = base + threadIdx.x;
+        const uint32_t v = k < nb ? cnt[k] : 0;
+        uint32_t tot, ctot;
+        const uint32_t ex = block_excl_scan(v, sm, &tot);
+        const uint32_t cex = block_excl_scan((v + CONJ_CHUNK - 1) / CONJ_CHUNK, sm, &ctot);
+        if (k < nb) {
+            off[k] = carry + ex;
+            choff[k] = ccarry + cex;
+            cursor[k] = 0;
+        }
+        carry += tot;
+        ccarry += ctot;
+    }
+    if (threadIdx.x == 0) {
+        off[nb] = carry;
+        choff[nb] = ccarry;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_conj_group(const conj_out *__restrict__ cq, uint64_t n, uint32_t nb,
+                                                     const uint32_t *__restrict__ off, uint32_t *__restrict__ cursor,
+                                                     uint64_t *__restrict__ gkey, uint32_t *__restrict__ gidx)
+{
+    __shared__ uint32_t hist[CONJ_HIST];
+    for (uint32_t s = threadIdx.x; s < min(nb, CONJ_HIST); s += blockDim.x) hist[s] = 0;
+    __syncthreads();
+    const uint64_t g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    const uint32_t s = g < n ? cq[g].step : 0;
+    uint32_t r = 0;
+    if (g < n) r = s < CONJ_HIST ? atomicAdd(&hist[s], 1u) : atomicAdd(cursor + s, 1u);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < min(nb, CONJ_HIST); q += blockDim.x)
+        if (hist[q]) hist[q] = atomicAdd(cursor + q, hist[q]);
+    __syncthreads();
+    if (g < n) {
+        const uint32_t at = off[s] + r + (s < CONJ_HIST ? hist[s] : 0);
+        gkey[at] = tca_key(cq[g].c.tca);
+        gidx[at] = uint32_t(g);
+    }
+}
+
+// The chunk of CTA c: its step, and its range in the grouped arrays.
+__device__ __forceinline__ uint32_t conj_chunk(const uint32_t *off, const uint32_t *choff, uint32_t nb, uint32_t c,
+                                               uint32_t &b, uint32_t &e)
+{
+    uint32_t lo = 0, hi = nb; // last step with choff <= c
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (choff[mid] <= c) lo = mid;
+        else hi = mid;
+    }
+    b = off[lo] + (c - choff[lo]) * CONJ_CHUNK;
+    e = min(off[lo + 1], b + CONJ_CHUNK);
+    return lo;
+}
+
+__global__ void __launch_bounds__(CONJ_T) k_conj_chunks(const conj_out *__restrict__ cq, uint32_t nb,
+                                                        const uint32_t *__restrict__ off,
+                                                        const uint32_t *__restrict__ choff,
+                                                        uint64_t *__restrict__ gkey, uint32_t *__restrict__ gidx)
+{
+    __shared__ uint64_t key[CONJ_CHUNK], pair[CONJ_CHUNK];
+    __shared__ uint32_t idx[CONJ_CHUNK];
+    if (blockIdx.x >= choff[nb]) return;
+    uint32_t b, e;
+    conj_chunk(off, choff, nb, blockIdx.x, b, e);
+    for (uint32_t k = threadIdx.x; k < e - b; k += CONJ_T) {
+        key[k] = gkey[b + k];
+        idx[k] = gidx[b + k];
+        pair[k] = pair_key(cq[idx[k]].c);
+    }
+    conj_sort_smem(key, pair, idx, nullptr, e - b, cq);
+    for (uint32_t k = threadIdx.x; k < e - b; k += CONJ_T) {
+        gkey[b + k] = key[k];
+        gidx[b + k] = idx[k];
+    }
+}
+
+__global__ void __launch_bounds__(CONJ_T) k_conj_merge(const conj_out *__restrict__ cq, uint32_t nb,
+                                                       const uint32_t *__restrict__ off,
+                                                       const uint32_t *__restrict__ choff,
+                                                       const uint64_t *__restrict__ gkey,
+                                                       const uint32_t *__restrict__ gidx, conj_rec *__restrict__ out)
+{
+    if (blockIdx.x >= choff[nb]) return;
+    uint32_t b, e;
+    const uint32_t s = conj_chunk(off, choff, nb, blockIdx.x, b, e);
+    for (uint32_t k = b + threadIdx.x; k < e; k += CONJ_T) {
+        const uint64_t key = gkey[k];
+        const conj_rec me = cq[gidx[k]].c;
+        const uint64_t pair = pair_key(me);
+        uint32_t place = k - b;
+        for (uint32_t c0 = off[s]; c0 < off[s + 1]; c0 += CONJ_CHUNK) {
+            if (c0 == b) continue;
+            const uint32_t c1 = min(off[s + 1], c0 + CONJ_CHUNK);
+            uint32_t lo = c0, hi = c1; // first (key, pair) >= mine
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) / 2;
+                const uint64_t o = gkey[mid];
+                if (o < key || (o == key && pair_key(cq[gidx[mid]].c) < pair)) lo = mid + 1;
+                else hi = mid;
+            }
+            // The same pair at the same TCA: by the record; of equal records
+            // the earlier chunk's come first.
+            while (lo < c1 && gkey[lo] == key) {
+                const conj_rec &o = cq[gidx[lo]].c;
+                if (pair_key(o) != pair || !(conj_less(o, me) || (c0 < b && !conj_less(me, o)))) break;
+                ++lo;
+            }
+            place += lo - c0;
+        }
+        out[off[s] + place] = me;
+    }
 }
 
 // ------------------------------------------------------------- launchers
@@ -1620,24 +1746,27 @@ void launch_roots(const dev_pj &pj, const root_item *rq, const unsigned long lon
     }
 }
 
-void launch_conj_sort(const conj_out *cq, uint64_t n, uint32_t nb, uint32_t *cnt, uint32_t *off, uint32_t *cursor,
-                      conj_out *grp, conj_rec *out, cudaStream_t stream)
+// cnt, off, choff, cursor: nb + 1 words; gkey, gidx: n entries (used when
+// there are more than CONJ_SMALL conjunctions).  Returns the launches.
+int launch_conj_sort(const conj_out *cq, uint64_t n, uint32_t nb, uint32_t *cnt, uint32_t *off, uint32_t *choff,
+                     uint32_t *cursor, uint64_t *gkey, uint32_t *gidx, conj_rec *out, cudaStream_t stream)
 {
+    if (n == 0) return 0;
+    if (n <= CONJ_SMALL) {
+        k_conj_small<<<1, CONJ_T, 0, stream>>>(cq, uint32_t(n), out);
+        return 1;
+    }
     cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * nb, stream);
-    if (n > 0) k_conj_count<<<unsigned((n + 255) / 256), 256, 0, stream>>>(cq, n, cnt);
-    k_conj_offsets<<<1, 1024, 0, stream>>>(cnt, nb, off, cursor);
-    if (n == 0) return;
-    k_conj_group<<<unsigned((n + 255) / 256), 256, 0, stream>>>(cq, n, off, cursor, grp);
-    k_conj_sort_step<<<nb, 1024, CONJ_SORT_SMEM, stream>>>(grp, off, out);
-    k_conj_rank<<<unsigned((n + 255) / 256), 256, 0, stream>>>(grp, n, off, out);
+    const unsigned g = unsigned((n + 1023) / 1024);
+    k_conj_count<<<std::min(g, 148u * 2), 1024, 0, stream>>>(cq, n, nb, cnt);
+    k_conj_offsets<<<1, 1024, 0, stream>>>(cnt, nb, off, choff, cursor);
+    k_conj_group<<<g, 1024, 0, stream>>>(cq, n, nb, off, cursor, gkey, gidx);
+    const unsigned chunks = unsigned(n / CONJ_CHUNK) + unsigned(std::min<uint64_t>(n, nb));
+    k_conj_chunks<<<chunks, CONJ_T, 0, stream>>>(cq, nb, off, choff, gkey, gidx);
+    k_conj_merge<<<chunks, CONJ_T, 0, stream>>>(cq, nb, off, choff, gkey, gidx, out);
+    return 5;
 }
 
-cudaError_t init_narrow_consts()
-{
-    const cudaError_t e = cudaFuncSetAttribute(k_conj_sort_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               int(CONJ_SORT_SMEM));
-    if (e != cudaSuccess) return e;
-    return upload_binom_table();
-}
+cudaError_t init_narrow_consts() { return upload_binom_table(); }
 
 } // namespace mzb

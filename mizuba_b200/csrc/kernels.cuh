@@ -115,8 +115,8 @@ void launch_roots(const dev_pj &pj, const root_item *rq, const unsigned long lon
                   double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                   conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,
                   dev_status *st, cudaStream_t stream);
-void launch_conj_sort(const conj_out *cq, uint64_t n, uint32_t nb, uint32_t *cnt, uint32_t *off, uint32_t *cursor,
-                      conj_out *grp, conj_rec *out, cudaStream_t stream);
+int launch_conj_sort(const conj_out *cq, uint64_t n, uint32_t nb, uint32_t *cnt, uint32_t *off, uint32_t *choff,
+                     uint32_t *cursor, uint64_t *gkey, uint32_t *gidx, conj_rec *out, cudaStream_t stream);
 
 // SGP4 polyjectory production (k_sgp4.cu).
 namespace sgp4pj

@@ -1083,7 +1083,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     // Batch scratch.
     const uint32_t nb_max = uint32_t(std::min<uint64_t>(S, spb));
     dbuf<uint64_t> keys_a(SL()), offs(SL()), block_sums(SL()), step_off(SL()), total(SL());
-    dbuf<uint32_t> vals_a(SL()), vals_b(SL()), counts(SL()), aux(SL()), cc_cnt(SL()), cc_off(SL()), cc_cur(SL());
+    dbuf<uint32_t> vals_a(SL()), vals_b(SL()), counts(SL()), aux(SL()), cc_cnt(SL()), cc_off(SL()), cc_ch(SL()), cc_cur(SL());
     dbuf<int32_t> ropes(SL());
     dbuf<walk_node> walks(SL());
     dbuf<dev_status> d_st(SL());
@@ -1133,6 +1133,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     cq_count.alloc(1, st);
     cc_cnt.alloc(nb_max + 1, st);
     cc_off.alloc(nb_max + 1, st);
+    cc_ch.alloc(nb_max + 1, st);
     cc_cur.alloc(nb_max + 1, st);
     CK(cudaMemsetAsync(d_st.p, 0, sizeof(dev_status), st));
     visits.alloc(1, st);
@@ -1144,7 +1145,9 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     surv_count.alloc(1, st);
     cand_count.alloc(1, st);
     const unsigned narrow_grid = 148 * 6;
-    dbuf<conj_out> cq(SL()), cgrp(SL());
+    dbuf<conj_out> cq(SL());
+    dbuf<uint64_t> ckey(SL());
+    dbuf<uint32_t> cidx(SL());
     dbuf<double> wl(SL()), wl_full(SL());
     dbuf<uint32_t> retry(SL());
     dbuf<unsigned long long> retry_count(SL());
@@ -1242,7 +1245,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             }
         }
         float t_bp = 0, t_np = 0, t_rt = 0;
-        uint64_t n_narrow_launches = 0, n_roots_launches = 0, n_broad_launches = 0;
+        uint64_t n_narrow_launches = 0, n_roots_launches = 0, n_broad_launches = 0, n_conj_launches = 0;
         // Mailbox read-backs of the batch: the status word, the tree sizes,
         // the pair counts and one per narrow-phase run.
         uint64_t n_mbox = want_trees ? 2 : 1;
@@ -1411,20 +1414,23 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 R.narrow_split[1] += h_surv + h_ctr[7];
             }
             // Per-step ordering, appended to the result.
-            if (cgrp.n < h_cq) cgrp.alloc(h_cq, st);
+            if (ckey.n < h_cq) ckey.alloc_queue(h_cq, st);
+            if (cidx.n < h_cq) cidx.alloc_queue(h_cq, st);
             if (R.conj.n < R.n_conj + h_cq)
                 R.conj.grow(std::max<uint64_t>(R.n_conj + h_cq, whole_call(R.n_conj + h_cq)), R.n_conj, st);
             CK(cudaEventRecord(ev[6].a, st));
-            launch_conj_sort(cq.p, h_cq, nb, cc_cnt.p, cc_off.p, cc_cur.p, cgrp.p, R.conj.p + R.n_conj, st);
+            n_conj_launches =
+                launch_conj_sort(cq.p, h_cq, nb, cc_cnt.p, cc_off.p, cc_ch.p, cc_cur.p, ckey.p, cidx.p,
+                                 R.conj.p + R.n_conj, st);
             CK(cudaEventRecord(ev[6].b, st));
             R.n_conj += h_cq;
             t_bp = ev[3].ms();
         }
         // aabb (2 passes + global box) + morton + sort + bvh; broad half walk, 3 scan kernels,
         // step offsets, scatter + list sorts,
-        // items + narrow, roots (+ retry), 5 conj-order kernels.
+        // items + filter + narrow, roots (+ retry), conj-order kernels.
         R.n_launches += 6 + n_mbox;
-        if (!skip_cd) R.n_launches += n_broad_launches + n_narrow_launches + n_roots_launches + 5;
+        if (!skip_cd) R.n_launches += n_broad_launches + n_narrow_launches + n_roots_launches + n_conj_launches;
         tr.dev_mark(bname + ": screened", st);
         if (dst) tr.dev_mark(bname + ": per-step outputs copied", cs);
         check_status();
