@@ -704,13 +704,13 @@ static void aabb_t(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_
 
 // scr (mixed form only): two 32-byte screen models per (step, object) of the
 // batch, for the first and second segment overlapping the step.
+// *more_count starts at zero.
 // srange[b * N + i]: the segments of object i overlapping the batch's step b,
 // as step_range gives them (time-point indices [tb, te); (0, 0) if none).
 void launch_aabb(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_first, uint32_t nb,
                  double radius, float *aabbs, uint2 *more, unsigned long long *more_count, float4 *scr,
                  uint2 *srange, dev_status *st, cudaStream_t stream)
 {
-    cudaMemsetAsync(more_count, 0, sizeof(unsigned long long), stream);
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \

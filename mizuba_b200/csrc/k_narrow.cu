@@ -47,6 +47,28 @@ __device__ __forceinline__ void warp_add(unsigned long long *ctr, unsigned long 
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(ctr, v);
 }
 
+// The sums of a and b over the CTA, added to *pa (and *pa2, when given) and
+// *pb: one atomic each per CTA.  Every thread of the CTA takes part.
+__device__ __forceinline__ void block_add2(unsigned long long *pa, unsigned long long *pa2, unsigned a,
+                                           unsigned long long *pb, unsigned b)
+{
+    __shared__ unsigned sa, sb;
+    if (threadIdx.x == 0) sa = sb = 0;
+    __syncthreads();
+    a = __reduce_add_sync(0xffffffffu, a);
+    b = __reduce_add_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31) == 0) {
+        if (a) atomicAdd(&sa, a);
+        if (b) atomicAdd(&sb, b);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sa) atomicAdd(pa, (unsigned long long)sa);
+        if (sa && pa2) atomicAdd(pa2, (unsigned long long)sa);
+        if (sb) atomicAdd(pb, (unsigned long long)sb);
+    }
+}
+
 // Warp-aggregated append of one slot per active lane; returns this lane's
 // slot.
 __device__ __forceinline__ unsigned long long warp_append(unsigned long long *counter, bool want)
@@ -103,7 +125,7 @@ __global__ void __launch_bounds__(128) k_items(const dev_pj pj, const double2 *_
         it_i = ri.x, ei = ri.y;
         it_j = rj.x, ej = rj.y;
     }
-    unsigned long long n_cand = 0;
+    unsigned n_cand = 0;
     uint32_t budget = (ei - it_i) + (ej - it_j);
     // Warp-synchronous loop: every lane iterates until all lanes are done.
     for (;;) {
@@ -135,7 +157,7 @@ __global__ void __launch_bounds__(128) k_items(const dev_pj pj, const double2 *_
             --budget;
         }
     }
-    warp_add(counters + 0, n_cand);
+    block_add2(counters + 0, nullptr, n_cand, counters + 1, 0u);
 }
 
 // The reference formulation of one item, operation for operation.  Persistent
@@ -817,7 +839,7 @@ __global__ void __launch_bounds__(128, 6) k_items_screen(const dev_pj pj, const 
         it_i = ri.x, ei = ri.y;
         it_j = rj.x, ej = rj.y;
     }
-    unsigned long long n_items = 0, n_pruned = 0;
+    unsigned n_items = 0, n_pruned = 0; // a thread has fewer than 2^32 items
     uint32_t budget = (ei - it_i) + (ej - it_j);
     // Warp-synchronous loop as in k_items (bounded the same way).
     for (;;) {
@@ -854,9 +876,7 @@ __global__ void __launch_bounds__(128, 6) k_items_screen(const dev_pj pj, const 
             --budget;
         }
     }
-    warp_add(counters + 0, n_items);
-    warp_add(item_count, n_items);
-    warp_add(counters + 1, n_pruned);
+    block_add2(counters + 0, item_count, n_items, counters + 1, n_pruned);
 }
 
 template <int OP1>

@@ -80,13 +80,12 @@ void launch_broad_half(const float *srt_aabbs, const bvh_node *trees, uint64_t c
                        const uint32_t *tree_size, const int32_t *otypes, uint32_t s_first, uint32_t nb, uint64_t N,
                        uint32_t *counts, uint2 *qpair, uint32_t *qrank, uint64_t qcap, unsigned long long *qcount,
                        unsigned long long *walk_next, int walk, unsigned long long *visits, cudaStream_t stream);
-void launch_broad_lists(uint32_t nb, uint64_t N, const uint32_t *counts, const uint64_t *offs, const uint2 *qpair,
-                        const uint32_t *qrank, uint64_t n_pairs, uint2 *pairs, uint32_t *longer,
-                        unsigned long long *n_longer, cudaStream_t stream);
-void launch_scan(const uint32_t *counts, uint64_t n, uint64_t *offs, uint64_t *block_sums, uint64_t *total,
-                 cudaStream_t stream);
-void launch_step_offsets(const uint64_t *offs, uint64_t N, uint32_t nb, const uint64_t *total, uint64_t *step_off,
-                         cudaStream_t stream);
+void launch_pair_offsets(const uint32_t *counts, uint64_t N, uint32_t nb, uint32_t *offs, uint64_t *step_tot,
+                         uint64_t *step_off, uint64_t *host_off, const unsigned long long *visits,
+                         unsigned long long *host_visits, cudaStream_t stream);
+void launch_broad_lists(uint32_t nb, uint64_t N, const uint32_t *counts, const uint32_t *offs,
+                        const uint64_t *step_off, const uint2 *qpair, const uint32_t *qrank, uint64_t n_pairs,
+                        uint2 *pairs, uint32_t *longer, unsigned long long *n_longer, cudaStream_t stream);
 void launch_items(const dev_pj &pj, const double2 *cdb, uint32_t s_first, uint32_t nb, const uint2 *pairs,
                   const uint64_t *step_off, const uint2 *srange, uint64_t n_pairs, np_item *items, uint64_t cap,
                   unsigned long long *item_count, unsigned long long *counters, dev_status *st, cudaStream_t stream);

@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cerrno>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -862,6 +863,12 @@ struct host_mailbox {
         used = off + count * sizeof(T);
         return reinterpret_cast<T *>(h + off);
     }
+    // The device's address of a host area taken above.
+    template <typename T>
+    T *device(T *host_area) const
+    {
+        return reinterpret_cast<T *>(d + (reinterpret_cast<char *>(host_area) - h));
+    }
     // One launch copying device arrays into areas taken above.
     struct batch {
         host_mailbox &m;
@@ -884,6 +891,25 @@ struct host_mailbox {
         }
     };
     batch start() { return batch{*this}; }
+};
+
+// Device counters of a batch.  Each one that many warps add to has a line of
+// its own: side by side, the L2 serialised them (merge walk with the distance
+// screen of 60,000 objects x 48 steps 1.7 -> 3.1 ms).
+struct lone_counter {
+    unsigned long long v, pad[15];
+};
+struct narrow_counters {
+    // Items, root items, conjunctions, items for the full working list, left
+    // by the filter, past the distance screen.
+    lone_counter items, roots, conj, retry, surv, cand;
+    // The report's seven and the items the filter settled as single minima.
+    unsigned long long np[8], pad[8];
+};
+struct batch_counters {
+    lone_counter qcount, walk_next, visits; // zero before the walk (again)
+    narrow_counters narrow;                 // zero before the narrow phase (again)
+    lone_counter more, n_longer;
 };
 
 // The streams and events of one screening call: the device's cached set
@@ -963,13 +989,10 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     uint64_t tree_cursor = 0;
     // Host areas of the per-batch read-backs (see host_mailbox).
     const uint64_t nb_cap = std::max<uint64_t>(1, std::min<uint64_t>(S, spb));
-    host_mailbox mbox(lease.cache, nb_cap * 4 + (nb_cap + 1) * 8 + 1024);
+    host_mailbox mbox(lease.cache, nb_cap * 4 + (nb_cap + 1) * 8 + sizeof(narrow_counters) + 1024);
     uint32_t *h_tsz_pin = mbox.take<uint32_t>(nb_cap);
     uint64_t *h_so = mbox.take<uint64_t>(nb_cap + 1);
-    // Queue counts: items, root items, conjunctions, screened, left by the
-    // filter, then the 7 narrow-phase counters and the items that the filter
-    // settled as single minima.
-    unsigned long long *h_q = mbox.take<unsigned long long>(5 + 8);
+    narrow_counters *h_q = mbox.take<narrow_counters>(1);
     dev_status *h_status = mbox.take<dev_status>(1);
     unsigned long long *h_bad = mbox.take<unsigned long long>(1);
     unsigned long long *h_visits = mbox.take<unsigned long long>(1);
@@ -1006,11 +1029,8 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         cdb[kk] = make_double2(b, e);
         R.cd_end[kk] = e;
     }
-    dbuf<double2> d_cdb(SL());
-    d_cdb.alloc(S, st);
     // Tables of the narrow phase: nodes, inverse node differences, inverse
     // binomials, binomials of the translation.
-    dbuf<double> d_tab(SL());
     std::vector<double> h_tab;
     {
         const int op1 = pj.order + 1, n = pj.order;
@@ -1029,20 +1049,23 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         for (int k = 0; k < op1; ++k)
             for (int i = 0; i + k < op1; ++i)
                 sh[size_t(k) * op1 + i] = (k == 0 || i == 0) ? 1.0 : sh[size_t(k) * op1 + i - 1] + sh[size_t(k - 1) * op1 + i];
-        d_tab.alloc(h_tab.size(), st);
-        CK(cudaMemcpyAsync(d_tab.p, h_tab.data(), h_tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     }
-    const double *filter_tab = d_tab.p;
+    // One block and one copy for the step bounds, the tables and the object
+    // types (pageable memory: the copy has read it, or waits until it has,
+    // before the call returns).
+    const size_t at_tab = S * sizeof(double2), at_ot = at_tab + h_tab.size() * sizeof(double);
+    std::vector<char> h_in(at_ot + N * sizeof(int32_t));
+    std::memcpy(h_in.data(), cdb.data(), at_tab);
+    std::memcpy(h_in.data() + at_tab, h_tab.data(), at_ot - at_tab);
+    if (otypes_host) std::memcpy(h_in.data() + at_ot, otypes_host, N * sizeof(int32_t));
+    else std::fill_n(reinterpret_cast<int32_t *>(h_in.data() + at_ot), N, 1);
+    dbuf<char> d_in(SL());
+    d_in.alloc(h_in.size(), st);
+    CK(cudaMemcpyAsync(d_in.p, h_in.data(), h_in.size(), cudaMemcpyHostToDevice, st));
+    const double2 *d_cdb = reinterpret_cast<const double2 *>(d_in.p);
+    const double *filter_tab = reinterpret_cast<const double *>(d_in.p + at_tab);
+    const int32_t *d_ot = reinterpret_cast<const int32_t *>(d_in.p + at_ot);
     const filter_limits filter_lim = make_filter_limits(pj.order + 1);
-    CK(cudaMemcpyAsync(d_cdb.p, cdb.data(), S * sizeof(double2), cudaMemcpyHostToDevice, st));
-    dbuf<int32_t> d_ot(SL());
-    d_ot.alloc(N, st);
-    {
-        std::vector<int32_t> ot(N, 1);
-        if (otypes_host) std::memcpy(ot.data(), otypes_host, N * sizeof(int32_t));
-        CK(cudaMemcpyAsync(d_ot.p, ot.data(), N * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-        CK(cudaStreamSynchronize(st));
-    }
 
     tr.mark("inputs on the device", std::to_string(N) + " objects, " + std::to_string(S) + " steps, "
                                         + std::to_string(spb) + " per batch");
@@ -1082,76 +1105,62 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
 
     // Batch scratch.
     const uint32_t nb_max = uint32_t(std::min<uint64_t>(S, spb));
-    dbuf<uint64_t> keys_a(SL()), offs(SL()), block_sums(SL()), step_off(SL()), total(SL());
-    dbuf<uint32_t> vals_a(SL()), vals_b(SL()), counts(SL()), aux(SL()), cc_cnt(SL()), cc_off(SL()), cc_ch(SL()), cc_cur(SL());
+    dbuf<uint64_t> keys_a(SL()), step_tot(SL()), step_off(SL());
+    dbuf<uint32_t> offs(SL());
+    dbuf<uint32_t> vals_a(SL()), vals_b(SL()), aux(SL()), cc_cnt(SL()), cc_off(SL()), cc_ch(SL()), cc_cur(SL());
     dbuf<int32_t> ropes(SL());
     dbuf<walk_node> walks(SL());
     dbuf<dev_status> d_st(SL());
-    dbuf<unsigned long long> visits(SL()); // broad-phase node visits of the batch
-    dbuf<unsigned long long> ctr(SL()), rq_count(SL()), cq_count(SL());
+    // The batch's device counters, and behind them the pair counts per (step,
+    // object): one memset clears them all.
+    constexpr size_t counters_bytes = (sizeof(batch_counters) + 255) & ~size_t(255);
+    dbuf<char> zeroed(SL());
+    zeroed.alloc(counters_bytes + uint64_t(nb_max) * N * sizeof(uint32_t), st);
+    batch_counters *const C = reinterpret_cast<batch_counters *>(zeroed.p); // device addresses
+    uint32_t *const counts = reinterpret_cast<uint32_t *>(zeroed.p + counters_bytes);
     keys_a.alloc(uint64_t(nb_max) * N, st);
     vals_a.alloc(uint64_t(nb_max) * N, st);
     vals_b.alloc(uint64_t(nb_max) * N, st);
     dbuf<uint2> more(SL());
     dbuf<uint2> srange(SL());
-    dbuf<unsigned long long> more_count(SL());
     // Mixed form: two distance-screen models (2 x 16 bytes each) per object
     // and step of the batch, written by the AABB pass.
     dbuf<float4> scr(SL());
     if (mixed) scr.alloc(uint64_t(nb_max) * N * 4, st);
     more.alloc(uint64_t(nb_max) * N, st);
     srange.alloc(uint64_t(nb_max) * N, st);
-    more_count.alloc(1, st);
     ropes.alloc(uint64_t(nb_max) * R.cap, st);
     walks.alloc(uint64_t(nb_max) * R.cap, st);
     const uint64_t aux_step = bvh_aux_words(N, R.cap);
     aux.alloc(uint64_t(nb_max) * aux_step, st);
-    counts.alloc(uint64_t(nb_max) * N, st);
     dbuf<uint32_t> leaf_of(SL()), longer(SL());
-    dbuf<unsigned long long> n_longer(SL());
     leaf_of.alloc(uint64_t(nb_max) * N, st);
     longer.alloc(uint64_t(nb_max) * N, st);
-    n_longer.alloc(1, st);
     // The batch's pair queue: one pair per object and step to begin with
     // (half of that on the 20,000-object day); a batch with more grows it and
     // walks again, and later calls keep the larger block.
     dbuf<uint2> qpair(SL());
     dbuf<uint32_t> qrank(SL());
-    dbuf<unsigned long long> qcount(SL());
-    dbuf<unsigned long long> walk_next(SL());
     qpair.alloc_queue(std::max<uint64_t>(1 << 16, uint64_t(nb_max) * N), st);
     qrank.alloc_queue(std::max<uint64_t>(1 << 16, uint64_t(nb_max) * N), st);
-    qcount.alloc(1, st);
-    walk_next.alloc(1, st);
     offs.alloc(uint64_t(nb_max) * N, st);
-    block_sums.alloc((uint64_t(nb_max) * N + 1023) / 1024 + 1, st);
+    step_tot.alloc(nb_max, st);
     step_off.alloc(nb_max + 1, st);
-    total.alloc(1, st);
     d_st.alloc(1, st);
-    ctr.alloc(8, st);
-    rq_count.alloc(1, st);
-    cq_count.alloc(1, st);
     cc_cnt.alloc(nb_max + 1, st);
     cc_off.alloc(nb_max + 1, st);
     cc_ch.alloc(nb_max + 1, st);
     cc_cur.alloc(nb_max + 1, st);
     CK(cudaMemsetAsync(d_st.p, 0, sizeof(dev_status), st));
-    visits.alloc(1, st);
 
     dbuf<root_item> rq(SL());
     dbuf<np_item> items(SL()), surv(SL()), cand(SL());
-    dbuf<unsigned long long> item_count(SL()), surv_count(SL()), cand_count(SL());
-    item_count.alloc(1, st);
-    surv_count.alloc(1, st);
-    cand_count.alloc(1, st);
     const unsigned narrow_grid = 148 * 6;
     dbuf<conj_out> cq(SL());
     dbuf<uint64_t> ckey(SL());
     dbuf<uint32_t> cidx(SL());
     dbuf<double> wl(SL()), wl_full(SL());
     dbuf<uint32_t> retry(SL());
-    dbuf<unsigned long long> retry_count(SL());
-    retry_count.alloc(1, st);
     const unsigned roots_grid = 148 * 4, roots_grid_full = 8;
     const uint64_t ent = uint64_t(pj.order) + 3; // (lb, ub, order + 1 coefficients)
     wl.alloc(uint64_t(roots_grid) * 128 * ROOTS_WL_SMALL * ent, st);
@@ -1159,9 +1168,12 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
 
     tr.mark("batch scratch allocated");
     tr.dev_mark("origin", st);
+    // Stages that follow one another directly share the event between them.
     std::vector<event_pair> ev;
     ev.reserve(7);
-    for (int k = 0; k < 7; ++k) ev.emplace_back(cst.ev[2 * k], cst.ev[2 * k + 1]);
+    for (const auto &e : {std::pair(0, 1), std::pair(1, 2), std::pair(2, 3), std::pair(3, 4), std::pair(5, 6),
+                          std::pair(6, 7), std::pair(8, 9)})
+        ev.emplace_back(cst.ev[e.first], cst.ev[e.second]);
     // Queue entries per broad-phase pair seen so far in this call (items,
     // root items, conjunctions): the next batch's queues are sized from
     // them, since an overflow reruns the batch's narrow phase and root
@@ -1174,13 +1186,12 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     // in flight (mzb_pj_create_async): the segments this stream has waited
     // for are flagged by now, and a non-finite trajectory value is the
     // reference's constructor error, which comes before any screening error.
-    auto check_status = [&]() {
+    auto add_status = [&](host_mailbox::batch &job) {
         *h_bad = ~0ull;
-        auto job = mbox.start();
         job.add(h_status, d_st.p, 1);
         if (pj.async_upload()) job.add(h_bad, static_cast<const unsigned long long *>(pj.bad_seg.p), 1);
-        job.launch(st);
-        CK(cudaStreamSynchronize(st));
+    };
+    auto check_status = [&]() { // once the copies have arrived
         const dev_status h = *h_status;
         pj.throw_if_bad(*h_bad);
         if (h.code != 0) {
@@ -1195,11 +1206,11 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         pj.wait_upload(st, R.cd_end[s0 + nb - 1]);
         const std::string bname = "batch " + std::to_string(s0) + "+" + std::to_string(nb);
         tr.dev_mark(bname + ": its upload chunks in", st);
+        CK(cudaMemsetAsync(zeroed.p, 0, counters_bytes + uint64_t(nb) * N * sizeof(uint32_t), st));
         CK(cudaEventRecord(ev[0].a, st));
-        launch_aabb(P, d_cdb.p, mixed, sf, nb, radius, R.aabbs.p, more.p, more_count.p,
+        launch_aabb(P, d_cdb, mixed, sf, nb, radius, R.aabbs.p, more.p, &C->more.v,
                     mixed ? scr.p : nullptr, srange.p, d_st.p, st);
         CK(cudaEventRecord(ev[0].b, st));
-        CK(cudaEventRecord(ev[1].a, st));
         launch_morton(R.aabbs.p, sf, nb, N, R.mcodes.p, st);
         launch_sort(R.aabbs.p, R.mcodes.p, sf, nb, N, keys_a.p, vals_a.p, vals_b.p, R.srt_idx.p,
                     R.srt_mcodes.p, R.srt_aabbs.p, sort_threads, st);
@@ -1213,7 +1224,6 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             stream_rows(dst->srt_mcodes, R.srt_mcodes.p, N * sizeof(uint64_t), s0, nb);
             stream_rows(dst->srt_idx, R.srt_idx.p, N * sizeof(uint32_t), s0, nb);
         }
-        CK(cudaEventRecord(ev[2].a, st));
         launch_bvh(R.srt_aabbs.p, R.srt_mcodes.p, sf, nb, N, R.trees.p, R.cap, ropes.p, aux.p, leaf_of.p,
                    R.tree_size.p, walks.p, d_st.p, bvh_threads, st);
         CK(cudaEventRecord(ev[2].b, st));
@@ -1248,24 +1258,18 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         uint64_t n_narrow_launches = 0, n_roots_launches = 0, n_broad_launches = 0, n_conj_launches = 0;
         // Mailbox read-backs of the batch: the status word, the tree sizes,
         // the pair counts and one per narrow-phase run.
-        uint64_t n_mbox = want_trees ? 2 : 1;
+        uint64_t n_mbox = (want_trees ? 1 : 0) + (skip_cd ? 1 : 0);
         if (!skip_cd) {
-            CK(cudaEventRecord(ev[3].a, st));
             uint64_t np_batch = 0;
             for (bool again = true; again;) {
                 const uint64_t qcap = std::min(qpair.n, qrank.n);
-                CK(cudaMemsetAsync(visits.p, 0, sizeof(unsigned long long), st));
                 launch_broad_half(R.srt_aabbs.p, R.trees.p, R.cap, ropes.p, walks.p, leaf_of.p, R.srt_idx.p,
-                                  R.tree_size.p, d_ot.p, sf, nb, N, counts.p, qpair.p, qrank.p, qcap, qcount.p,
-                                  walk_next.p, broad_walk, visits.p, st);
-                launch_scan(counts.p, uint64_t(nb) * N, offs.p, block_sums.p, total.p, st);
-                launch_step_offsets(offs.p, N, nb, total.p, step_off.p, st);
-                mbox.start()
-                    .add(h_so, static_cast<const uint64_t *>(step_off.p), nb + 1)
-                    .add(h_visits, static_cast<const unsigned long long *>(visits.p), 1)
-                    .launch(st);
-                ++n_mbox;
-                n_broad_launches += 5;
+                                  R.tree_size.p, d_ot, sf, nb, N, counts, qpair.p, qrank.p, qcap, &C->qcount.v,
+                                  &C->walk_next.v, broad_walk, &C->visits.v, st);
+                launch_pair_offsets(counts, N, nb, offs.p, step_tot.p, step_off.p, mbox.device(h_so), &C->visits.v,
+                                    mbox.device(h_visits), st);
+                CK(cudaGetLastError());
+                n_broad_launches += 3;
                 CK(cudaStreamSynchronize(st));
                 np_batch = h_so[nb];
                 if (np_batch >= (1ull << 32)) throw std::runtime_error("too many broad-phase pairs in one batch");
@@ -1273,6 +1277,8 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 if (again) {
                     qpair.alloc_queue(np_batch + np_batch / 8, st);
                     qrank.alloc_queue(np_batch + np_batch / 8, st);
+                    CK(cudaMemsetAsync(C, 0, offsetof(batch_counters, narrow), st));
+                    CK(cudaMemsetAsync(counts, 0, uint64_t(nb) * N * sizeof(uint32_t), st));
                 }
             }
             R.broad_visits += *h_visits;
@@ -1292,8 +1298,8 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             if (R.bp.n < R.n_bp + np_batch)
                 R.bp.grow(std::max(R.n_bp + np_batch, whole_call(R.n_bp + np_batch)), R.n_bp, st);
             uint2 *bp_batch = R.bp.p + R.n_bp;
-            launch_broad_lists(nb, N, counts.p, offs.p, qpair.p, qrank.p, np_batch, bp_batch, longer.p, n_longer.p,
-                               st);
+            launch_broad_lists(nb, N, counts, offs.p, step_off.p, qpair.p, qrank.p, np_batch, bp_batch, longer.p,
+                               &C->n_longer.v, st);
             if (np_batch) n_broad_launches += 3;
             CK(cudaEventRecord(ev[3].b, st));
             for (uint32_t b = 0; b < nb; ++b) {
@@ -1326,57 +1332,48 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             tr.mark("pair list and queues allocated", std::to_string(np_batch) + " pairs");
             unsigned long long h_rq = 0, h_items = 0, h_cq = 0, h_ctr[8] = {}, h_cand = 0, h_surv = 0;
             for (;;) {
-                CK(cudaMemsetAsync(ctr.p, 0, 8 * sizeof(unsigned long long), st));
-                CK(cudaMemsetAsync(rq_count.p, 0, sizeof(unsigned long long), st));
-                CK(cudaMemsetAsync(item_count.p, 0, sizeof(unsigned long long), st));
-                CK(cudaMemsetAsync(cq_count.p, 0, sizeof(unsigned long long), st));
-                CK(cudaMemsetAsync(retry_count.p, 0, sizeof(unsigned long long), st));
                 CK(cudaEventRecord(ev[4].a, st));
-                CK(cudaMemsetAsync(surv_count.p, 0, sizeof(unsigned long long), st));
                 if (mixed) {
                     // Items screened as the merge walk finds them.
-                    CK(cudaMemsetAsync(cand_count.p, 0, sizeof(unsigned long long), st));
-                    launch_items_screen(P, d_cdb.p, sf, nb, bp_batch, step_off.p, srange.p, np_batch, thresh, scr.p,
-                                        cand.p, cand.n, cand_count.p, item_count.p, ctr.p, d_st.p, st);
+                    launch_items_screen(P, d_cdb, sf, nb, bp_batch, step_off.p, srange.p, np_batch, thresh, scr.p,
+                                        cand.p, cand.n, &C->narrow.cand.v, &C->narrow.items.v, C->narrow.np,
+                                        d_st.p, st);
                 } else {
-                    launch_items(P, d_cdb.p, sf, nb, bp_batch, step_off.p, srange.p, np_batch, items.p, items.n,
-                                 item_count.p, ctr.p, d_st.p, st);
+                    launch_items(P, d_cdb, sf, nb, bp_batch, step_off.p, srange.p, np_batch, items.p, items.n,
+                                 &C->narrow.items.v, C->narrow.np, d_st.p, st);
                 }
                 // The FMA filter, then the reference formulation on the items
                 // it leaves.
                 const dbuf<np_item> &src = mixed ? cand : items;
-                launch_narrow_filter(P, filter_tab, filter_lim, d_cdb.p, sf, src.p,
-                                     mixed ? cand_count.p : item_count.p, src.n, thresh2, surv.p, surv.n,
-                                     surv_count.p, ctr.p, st);
-                launch_narrow(P, filter_tab, d_cdb.p, sf, surv.p, surv_count.p, surv.n, thresh2, rq.p, rq.n, rq_count.p, ctr.p,
+                launch_narrow_filter(P, filter_tab, filter_lim, d_cdb, sf, src.p,
+                                     mixed ? &C->narrow.cand.v : &C->narrow.items.v, src.n, thresh2, surv.p, surv.n,
+                                     &C->narrow.surv.v, C->narrow.np, st);
+                launch_narrow(P, filter_tab, d_cdb, sf, surv.p, &C->narrow.surv.v, surv.n, thresh2, rq.p, rq.n,
+                              &C->narrow.roots.v, C->narrow.np,
                               d_st.p, narrow_grid, st);
                 CK(cudaEventRecord(ev[4].b, st));
-                CK(cudaEventRecord(ev[5].a, st));
-                launch_roots(P, rq.p, rq_count.p, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL, roots_grid,
-                             retry.p, retry_count.p, cq.p, cq.n, cq_count.p, ctr.p, d_st.p, st);
-                launch_roots(P, rq.p, rq_count.p, rq.n, retry.p, retry_count.p, thresh2, wl_full.p, ROOTS_WL_FULL,
-                             roots_grid_full, nullptr, nullptr, cq.p, cq.n, cq_count.p, ctr.p, d_st.p, st);
+                launch_roots(P, rq.p, &C->narrow.roots.v, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL,
+                             roots_grid, retry.p, &C->narrow.retry.v, cq.p, cq.n, &C->narrow.conj.v, C->narrow.np, d_st.p, st);
+                launch_roots(P, rq.p, &C->narrow.roots.v, rq.n, retry.p, &C->narrow.retry.v, thresh2, wl_full.p,
+                             ROOTS_WL_FULL, roots_grid_full, nullptr, nullptr, cq.p, cq.n, &C->narrow.conj.v,
+                             C->narrow.np, d_st.p, st);
                 CK(cudaEventRecord(ev[5].b, st));
                 n_narrow_launches += 3;
                 n_roots_launches += 2;
                 {
                     auto job = mbox.start();
-                    job.add(h_q + 0, static_cast<const unsigned long long *>(item_count.p), 1)
-                        .add(h_q + 1, static_cast<const unsigned long long *>(rq_count.p), 1)
-                        .add(h_q + 2, static_cast<const unsigned long long *>(cq_count.p), 1)
-                        .add(h_q + 4, static_cast<const unsigned long long *>(surv_count.p), 1)
-                        .add(h_q + 5, static_cast<const unsigned long long *>(ctr.p), 8);
-                    if (mixed) job.add(h_q + 3, static_cast<const unsigned long long *>(cand_count.p), 1);
+                    job.add(h_q, static_cast<const narrow_counters *>(&C->narrow), 1);
+                    add_status(job);
                     job.launch(st);
                     ++n_mbox;
                 }
                 CK(cudaStreamSynchronize(st));
-                h_items = h_q[0];
-                h_rq = h_q[1];
-                h_cq = h_q[2];
-                h_cand = mixed ? h_q[3] : 0;
-                h_surv = h_q[4];
-                for (int k = 0; k < 8; ++k) h_ctr[k] = h_q[5 + k];
+                h_items = h_q->items.v;
+                h_rq = h_q->roots.v;
+                h_cq = h_q->conj.v;
+                h_surv = h_q->surv.v;
+                h_cand = h_q->cand.v;
+                for (int k = 0; k < 8; ++k) h_ctr[k] = h_q->np[k];
                 tr.mark("narrow phase and root finding run",
                         std::to_string(h_items) + " items, " + std::to_string(h_rq) + " root items, "
                             + std::to_string(h_cq) + " conjunctions");
@@ -1400,7 +1397,9 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                     again = true;
                 }
                 if (!again) break;
+                CK(cudaMemsetAsync(&C->narrow, 0, sizeof(narrow_counters), st));
             }
+            check_status(); // the ordering below sets no error
             if (np_batch) {
                 items_per_pair = std::max(items_per_pair, double(h_items) / double(np_batch));
                 roots_per_pair = std::max(roots_per_pair, double(h_rq) / double(np_batch));
@@ -1426,14 +1425,20 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             R.n_conj += h_cq;
             t_bp = ev[3].ms();
         }
-        // aabb (2 passes + global box) + morton + sort + bvh; broad half walk, 3 scan kernels,
-        // step offsets, scatter + list sorts,
+        // aabb (2 passes + global box) + morton + sort + bvh (+ walk nodes); broad half walk,
+        // 2 offset kernels, scatter + list sorts,
         // items + filter + narrow, roots (+ retry), conj-order kernels.
         R.n_launches += 6 + n_mbox;
         if (!skip_cd) R.n_launches += n_broad_launches + n_narrow_launches + n_roots_launches + n_conj_launches;
         tr.dev_mark(bname + ": screened", st);
         if (dst) tr.dev_mark(bname + ": per-step outputs copied", cs);
-        check_status();
+        if (skip_cd) {
+            auto job = mbox.start();
+            add_status(job);
+            job.launch(st);
+        }
+        CK(cudaStreamSynchronize(st));
+        if (skip_cd) check_status();
         if (tr.on) {
             char b[160];
             std::snprintf(b, sizeof(b), "aabb %.3f, morton+sort %.3f, bvh %.3f, broad %.3f, narrow %.3f, roots %.3f, "
