@@ -250,8 +250,9 @@ uint64_t mzb_result_n_launches(const mzb_result *r);
  * that repeated calls allocate nothing; a freed result's block of per-step
  * outputs is also kept, as the spare the next call of the same size takes.
  * This returns the current device's cached blocks and spare to the
- * stream-ordered pool; it waits for a screening call in progress on the
- * device to finish.  No counterpart in the reference (its buffers are host
+ * stream-ordered pool, and frees the pinned buffers (32 MB at most) that
+ * copies to pageable memory and files keep; it waits for a screening call in
+ * progress on the device to finish.  No counterpart in the reference (its buffers are host
  * memory owned by each call). */
 int mzb_scratch_release(void);
 /* Bytes of batch scratch and spare output block cached on the current
