@@ -1042,7 +1042,8 @@ __device__ __forceinline__ bool fex_excludes_t(const double (&p)[OP1], double h)
     return lo > 0 || hi < 0;
 }
 
-// ---- TOMS 748 (Alefeld, Potra, Shi 1995, Algorithm 4.2) on horner(p, .).
+// ---- TOMS 748 (Alefeld, Potra, Shi 1995, Algorithm 4.2) on st.f, which
+// evaluates the polynomial and counts its calls in st.evals.
 template <int OP1>
 struct toms_t {
     const double (&p)[OP1];
@@ -1085,11 +1086,10 @@ __device__ void bracket_at_t(ST &st, double &a, double &b, double c, double &fa,
 
 // Returns the flag (0 ok, 33 = EDOM for a non-bracketing interval, -1 for an
 // exhausted budget of 100 evaluations) and the root in *root.
-template <int OP1>
-__device__ int toms748_t(const double (&p)[OP1], double lo, double hi, double *root)
+template <typename ST>
+__device__ int toms748_t(ST &st, double lo, double hi, double *root)
 {
     constexpr int budget = 100;
-    toms_t<OP1> st{p, 0};
     double a = lo, b = hi;
     double fa = st.f(a), fb = st.f(b);
     if (!(a < b)) return 33;
@@ -1164,12 +1164,254 @@ __device__ void states_at_t(const dev_pj &pj, uint64_t gseg, double delta, doubl
     }
 }
 
+// ---- One item by one warp (OP1 <= 32), for launches with few items.
+//
+// One thread takes 45 to 70 us for an item however few there are: a chain of
+// Taylor shifts, evaluations and, for a conjunction, twelve translated
+// polynomials one after the other.  Here lane I computes coefficient I of a
+// shift, lanes 0 to 11 one state variable each, and all lanes run the scalar
+// part (fast exclusion, TOMS 748) on coefficients in shared memory; every
+// value comes from the same operations in the same order.  52 items 46 -> 23
+// us, 2,500 sub-intervals' left-overs of the 1,000-object day 73 -> 28 us;
+// beyond one item a resident warp (2,368 of them) the thread per item is as
+// fast and keeps all lanes busy (11,000 items: 79 against 95 us).
+constexpr uint64_t ROOTS_WARP_ITEMS = 2048;
+constexpr int ROOTS_T = 128;
+
+template <int OP1>
+struct roots_smem {
+    double pt[OP1], d[OP1], sp[OP1]; // dist^2, its derivative, the derivative on [0, 1]
+    double roots[MAX_ROOTS], isol[OP1 + 1][2];
+};
+
+__device__ __noinline__ double horner_smem(const double *p, int n, double x)
+{
+    double r = p[n];
+#pragma unroll 4
+    for (int k = n - 1; k >= 0; --k) r = p[k] + r * x;
+    return r;
+}
+struct toms_smem {
+    const double *p;
+    int n, evals;
+    __device__ double f(double x)
+    {
+        ++evals;
+        return horner_smem(p, n, x);
+    }
+};
+
+// Taylor shift by 1 of the polynomial whose coefficient I lane I holds (see
+// narrow_by_warp for the table and the sums).
+template <int OP1>
+__device__ __noinline__ double shift1_by_warp(const double *__restrict__ shift, double c)
+{
+    constexpr int n = OP1 - 1;
+    const unsigned lane = threadIdx.x & 31;
+    double t[OP1];
+#pragma unroll
+    for (int k = 0; k < OP1; ++k) {
+        const double ck = __shfl_down_sync(0xffffffffu, c, k);
+        t[k] = lane + k <= n ? __ldg(shift + k * OP1 + lane) * ck : -0.0;
+    }
+    return pw<OP1>::reduce(t, add_op{});
+}
+
+// counts: root findings, fast exclusions, without a root, minima, discarded.
+template <int OP1>
+__device__ __forceinline__ void roots_by_warp(const dev_pj &pj, const double *__restrict__ shift, const root_item &q,
+                                              double thresh2, double *__restrict__ wl, roots_smem<OP1> &S,
+                                              conj_out *__restrict__ cq, uint64_t cq_cap,
+                                              unsigned long long *cq_count, unsigned (&counts)[5], dev_status *st)
+{
+    constexpr int n = OP1 - 1;
+    constexpr int ENT = OP1 + 2;
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31;
+    const bool in = lane < OP1;
+    const double rf_int = q.rf_int;
+    const double pt = in ? q.ptd2[lane] : 0.0;
+    const double d2 = __shfl_down_sync(ALL, pt, 1);
+    const double d = lane < unsigned(n) ? (lane + 1u) * d2 : 0.0;
+    double fct = 1; // rf_int^lane, by repeated multiplication
+#pragma unroll 1
+    for (int k = 0; k < n; ++k)
+        if (int(lane) > k) fct *= rf_int;
+    __syncwarp();
+    if (in) {
+        S.pt[lane] = pt;
+        S.d[lane] = d;
+        S.sp[lane] = fct * d;
+    }
+    __syncwarp();
+    int nroots = 0;
+    bool failed = false;
+    auto error = [&](int code, double x, double y) {
+        if (lane == 0) set_error(st, code, q.i, q.j, x, y);
+        failed = true;
+    };
+    auto add_root = [&](double root) {
+        if (!isfinite(root)) {
+            error(ERR_ROOT_NONFINITE, root, 0);
+            return;
+        }
+        double der = S.d[n] * n;
+#pragma unroll 1
+        for (int i = 1; i < n; ++i) der = S.d[n - i] * (n - i) + der * root;
+        if (!isfinite(der)) {
+            error(ERR_ROOT_DER, root, der);
+            return;
+        }
+        if (sgn(der) == 1) {
+            if (nroots < MAX_ROOTS) {
+                if (lane == 0) S.roots[nroots] = root;
+                ++nroots;
+            } else {
+                error(ERR_ISOLATION, MAX_ROOTS, 0);
+            }
+        }
+    };
+    // Fast exclusion: interval Horner over [0, rf_int].
+    bool fex;
+    {
+        double lo = S.d[n], hi = lo;
+#pragma unroll 1
+        for (int o = 1; o <= n; ++o) {
+            const double a = lo * rf_int, b = hi * rf_int;
+            const double plo = fmin(0., fmin(a, b)), phi = fmax(0., fmax(a, b));
+            lo = S.d[n - o] + plo;
+            hi = S.d[n - o] + phi;
+        }
+        fex = lo > 0 || hi < 0;
+    }
+    if (!fex) {
+        if (lane == 0) wl[0] = 0, wl[1] = 1;
+        if (in) wl[2 + lane] = fct * d;
+        int wsz = 1, nisol = 0;
+        do {
+            --wsz;
+            __syncwarp();
+            const double *ent = wl + uint64_t(wsz) * ENT;
+            const double lb = ent[0], ub = ent[1];
+            const double cur = in ? ent[2 + lane] : 0.0;
+            const bool tail_finite = __all_sync(ALL, lane == 0 || !in || isfinite(cur));
+            if (__shfl_sync(ALL, cur, 0) == 0 && tail_finite) add_root(lb * rf_int);
+            const double r2 = shift1_by_warp<OP1>(shift, __shfl_sync(ALL, cur, (n - lane) & 31));
+            // Descartes sign changes, zeros skipped.
+            const int sg = in ? sgn(r2) : 0;
+            const unsigned pos = __ballot_sync(ALL, sg > 0), nz = __ballot_sync(ALL, sg != 0);
+            const unsigned before = nz & lanemask_lt();
+            const bool change = sg != 0 && before && ((pos >> lane) & 1u) != ((pos >> (31 - __clz(before))) & 1u);
+            const int nsc = __popc(__ballot_sync(ALL, change));
+            if (nsc == 1) {
+                if (nisol < OP1 + 1 && lane == 0) S.isol[nisol][0] = lb, S.isol[nisol][1] = ub;
+                ++nisol;
+            } else if (nsc > 1) {
+                if (wsz + 2 > WL_CAP) {
+                    error(ERR_ISOLATION, wsz + 2, nisol);
+                    break;
+                }
+                const double L = in ? double(1ull << (n - lane)) * cur : 0.0;
+                const double R = shift1_by_warp<OP1>(shift, L);
+                const double mid = lb / 2 + ub / 2;
+                double *El = wl + uint64_t(wsz) * ENT, *Er = El + ENT;
+                __syncwarp(); // every lane has read the entry that El replaces
+                if (lane == 0) El[0] = lb, El[1] = mid, Er[0] = mid, Er[1] = ub;
+                if (in) El[2 + lane] = L, Er[2 + lane] = R;
+                wsz += 2;
+            }
+            if (wsz > 250 || nisol > n) {
+                error(ERR_ISOLATION, wsz, nisol);
+                break;
+            }
+        } while (wsz > 0 && !failed);
+        __syncwarp();
+        for (int r = 0; r < nisol && !failed; ++r) {
+            const double lb = S.isol[r][0];
+            double ub = S.isol[r][1];
+            if (isfinite(lb) && isfinite(ub) && ub > lb) ub = nextafter(ub, lb);
+            double root = 0;
+            toms_smem ev{S.sp, n, 0};
+            const int flag = toms748_t(ev, lb, ub, &root);
+            if (flag == -1) error(ERR_TOMS_ITER, 0, 0);
+            else if (flag != 0) error(ERR_TOMS_ERRNO, flag, 0);
+            else add_root(root * rf_int);
+        }
+    }
+    if (failed) return;
+    __syncwarp();
+    ++counts[0];
+    counts[1] += fex;
+    counts[2] += nroots == 0;
+    counts[3] += nroots;
+    // The minima below the threshold, then the boundary minima: entry nroots
+    // is the end of the data, nroots + 1 their start.
+#pragma unroll 1
+    for (int r = 0; r < nroots + 2; ++r) {
+        double tm = 0.0;
+        if (r < nroots) {
+            tm = S.roots[r];
+        } else if (r == nroots) {
+            if (!(q.flags & 1u)) continue;
+            tm = nextafter(rf_int, -1.);
+            const double dv = horner_smem(S.d, n, tm);
+            if (!isfinite(dv)) error(ERR_UB_DER, dv, 0);
+            if (!(dv < 0)) continue;
+        } else {
+            if (!(q.flags & 2u)) continue;
+            const double dv = horner_smem(S.d, n, 0.);
+            if (!isfinite(dv)) error(ERR_LB_DER, dv, 0);
+            if (!(dv > 0)) continue;
+        }
+        const double m2 = horner_smem(S.pt, n, tm);
+        if (!isfinite(m2)) {
+            error(r < nroots ? ERR_CONJ_D2 : r == nroots ? ERR_UB_D2 : ERR_LB_D2, m2, 0);
+            continue;
+        }
+        if (!(m2 < thresh2)) {
+            counts[4] += r < nroots;
+            continue;
+        }
+        // Lane o * 6 + v: variable v of object o at tm (states_at_t).
+        double x = 0;
+        if (lane < 12) {
+            const unsigned o = lane / 6, v = lane % 6;
+            const double delta = o ? q.dj : q.di;
+            double c[OP1], t[OP1];
+            load_row<OP1>(coef_row<OP1>(pj, o ? q.seg_j : q.seg_i, int(v)), c);
+            if (delta != 0) translate<OP1>(c, delta, t);
+            else
+#pragma unroll
+                for (int k = 0; k < OP1; ++k) t[k] = c[k];
+            x = horner<OP1>(t, tm);
+        }
+        const double y = __shfl_down_sync(ALL, x, 6); // the other object's
+        const double df = x - y, sq = df * df;
+        const double s1 = __shfl_sync(ALL, sq, 1), s2 = __shfl_sync(ALL, sq, 2);
+        unsigned long long slot = 0;
+        if (lane == 0) slot = atomicAdd(cq_count, 1ull);
+        slot = __shfl_sync(ALL, slot, 0);
+        if (slot < cq_cap) {
+            double *rec = reinterpret_cast<double *>(&cq[slot].c);
+            if (lane < 12) rec[3 + lane] = x; // ri, vi, rj, vj
+            if (lane == 0) {
+                cq[slot].c.i = q.i;
+                cq[slot].c.j = q.j;
+                cq[slot].c.tca = q.lb_rf + tm;
+                cq[slot].c.dca = sqrt(sq + s1 + s2);
+                cq[slot].step = q.step;
+            }
+        }
+    }
+}
+
 // wl_cap: working-list entries available per thread.  With wl_cap < 251 an
 // item whose list would outgrow it is deferred to `retry` untouched and is
 // run again with the full 251-entry list by a second, smaller launch.  The
 // item count is read on the device (persistent grid).
 template <int OP1>
-__global__ void __launch_bounds__(128) k_roots(dev_pj pj, const root_item *__restrict__ rq,
+__global__ void __launch_bounds__(ROOTS_T) k_roots(dev_pj pj, const double *__restrict__ shift,
+                                               const root_item *__restrict__ rq,
                                                const unsigned long long *rq_count, uint64_t rq_cap,
                                                const uint32_t *__restrict__ item_list,
                                                const unsigned long long *item_list_count, double thresh2,
@@ -1184,6 +1426,23 @@ __global__ void __launch_bounds__(128) k_roots(dev_pj pj, const root_item *__res
     const uint64_t tid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     const uint64_t nthreads = uint64_t(gridDim.x) * blockDim.x;
     const uint64_t n_items = item_list ? *item_list_count : min(*rq_count, (unsigned long long)rq_cap);
+    if constexpr (OP1 <= 32) {
+        // Few items: a warp each, with its lanes' working lists as one (the
+        // full list fits: 32 x ROOTS_WL_SMALL entries), so none is deferred.
+        static_assert(32 * ROOTS_WL_SMALL >= WL_CAP, "a warp's share holds the full working list");
+        if (n_items <= ROOTS_WARP_ITEMS && !item_list) {
+            __shared__ roots_smem<OP1> S[ROOTS_T / 32];
+            unsigned counts[5] = {0, 0, 0, 0, 0};
+            double *wwl = wl_scratch + (tid & ~uint64_t(31)) * uint64_t(wl_cap) * ENT;
+            for (uint64_t w = tid / 32; w < n_items; w += nthreads / 32)
+                roots_by_warp<OP1>(pj, shift, rq[w], thresh2, wwl, S[threadIdx.x >> 5], cq, cq_cap, cq_count, counts,
+                                   st);
+            if ((threadIdx.x & 31) == 0)
+                for (int k = 0; k < 5; ++k)
+                    if (counts[k]) atomicAdd(counters + 2 + k, (unsigned long long)counts[k]);
+            return;
+        }
+    }
     double *wl = wl_scratch + tid * uint64_t(wl_cap) * ENT;
     unsigned long long n_roots = 0, n_fex = 0, n_noroot = 0, n_minima = 0, n_disc = 0;
     for (uint64_t it = tid; it < n_items; it += nthreads) {
@@ -1307,7 +1566,8 @@ __global__ void __launch_bounds__(128) k_roots(dev_pj pj, const root_item *__res
                     double lb = isol_lb[r], ub = isol_ub[r];
                     if (isfinite(lb) && isfinite(ub) && ub > lb) ub = nextafter(ub, lb);
                     double root = 0;
-                    const int flag = toms748_t<OP1>(sp, lb, ub, &root);
+                    toms_t<OP1> ev{sp, 0};
+                    const int flag = toms748_t(ev, lb, ub, &root);
                     if (flag == -1) {
                         set_error(st, ERR_TOMS_ITER, q.i, q.j, 0, 0);
                         failed = true;
@@ -1737,17 +1997,18 @@ filter_limits make_filter_limits(int op1)
 }
 
 template <int OP1>
-static void roots_t(const dev_pj &pj, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+static void roots_t(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                     const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                     double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                     conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,
                     dev_status *st, cudaStream_t stream)
 {
-    k_roots<OP1><<<grid, 128, 0, stream>>>(pj, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch,
+    k_roots<OP1><<<grid, ROOTS_T, 0, stream>>>(pj, tab + OP1 * (OP1 + 2), rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch,
                                             wl_cap, retry, retry_count, cq, cq_cap, cq_count, counters, st);
 }
 
-void launch_roots(const dev_pj &pj, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+// tab: the tables of launch_narrow_filter.
+void launch_roots(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                   const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                   double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                   conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,
@@ -1756,7 +2017,7 @@ void launch_roots(const dev_pj &pj, const root_item *rq, const unsigned long lon
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        roots_t<K>(pj, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch, wl_cap, grid, retry,    \
+        roots_t<K>(pj, tab, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch, wl_cap, grid, retry,    \
                    retry_count, cq, cq_cap, cq_count, counters, st, stream);                                          \
         break;
         MZB_FOR_EACH_OP1(X)

@@ -109,7 +109,7 @@ void launch_narrow_filter(const dev_pj &pj, const double *tab, const filter_limi
                           unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream);
 constexpr int ROOTS_WL_SMALL = 24;  // working-list entries per thread, first pass
 constexpr int ROOTS_WL_FULL = 251;  // the reference's bound (list size > 250 fails)
-void launch_roots(const dev_pj &pj, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+void launch_roots(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                   const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                   double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                   conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,

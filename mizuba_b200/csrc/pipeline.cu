@@ -1354,9 +1354,9 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                               &C->narrow.roots.v, C->narrow.np,
                               d_st.p, narrow_grid, st);
                 CK(cudaEventRecord(ev[4].b, st));
-                launch_roots(P, rq.p, &C->narrow.roots.v, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL,
+                launch_roots(P, filter_tab, rq.p, &C->narrow.roots.v, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL,
                              roots_grid, retry.p, &C->narrow.retry.v, cq.p, cq.n, &C->narrow.conj.v, C->narrow.np, d_st.p, st);
-                launch_roots(P, rq.p, &C->narrow.roots.v, rq.n, retry.p, &C->narrow.retry.v, thresh2, wl_full.p,
+                launch_roots(P, filter_tab, rq.p, &C->narrow.roots.v, rq.n, retry.p, &C->narrow.retry.v, thresh2, wl_full.p,
                              ROOTS_WL_FULL, roots_grid_full, nullptr, nullptr, cq.p, cq.n, &C->narrow.conj.v,
                              C->narrow.np, d_st.p, st);
                 CK(cudaEventRecord(ev[5].b, st));
