@@ -253,8 +253,6 @@ __global__ void __launch_bounds__(BVH_T, 1024 / BVH_T) k_bvh(const float *__rest
 // std::min / std::max keep the first of equal values, so the union of a
 // node equals the left-to-right fold over its range whatever the grouping,
 // and the boxes are bit-identical to the reference's.
-constexpr int FLAT_T = 1024;
-constexpr int FLAT_W = FLAT_T / 32;
 constexpr int FLAT_LEVELS = 66; // 64 split levels below the root at most, then leaves
 constexpr int FLAT_G = 4;       // positions whose loads a thread issues together
 constexpr uint32_t NOT_ITEM = 0xFFFFFFFEu, ROOT_PARENT = 0xFFFFFFFFu;
@@ -274,12 +272,18 @@ __device__ __forceinline__ uint32_t parent_word(const uint64_t *c, uint32_t b, u
     return split_bit(c, b - 1) > split_bit(c, e - 1) ? (((b - 1) << 1) | 1u) : ((e - 1) << 1);
 }
 
-__global__ void __launch_bounds__(FLAT_T, 1)
+// FLAT_T threads a CTA, 1,024 an SM.  BVH stage, 480 steps of 1,000 objects:
+// 1,024 threads 120 us, 512 91, 256 83, 128 95; 188 steps of 3,001 objects:
+// 130, 108, 130, 189; 480 steps of 20,000: 1,700, 1,951 (shared memory for one
+// CTA an SM), 2,755.
+template <int FLAT_T>
+__global__ void __launch_bounds__(FLAT_T, 1024 / FLAT_T)
     k_bvh_flat(const float *__restrict__ srt_aabbs, const uint64_t *__restrict__ srt_mcodes, uint32_t s_first,
                uint64_t N, bvh_node *__restrict__ trees, uint64_t cap, int32_t *__restrict__ ropes,
                uint32_t *__restrict__ aux, uint32_t *__restrict__ leaf_of, uint32_t *__restrict__ tree_size,
                dev_status *st, bool codes_in_smem, bool depth_in_smem)
 {
+    constexpr int FLAT_W = FLAT_T / 32;
     extern __shared__ __align__(16) unsigned char fsm[];
     __shared__ uint32_t cnt[FLAT_W][FLAT_LEVELS];
     __shared__ uint32_t lvl_off[FLAT_LEVELS + 1];
@@ -686,8 +690,15 @@ void launch_bvh(const float *srt_aabbs, const uint64_t *srt_mcodes, uint32_t s_f
     // global scratch otherwise.
     const bool csm = N * 8 <= BVH_SMEM_CODES, dsm = N * 6 <= BVH_SMEM_CODES;
     const size_t bytes = std::max(csm ? N * 8 : 0, dsm ? N * 6 : 0);
-    k_bvh_flat<<<nb, FLAT_T, bytes, stream>>>(srt_aabbs, srt_mcodes, s_first, N, trees, cap, ropes, aux, leaf_of,
-                                              tree_size, st, csm, dsm);
+    auto launch = [&](auto *kernel, int T) {
+        kernel<<<nb, T, bytes, stream>>>(srt_aabbs, srt_mcodes, s_first, N, trees, cap, ropes, aux, leaf_of, tree_size,
+                                         st, csm, dsm);
+    };
+    // Small steps leave most of a 1,024-thread CTA idle between its barriers:
+    // smaller CTAs, several an SM, where there are steps enough for that.
+    if (N <= 1024) launch(k_bvh_flat<256>, 256);
+    else if (N <= 4096 && nb > 148) launch(k_bvh_flat<512>, 512);
+    else launch(k_bvh_flat<1024>, 1024);
     k_walk_nodes<<<dim3(unsigned((cap + 255) / 256), nb), 256, 0, stream>>>(srt_aabbs, trees, cap, ropes, tree_size,
                                                                             s_first, N, walks);
 }
@@ -702,7 +713,11 @@ cudaError_t init_bvh_attrs()
     const cudaError_t e =
         cudaFuncSetAttribute(k_bvh<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BVH_SMEM_CODES));
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_bvh_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BVH_SMEM_CODES));
+    for (auto *k : {k_bvh_flat<256>, k_bvh_flat<512>, k_bvh_flat<1024>}) {
+        const cudaError_t f = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BVH_SMEM_CODES));
+        if (f != cudaSuccess) return f;
+    }
+    return cudaSuccess;
 }
 
 } // namespace mzb

@@ -274,6 +274,74 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
     }
 }
 
+// Steps of up to SMALL_MAX objects: the whole sort in shared memory, one
+// bitonic network over (code, no-data flag and object index) per step.  A
+// no-data box has the largest code, so code, flag, index is the reference's
+// order.  The radix passes' fixed work (clearing and scanning 256 x 17
+// counters, six barriers, eight times) does not shrink with the step: Morton
+// and sort of 60 steps of 150 objects 44 -> 15 us, of 480 steps of 1,000
+// objects 142 -> 56 us.  At 3,001 objects (a network of 4,096) the radix sort
+// is ahead, 107 against 112 us for 188 steps.
+constexpr uint64_t SMALL_MAX = 2048;
+
+template <int SORT_T, int CAP>
+__global__ void __launch_bounds__(SORT_T) k_sort_small(const float *__restrict__ aabbs,
+                                                       const uint64_t *__restrict__ mcodes, uint32_t s_first,
+                                                       uint32_t N, uint32_t *__restrict__ srt_idx,
+                                                       uint64_t *__restrict__ srt_mcodes,
+                                                       float *__restrict__ srt_aabbs)
+{
+    __shared__ uint64_t key[CAP];
+    __shared__ uint16_t tie[CAP]; // bit 15: no data; below: object index
+    static_assert(CAP <= 1 << 15, "indices leave the flag's bit free");
+    const uint64_t s = uint64_t(s_first) + blockIdx.x;
+    const unsigned tid = threadIdx.x;
+    const uint64_t *mc = mcodes + s * N;
+    const float *ab = aabbs + s * (uint64_t(N) + 1) * 8;
+    uint32_t P = 1;
+    while (P < N) P <<= 1;
+    for (uint32_t i = tid; i < P; i += SORT_T) {
+        key[i] = i < N ? mc[i] : ~0ull;
+        tie[i] = uint16_t(i < N ? (isfinite(ab[uint64_t(i) * 8]) ? i : (0x8000u | i)) : 0xffffu);
+    }
+    __syncthreads();
+    auto exchange = [&](uint32_t t, uint32_t size, uint32_t stride) {
+        const uint32_t i = 2 * t - (t & (stride - 1)), j = i + stride;
+        const uint64_t ki = key[i], kj = key[j];
+        const uint16_t ti = tie[i], tj = tie[j];
+        const bool gt = ki != kj ? ki > kj : ti > tj;
+        if (gt == ((i & size) == 0)) {
+            key[i] = kj;
+            key[j] = ki;
+            tie[i] = tj;
+            tie[j] = ti;
+        }
+    };
+    for (uint32_t size = 2; size <= P; size <<= 1)
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t t = tid; t < P / 2; t += SORT_T) exchange(t, size, stride);
+            // Strides up to 32 exchange within the 64 entries that the same
+            // warp handles in the next round too.
+            if (stride > 32 || (stride == 1 && size >= 64)) __syncthreads();
+            else __syncwarp();
+        }
+    __syncthreads();
+    for (uint32_t p = tid; p < N; p += SORT_T) {
+        const uint32_t o = tie[p] & 0x7fffu;
+        srt_idx[s * N + p] = o;
+        srt_mcodes[s * N + p] = key[p];
+        const float4 *src = reinterpret_cast<const float4 *>(ab + uint64_t(o) * 8);
+        float4 *dst = reinterpret_cast<float4 *>(srt_aabbs + (s * (uint64_t(N) + 1) + p) * 8);
+        dst[0] = src[0];
+        dst[1] = src[1];
+    }
+    if (tid < 2) {
+        const float4 *src = reinterpret_cast<const float4 *>(ab + uint64_t(N) * 8);
+        float4 *dst = reinterpret_cast<float4 *>(srt_aabbs + (s * (uint64_t(N) + 1) + N) * 8);
+        dst[tid] = src[tid];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Allocation-free variant of the step sort.
 //
@@ -325,14 +393,21 @@ cudaError_t sort_step_noalloc(const float *aabbs, const uint64_t *mcodes, uint64
 
 uint64_t sort_noalloc_max_objs() { return NOALLOC_MAX_OBJS; }
 
-// threads: the CTA size, 256 or 512 (anything else: 512).  Four 256-thread
+// Up to SMALL_MAX objects: k_sort_small.  Above, threads is the radix sort's
+// CTA size, 256 or 512 (anything else: 512).  Four 256-thread
 // CTAs fit on an SM against two of 512, which matters when the batch holds
 // between one and two waves of steps.
 void launch_sort(const float *aabbs, const uint64_t *mcodes, uint32_t s_first, uint32_t nb, uint64_t N,
                  uint64_t *keys_a, uint32_t *vals_a, uint32_t *vals_b, uint32_t *srt_idx,
                  uint64_t *srt_mcodes, float *srt_aabbs, int threads, cudaStream_t stream)
 {
-    if (threads == 256)
+    if (N <= 512)
+        k_sort_small<256, 512><<<nb, 256, 0, stream>>>(aabbs, mcodes, s_first, uint32_t(N), srt_idx, srt_mcodes,
+                                                       srt_aabbs);
+    else if (N <= SMALL_MAX)
+        k_sort_small<512, SMALL_MAX><<<nb, 512, 0, stream>>>(aabbs, mcodes, s_first, uint32_t(N), srt_idx, srt_mcodes,
+                                                        srt_aabbs);
+    else if (threads == 256)
         k_sort_step<256><<<nb, 256, 0, stream>>>(aabbs, mcodes, s_first, N, keys_a, vals_a, vals_b, srt_idx,
                                                  srt_mcodes, srt_aabbs);
     else
