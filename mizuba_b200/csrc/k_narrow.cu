@@ -432,11 +432,12 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 // where all but 1 % turn out to have one minimum, above the threshold.  The
 // reference formulation takes 8,921 FP64 operations and 190 divisions for an
 // item, and root finding as much again; which of the two outcomes it will
-// have can be proven from an FMA-native evaluation of 3,000 operations:
+// have can be proven from an FMA-native evaluation of 2,500 operations:
 //
-// * each object's segment polynomial is evaluated by FMA Horner at the nodes
-//   delta + c_m rf_int (mathematically the translated polynomial at
-//   c_m rf_int: the explicit translation is skipped); the squared distances
+// * both objects' segment polynomials are shifted to the sub-interval's
+//   midpoint (synthetic division) and subtracted, and the difference is
+//   scaled to [-1, 1], where the nodes are symmetric: its even and odd parts
+//   give the values at a node and its mirror together.  The squared distances
 //   are interpolated in the normalised time s = t / rf_int on the fixed nodes
 //   c_m by Bjorck-Pereyra with precomputed reciprocals 1 / (c_j - c_{j-k-1}),
 //   and their Bernstein coefficients b_i over [0, 1] come from the difference
@@ -449,15 +450,15 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 //   A_n = C(2n, n) / C(n, n / 2), for a single value.  Over random pairs of
 //   catalogue segments (orders 2 to 32, sub-intervals from 1e-6 of a segment
 //   to a whole one, distances from 1 m to 2,000 km) the largest difference was
-//   1.5 u A_n (P sqrt(max f) + max f) at order 2 and at most 0.5 of that from
+//   1.3 u A_n (P sqrt(max f) + max f) at order 2 and at most 0.33 of that from
 //   order 12 on; the margin M takes 32 (and a P^2 term for vanishing f);
 // * min b >= threshold^2 + M: the reference prunes the item (counter 1);
 // * b_1 - b_0 < -2M, b_n - b_{n-1} > 2M, every second difference > 4M and
 //   min b < threshold^2 - M: the reference keeps the item and finds exactly
 //   one root of the derivative, a minimum.  The polynomial is convex with
 //   p'' / 2 >= kappa = n (n - 1) / 2 min (second difference), so p is at least
-//   p(s) - p'(s)^2 / (4 kappa) for any s; after two Newton steps from the
-//   secant of p' that bound is the minimum itself for all purposes.  If it is
+//   p(s) - p'(s)^2 / (4 kappa) for any s; after a Newton step from the secant
+//   of p' that bound is the minimum itself for all purposes.  If it is
 //   at least threshold^2 + 2M, the minimum is discarded (counters 2, 5 and 6)
 //   and no trajectory boundary in the item can be below the threshold either;
 // * everything else (also values outside the range in which neither
@@ -468,58 +469,86 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 // Bound by the FP64 pipe, if the coefficients arrive: 960 bytes an item, in
 // rows of 160 (order 18).  Loaded by each thread for itself, a 16-byte load of
 // a warp touched 32 lines and the load pipe was the bound (31 % of the FP64
-// rate).  Here a warp copies its items' rows of one coordinate to shared
-// memory together (cp.async, consecutive lanes on consecutive bytes of a row),
-// reads them back at an odd stride of 16-byte units (conflict-free), and has
-// the next coordinate's copies in flight while it computes.  6.38 M items of
-// the 20,000-object day: 2.6 ms, 49 % of the FP64 rate (three warps a
-// scheduler at 168 registers; the rest is latency of the dependent FMAs).
-// Narrow phase with root finding, plain form, 10.4 -> 3.1 ms; mixed form
-// 3.1 -> 1.2 ms; 60,000 objects x 48 steps at 20 km, mixed, 11.9 -> 4.7 ms.
-//
-// tab layout (doubles): [0, OP1) nodes c_m; [OP1, OP1 + OP1^2) inverse node
-// differences, row k; then OP1 inverse binomials 1 / C(n, i); then the
-// binomials of k_narrow's warp path, row k: C(i + k, k).
-//
-// One warp a CTA: the work is per warp, and its shared memory (rows and f)
-// stays below 48 KB up to order 32.
+// rate).  Here a warp copies its items' rows of one coordinate and object to
+// shared memory together (cp.async, consecutive lanes on consecutive bytes of
+// a row), reads them back at an odd stride of 16-byte units (conflict-free),
+// and has the next rows in flight while it computes.  One object's rows at a
+// time, the sums of squares in shared memory between the coordinates and all
+// constants as kernel parameters (operands of the instructions instead of
+// loads) leave room for 16 warps an SM at order 18 (124 registers; 12 warps
+// are 4 % slower, 18 with spills 14 %).  6.38 M items of the 20,000-object day:
+// 1.7 ms (2.6 with Horner at every node and both objects' rows, 168
+// registers and 12 warps).  With the merge walk and root finding, the plain
+// form's narrow phase took 10.4 ms with the reference formulation for every
+// item and takes 2.2; 60,000 objects x 48 steps at 20 km, mixed, 11.9 and 4.2.
+struct filter_tables {
+    double x[MAX_OP1 / 2], y[MAX_OP1 / 2]; // nodes in (0, 1] of [-1, 1], descending, and their squares
+    double node[MAX_OP1];                  // nodes of [0, 1], ascending
+    double inv_binom[MAX_OP1];
+};
+// Reciprocal node differences, row k: 1 / (c_j - c_{j-k-1}), j = k + 1 .. n.
+template <int OP1>
+struct filter_consts {
+    filter_tables t;
+    double inv_dd[OP1 * (OP1 - 1) / 2];
+};
+template <int OP1>
+static filter_consts<OP1> make_filter_consts()
+{
+    filter_consts<OP1> f{};
+    const int n = OP1 - 1;
+    const cheb_nodes c = make_cheb_nodes(OP1);
+    int at = 0;
+    for (int k = 0; k < n; ++k)
+        for (int j = k + 1; j <= n; ++j) f.inv_dd[at++] = 1.0 / (c.v[j] - c.v[j - k - 1]);
+    double b = 1.0;
+    for (int i = 0; i <= n; ++i) {
+        f.t.node[i] = c.v[i];
+        f.t.inv_binom[i] = 1.0 / b;
+        b = b * (n - i) / (i + 1);
+    }
+    for (int m = 0; m < OP1 / 2; ++m) {
+        f.t.x[m] = 2.0 * c.v[n - m] - 1.0;
+        f.t.y[m] = f.t.x[m] * f.t.x[m];
+    }
+    return f;
+}
+__host__ __device__ constexpr int filter_row(int op1, int k) { return k * (op1 - 1) - k * (k - 1) / 2; } // start of row k
+
+// One warp a CTA: the work is per warp.
 template <int OP1>
 struct filter_shape {
     static constexpr int UNITS = row_ld(OP1) / 2; // 16-byte units of a row
     static constexpr int STRIDE = UNITS | 1;      // odd: conflict-free 16-byte reads
     static constexpr int GROUPS = 32 / UNITS;     // rows copied per instruction
-    static constexpr int CTAS = OP1 <= 22 ? 12 : 8;
+    static constexpr int CTAS = OP1 <= 20 ? 16 : 8;
 };
 
 template <int OP1>
 __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
-    k_narrow_filter(dev_pj pj, const double *__restrict__ tab, filter_limits lim,
-                    const double2 *__restrict__ cd_bounds, uint32_t s_first, const np_item *__restrict__ items,
-                    const unsigned long long *item_count, uint64_t item_cap, double thresh2,
-                    np_item *__restrict__ surv, uint64_t surv_cap, unsigned long long *surv_count,
-                    unsigned long long *counters)
+    k_narrow_filter(dev_pj pj, const filter_consts<OP1> K, filter_limits lim, const double2 *__restrict__ cd_bounds,
+                    uint32_t s_first, const np_item *__restrict__ items, const unsigned long long *item_count,
+                    uint64_t item_cap, double thresh2, np_item *__restrict__ surv, uint64_t surv_cap,
+                    unsigned long long *surv_count, unsigned long long *counters)
 {
     using F = filter_shape<OP1>;
     constexpr int n = OP1 - 1;
-    __shared__ __align__(16) double2 rows[64 * F::STRIDE];
+    __shared__ __align__(16) double2 rows[32 * F::STRIDE];
     __shared__ double fs[OP1][32];
-    __shared__ const double2 *base[64];
+    __shared__ const double2 *base[2][32];
     const unsigned lane = threadIdx.x;
-    const double *cheb = tab;
-    const double *inv_dd = tab + OP1;
-    const double *inv_binom = tab + OP1 + OP1 * OP1;
     const uint64_t n_items = min(*item_count, (unsigned long long)item_cap);
-    unsigned long long n_pruned = 0, n_single = 0;
-    // The rows of coordinate c of the warp's 32 items (first object: rows
-    // 0..31, second: 32..63), GROUPS rows at a time.
+    unsigned n_pruned = 0, n_single = 0;
+    // The rows of coordinate c and object o of the warp's 32 items, GROUPS
+    // rows at a time.
     const unsigned part = lane % F::UNITS, grp = lane / F::UNITS;
     const unsigned dst0 = unsigned(__cvta_generic_to_shared(rows + grp * F::STRIDE + part));
-    auto fetch = [&](int c) {
+    auto fetch = [&](int o, int c) {
 #pragma unroll
-        for (int k = 0; k < (64 + F::GROUPS - 1) / F::GROUPS; ++k) {
+        for (int k = 0; k < (32 + F::GROUPS - 1) / F::GROUPS; ++k) {
             const unsigned r = grp + unsigned(k * F::GROUPS);
-            if (grp < F::GROUPS && r < 64) {
-                const double2 *src = base[r] + c * F::UNITS + part;
+            if (grp < F::GROUPS && r < 32) {
+                const double2 *src = base[o][r] + c * F::UNITS + part;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                                  dst0 + unsigned(k * F::GROUPS * F::STRIDE * 16)),
                              "l"(src)
@@ -528,7 +557,12 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto row_in = [&](const double2 *r, double(&c)[OP1]) {
+    // The fetched row into registers, when it has arrived; afterwards the next
+    // rows may land.
+    auto row_in = [&](double(&c)[OP1]) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        const double2 *r = rows + lane * F::STRIDE;
 #pragma unroll
         for (int k = 0; k < OP1 / 2; ++k) {
             const double2 v = r[k];
@@ -536,6 +570,18 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             c[2 * k + 1] = v.y;
         }
         if (OP1 & 1) c[OP1 - 1] = r[OP1 / 2].x;
+        __syncwarp();
+    };
+    // Shift to the origin a; returns sum |c_k| e^k first.
+    auto shifted = [](double(&c)[OP1], double a, double e) {
+        double p = fabs(c[n]);
+#pragma unroll
+        for (int k = n - 1; k >= 0; --k) p = fma(p, e, fabs(c[k]));
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+#pragma unroll
+            for (int k = n - 1; k >= i; --k) c[k] = fma(a, c[k + 1], c[k]);
+        return p;
     };
     for (uint64_t b0 = blockIdx.x * uint64_t(32); b0 < n_items; b0 += uint64_t(gridDim.x) * 32) {
         const uint64_t q_idx = b0 + lane;
@@ -563,82 +609,84 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             gsj = pj.seg_off[it.j] + it.it_j - 1;
         }
         // Rows of lanes without an item are segment 0's: copied, not used.
-        base[lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsi, 0));
-        base[32 + lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsj, 0));
+        base[0][lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsi, 0));
+        base[1][lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsj, 0));
         __syncwarp();
-        fetch(0);
+        fetch(0, 0);
         double P = 0;
-        const double ei = di + rf_int, ej = dj + rf_int;
+        const double h = 0.5 * rf_int;
 #pragma unroll 1
         for (int c = 0; c < 3; ++c) {
-            double ci[OP1], cj[OP1];
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncwarp();
-            row_in(rows + lane * F::STRIDE, ci);
-            row_in(rows + (32 + lane) * F::STRIDE, cj);
-            __syncwarp(); // every row is in registers: the next ones may land
-            if (c < 2) fetch(c + 1);
-            double pi = fabs(ci[n]), pj_ = fabs(cj[n]);
+            double g[OP1], t[OP1];
+            row_in(g);
+            fetch(1, c);
+            P += shifted(g, di + h, di + rf_int);
+            row_in(t);
+            if (c < 2) fetch(0, c + 1);
+            P += shifted(t, dj + h, dj + rf_int);
+            double hp = h;
+            g[0] = g[0] - t[0];
 #pragma unroll
-            for (int k = n - 1; k >= 0; --k) {
-                pi = fma(pi, ei, fabs(ci[k]));
-                pj_ = fma(pj_, ej, fabs(cj[k]));
+            for (int k = 1; k < OP1; ++k) {
+                g[k] = (g[k] - t[k]) * hp;
+                hp *= h;
             }
-            P += pi + pj_;
-            // The sums of squares stay in shared memory between coordinates:
-            // in registers they made this loop spill, and unrolled whole it
-            // was 10,000 instructions, whose fetch was most of a small call.
-#pragma unroll 4
-            for (int m = 0; m < OP1; ++m) {
-                const double am = __ldg(cheb + m) * rf_int;
-                const double tii = di + am, tjj = dj + am;
-                double xi = ci[n], xj = cj[n];
+            // Node n - m and its mirror m: even part +- x times odd part.
+            auto add = [&](int m, double d) { fs[m][lane] = (c == 0) ? d * d : fma(d, d, fs[m][lane]); };
+            constexpr int EV = n & ~1, OD = (n - 1) | 1;
 #pragma unroll
-                for (int k = n - 1; k >= 0; --k) {
-                    xi = fma(xi, tii, ci[k]);
-                    xj = fma(xj, tjj, cj[k]);
-                }
-                const double d = xi - xj;
-                fs[m][lane] = (c == 0) ? d * d : fma(d, d, fs[m][lane]);
+            for (int m = 0; m < OP1 / 2; ++m) {
+                double even = g[EV], odd = g[OD];
+#pragma unroll
+                for (int k = EV - 2; k >= 0; k -= 2) even = fma(even, K.t.y[m], g[k]);
+#pragma unroll
+                for (int k = OD - 2; k >= 1; k -= 2) odd = fma(odd, K.t.y[m], g[k]);
+                add(n - m, fma(K.t.x[m], odd, even));
+                add(m, fma(-K.t.x[m], odd, even));
             }
+            if (OP1 & 1) add(n / 2, g[0]);
         }
         double f[OP1];
 #pragma unroll
         for (int m = 0; m < OP1; ++m) f[m] = fs[m][lane];
         double fmax_s = f[0];
 #pragma unroll
-        for (int m = 1; m < OP1; ++m) fmax_s = fmax(fmax_s, f[m]);
+        for (int m = 1; m < OP1; ++m) fmax_s = f[m] > fmax_s ? f[m] : fmax_s;
         // Bjorck-Pereyra on the normalised nodes.
 #pragma unroll
         for (int k = 0; k < n; ++k)
 #pragma unroll
-            for (int jj = n; jj > k; --jj) f[jj] = (f[jj] - f[jj - 1]) * __ldg(inv_dd + k * OP1 + jj);
+            for (int jj = n; jj > k; --jj) f[jj] = (f[jj] - f[jj - 1]) * K.inv_dd[filter_row(OP1, k) + jj - k - 1];
 #pragma unroll
-        for (int k = n - 1; k >= 0; --k) {
-            const double ck = __ldg(cheb + k);
+        for (int k = n - 1; k >= 0; --k)
 #pragma unroll
-            for (int jj = k; jj < n; ++jj) f[jj] = fma(-ck, f[jj + 1], f[jj]);
-        }
+            for (int jj = k; jj < n; ++jj) f[jj] = fma(-K.t.node[k], f[jj + 1], f[jj]);
         // Bernstein coefficients over s in [0, 1], each one's first and
         // second differences as it appears.
         double e[OP1];
 #pragma unroll
-        for (int k = 0; k < OP1; ++k) e[k] = f[k] * __ldg(inv_binom + k);
+        for (int k = 0; k < OP1; ++k) e[k] = f[k] * K.t.inv_binom[k];
         double emin = e[0], b1 = e[0], d_first = 0, d_prev = 0, dd_min = INFINITY;
 #pragma unroll
         for (int k = 1; k < OP1; ++k) {
 #pragma unroll
             for (int jj = 0; jj + k < OP1; ++jj) e[jj] = e[jj] + e[jj + 1];
-            emin = fmin(emin, e[0]);
+            emin = e[0] < emin ? e[0] : emin;
             const double d = e[0] - b1;
-            if (k == 1) d_first = d;
-            else dd_min = fmin(dd_min, d - d_prev);
+            if (k == 1) {
+                d_first = d;
+            } else {
+                const double dd = d - d_prev;
+                dd_min = dd < dd_min ? dd : dd_min;
+            }
             d_prev = d;
             b1 = e[0];
         }
         const double root_f = double(__fsqrt_ru(__double2float_ru(fmax_s)));
         const double M = lim.margin * (root_f * P + fmax_s + 1e-14 * P * P);
-        usable = usable && fmax_s <= 1e30 && P <= 1e15; // false for non-finite values
+        // P is NaN or too large for non-finite values (the comparisons above
+        // would drop a NaN).
+        usable = usable && fmax_s <= 1e30 && P <= 1e15;
         const bool pruned = usable && emin >= thresh2 + M;
         bool single = false;
         if (usable && !pruned && emin < thresh2 - M && d_first < -2 * M && d_prev > 2 * M && dd_min > 4 * M) {
@@ -646,7 +694,7 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             double s = d_first / (d_first - d_prev);
             double p = 0, p1 = 0;
 #pragma unroll 1
-            for (int r = 0; r < 3; ++r) {
+            for (int r = 0; r < 2; ++r) {
                 double p2 = 0;
                 p = f[n], p1 = 0;
 #pragma unroll
@@ -655,7 +703,7 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
                     p1 = fma(p1, s, p);
                     p = fma(p, s, f[k]);
                 }
-                if (r < 2) s = fmin(fmax(s - p1 / (2 * p2), 0.0), 1.0);
+                if (r == 0) s = fmin(fmax(s - p1 / (2 * p2), 0.0), 1.0);
             }
             single = p - p1 * p1 / (4 * kappa) >= thresh2 + 2 * M;
         }
@@ -665,11 +713,13 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
         const unsigned long long slot = warp_append(surv_count, push);
         if (push && slot < surv_cap) surv[slot] = it;
     }
-    warp_add(counters + 1, n_pruned);
-    warp_add(counters + 2, n_single);
-    warp_add(counters + 5, n_single);
-    warp_add(counters + 6, n_single);
-    warp_add(counters + 7, n_single);
+    n_pruned = __reduce_add_sync(0xffffffffu, n_pruned);
+    n_single = __reduce_add_sync(0xffffffffu, n_single);
+    if (lane == 0) {
+        if (n_pruned) atomicAdd(counters + 1, (unsigned long long)n_pruned);
+        if (n_single)
+            for (int k : {2, 5, 6, 7}) atomicAdd(counters + k, (unsigned long long)n_single);
+    }
 }
 
 // Screen ahead of the filter (mixed form): a rigorous lower bound on the
@@ -1912,17 +1962,17 @@ void launch_items(const dev_pj &pj, const double2 *cdb, uint32_t s_first, uint32
 }
 
 template <int OP1>
-static void narrow_t(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first, const np_item *items,
+static void narrow_t(const dev_pj &pj, const double *shift, const double2 *cdb, uint32_t s_first, const np_item *items,
                      const unsigned long long *item_count, uint64_t item_cap, double thresh2, root_item *rq,
                      uint64_t rq_cap, unsigned long long *rq_count, unsigned long long *counters, dev_status *st,
                      unsigned grid, cudaStream_t stream)
 {
-    k_narrow<OP1><<<grid, NARROW_T, 0, stream>>>(pj, make_cheb_nodes(OP1), tab + OP1 * (OP1 + 2), cdb, s_first, items,
+    k_narrow<OP1><<<grid, NARROW_T, 0, stream>>>(pj, make_cheb_nodes(OP1), shift, cdb, s_first, items,
                                                   item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st);
 }
 
-// tab: the tables of launch_narrow_filter.
-void launch_narrow(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first, const np_item *items,
+// shift[k * op1 + i] = C(i + k, k), device memory.
+void launch_narrow(const dev_pj &pj, const double *shift, const double2 *cdb, uint32_t s_first, const np_item *items,
                    const unsigned long long *item_count, uint64_t item_cap, double thresh2, root_item *rq,
                    uint64_t rq_cap, unsigned long long *rq_count, unsigned long long *counters, dev_status *st,
                    unsigned grid, cudaStream_t stream)
@@ -1930,7 +1980,7 @@ void launch_narrow(const dev_pj &pj, const double *tab, const double2 *cdb, uint
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        narrow_t<K>(pj, tab, cdb, s_first, items, item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st, grid, \
+        narrow_t<K>(pj, shift, cdb, s_first, items, item_count, item_cap, thresh2, rq, rq_cap, rq_count, counters, st, grid, \
                     stream);                                                                                           \
         break;
         MZB_FOR_EACH_OP1(X)
@@ -1941,17 +1991,18 @@ void launch_narrow(const dev_pj &pj, const double *tab, const double2 *cdb, uint
 }
 
 template <int OP1>
-static void filter_t(const dev_pj &pj, const double *tab, const filter_limits &lim, const double2 *cdb,
+static void filter_t(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
                      uint32_t s_first, const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
                      double thresh2, np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
                      unsigned long long *counters, cudaStream_t stream)
 {
     using F = filter_shape<OP1>;
-    k_narrow_filter<OP1><<<148 * F::CTAS, 32, 0, stream>>>(pj, tab, lim, cdb, s_first, items, item_count, item_cap,
+    static const filter_consts<OP1> consts = make_filter_consts<OP1>();
+    k_narrow_filter<OP1><<<148 * F::CTAS, 32, 0, stream>>>(pj, consts, lim, cdb, s_first, items, item_count, item_cap,
                                                              thresh2, surv, surv_cap, surv_count, counters);
 }
 
-void launch_narrow_filter(const dev_pj &pj, const double *tab, const filter_limits &lim, const double2 *cdb,
+void launch_narrow_filter(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
                           uint32_t s_first, const np_item *items, const unsigned long long *item_count,
                           uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
                           unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream)
@@ -1959,7 +2010,7 @@ void launch_narrow_filter(const dev_pj &pj, const double *tab, const filter_limi
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        filter_t<K>(pj, tab, lim, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,     \
+        filter_t<K>(pj, lim, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,     \
                     counters, stream);                                                                                 \
         break;
         MZB_FOR_EACH_OP1(X)
@@ -1997,18 +2048,18 @@ filter_limits make_filter_limits(int op1)
 }
 
 template <int OP1>
-static void roots_t(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+static void roots_t(const dev_pj &pj, const double *shift, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                     const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                     double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                     conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,
                     dev_status *st, cudaStream_t stream)
 {
-    k_roots<OP1><<<grid, ROOTS_T, 0, stream>>>(pj, tab + OP1 * (OP1 + 2), rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch,
+    k_roots<OP1><<<grid, ROOTS_T, 0, stream>>>(pj, shift, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch,
                                             wl_cap, retry, retry_count, cq, cq_cap, cq_count, counters, st);
 }
 
-// tab: the tables of launch_narrow_filter.
-void launch_roots(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+// shift as for launch_narrow.
+void launch_roots(const dev_pj &pj, const double *shift, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                   const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                   double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                   conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,
@@ -2017,7 +2068,7 @@ void launch_roots(const dev_pj &pj, const double *tab, const root_item *rq, cons
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        roots_t<K>(pj, tab, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch, wl_cap, grid, retry,    \
+        roots_t<K>(pj, shift, rq, rq_count, rq_cap, item_list, item_list_count, thresh2, wl_scratch, wl_cap, grid, retry,    \
                    retry_count, cq, cq_cap, cq_count, counters, st, stream);                                          \
         break;
         MZB_FOR_EACH_OP1(X)

@@ -89,7 +89,7 @@ void launch_broad_lists(uint32_t nb, uint64_t N, const uint32_t *counts, const u
 void launch_items(const dev_pj &pj, const double2 *cdb, uint32_t s_first, uint32_t nb, const uint2 *pairs,
                   const uint64_t *step_off, const uint2 *srange, uint64_t n_pairs, np_item *items, uint64_t cap,
                   unsigned long long *item_count, unsigned long long *counters, dev_status *st, cudaStream_t stream);
-void launch_narrow(const dev_pj &pj, const double *tab, const double2 *cdb, uint32_t s_first, const np_item *items,
+void launch_narrow(const dev_pj &pj, const double *shift, const double2 *cdb, uint32_t s_first, const np_item *items,
                    const unsigned long long *item_count, uint64_t item_cap, double thresh2, root_item *rq,
                    uint64_t rq_cap, unsigned long long *rq_count, unsigned long long *counters, dev_status *st,
                    unsigned grid, cudaStream_t stream);
@@ -103,13 +103,13 @@ struct filter_limits {
     double rf_lo, rf_hi, margin;
 };
 filter_limits make_filter_limits(int op1);
-void launch_narrow_filter(const dev_pj &pj, const double *tab, const filter_limits &lim, const double2 *cdb,
+void launch_narrow_filter(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
                           uint32_t s_first, const np_item *items, const unsigned long long *item_count,
                           uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
                           unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream);
 constexpr int ROOTS_WL_SMALL = 24;  // working-list entries per thread, first pass
 constexpr int ROOTS_WL_FULL = 251;  // the reference's bound (list size > 250 fails)
-void launch_roots(const dev_pj &pj, const double *tab, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
+void launch_roots(const dev_pj &pj, const double *shift, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
                   const uint32_t *item_list, const unsigned long long *item_list_count, double thresh2,
                   double *wl_scratch, int wl_cap, unsigned grid, uint32_t *retry, unsigned long long *retry_count,
                   conj_out *cq, uint64_t cq_cap, unsigned long long *cq_count, unsigned long long *counters,

@@ -1031,41 +1031,27 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         cdb[kk] = make_double2(b, e);
         R.cd_end[kk] = e;
     }
-    // Tables of the narrow phase: nodes, inverse node differences, inverse
-    // binomials, binomials of the translation.
-    std::vector<double> h_tab;
-    {
-        const int op1 = pj.order + 1, n = pj.order;
-        const cheb_nodes cn = make_cheb_nodes(op1);
-        h_tab.assign(size_t(op1) * (2 * op1 + 2), 0.0);
-        for (int m = 0; m < op1; ++m) h_tab[m] = cn.v[m];
-        for (int k = 0; k < n; ++k)
-            for (int j = k + 1; j < op1; ++j) h_tab[op1 + size_t(k) * op1 + j] = 1.0 / (cn.v[j] - cn.v[j - k - 1]);
-        double c = 1.0;
-        for (int i = 0; i <= n; ++i) {
-            h_tab[op1 + size_t(op1) * op1 + i] = 1.0 / c;
-            c = c * (n - i) / (i + 1);
-        }
-        // C(i + k, k), exact: Pascal's rule along row k.
-        double *sh = h_tab.data() + size_t(op1) * (op1 + 2);
-        for (int k = 0; k < op1; ++k)
-            for (int i = 0; i + k < op1; ++i)
-                sh[size_t(k) * op1 + i] = (k == 0 || i == 0) ? 1.0 : sh[size_t(k) * op1 + i - 1] + sh[size_t(k - 1) * op1 + i];
-    }
-    // One block and one copy for the step bounds, the tables and the object
+    // Binomials C(i + k, k) of the narrow phase's warp paths, row k (Pascal's
+    // rule, exact).
+    const size_t op1 = size_t(pj.order) + 1;
+    std::vector<double> h_shift(op1 * op1, 0.0);
+    for (size_t k = 0; k < op1; ++k)
+        for (size_t i = 0; i + k < op1; ++i)
+            h_shift[k * op1 + i] = (k == 0 || i == 0) ? 1.0 : h_shift[k * op1 + i - 1] + h_shift[(k - 1) * op1 + i];
+    // One block and one copy for the step bounds, the binomials and the object
     // types (pageable memory: the copy has read it, or waits until it has,
     // before the call returns).
-    const size_t at_tab = S * sizeof(double2), at_ot = at_tab + h_tab.size() * sizeof(double);
+    const size_t at_shift = S * sizeof(double2), at_ot = at_shift + h_shift.size() * sizeof(double);
     std::vector<char> h_in(at_ot + N * sizeof(int32_t));
-    std::memcpy(h_in.data(), cdb.data(), at_tab);
-    std::memcpy(h_in.data() + at_tab, h_tab.data(), at_ot - at_tab);
+    std::memcpy(h_in.data(), cdb.data(), at_shift);
+    std::memcpy(h_in.data() + at_shift, h_shift.data(), at_ot - at_shift);
     if (otypes_host) std::memcpy(h_in.data() + at_ot, otypes_host, N * sizeof(int32_t));
     else std::fill_n(reinterpret_cast<int32_t *>(h_in.data() + at_ot), N, 1);
     dbuf<char> d_in(SL());
     d_in.alloc(h_in.size(), st);
     CK(cudaMemcpyAsync(d_in.p, h_in.data(), h_in.size(), cudaMemcpyHostToDevice, st));
     const double2 *d_cdb = reinterpret_cast<const double2 *>(d_in.p);
-    const double *filter_tab = reinterpret_cast<const double *>(d_in.p + at_tab);
+    const double *shift = reinterpret_cast<const double *>(d_in.p + at_shift);
     const int32_t *d_ot = reinterpret_cast<const int32_t *>(d_in.p + at_ot);
     const filter_limits filter_lim = make_filter_limits(pj.order + 1);
 
@@ -1347,16 +1333,16 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 // The FMA filter, then the reference formulation on the items
                 // it leaves.
                 const dbuf<np_item> &src = mixed ? cand : items;
-                launch_narrow_filter(P, filter_tab, filter_lim, d_cdb, sf, src.p,
+                launch_narrow_filter(P, filter_lim, d_cdb, sf, src.p,
                                      mixed ? &C->narrow.cand.v : &C->narrow.items.v, src.n, thresh2, surv.p, surv.n,
                                      &C->narrow.surv.v, C->narrow.np, st);
-                launch_narrow(P, filter_tab, d_cdb, sf, surv.p, &C->narrow.surv.v, surv.n, thresh2, rq.p, rq.n,
+                launch_narrow(P, shift, d_cdb, sf, surv.p, &C->narrow.surv.v, surv.n, thresh2, rq.p, rq.n,
                               &C->narrow.roots.v, C->narrow.np,
                               d_st.p, narrow_grid, st);
                 CK(cudaEventRecord(ev[4].b, st));
-                launch_roots(P, filter_tab, rq.p, &C->narrow.roots.v, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL,
+                launch_roots(P, shift, rq.p, &C->narrow.roots.v, rq.n, nullptr, nullptr, thresh2, wl.p, ROOTS_WL_SMALL,
                              roots_grid, retry.p, &C->narrow.retry.v, cq.p, cq.n, &C->narrow.conj.v, C->narrow.np, d_st.p, st);
-                launch_roots(P, filter_tab, rq.p, &C->narrow.roots.v, rq.n, retry.p, &C->narrow.retry.v, thresh2, wl_full.p,
+                launch_roots(P, shift, rq.p, &C->narrow.roots.v, rq.n, retry.p, &C->narrow.retry.v, thresh2, wl_full.p,
                              ROOTS_WL_FULL, roots_grid_full, nullptr, nullptr, cq.p, cq.n, &C->narrow.conj.v,
                              C->narrow.np, d_st.p, st);
                 CK(cudaEventRecord(ev[5].b, st));
