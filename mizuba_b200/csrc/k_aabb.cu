@@ -721,7 +721,7 @@ void launch_aabb(const dev_pj &pj, const double2 *cdb, bool mixed, uint32_t s_fi
     default:
         break;
     }
-    k_gbox<<<nb, 512, 0, stream>>>(s_first, pj.n_objs, aabbs, st);
+    k_gbox<<<nb, nb <= 148 ? 1024 : 512, 0, stream>>>(s_first, pj.n_objs, aabbs, st);
 }
 
 void launch_morton(const float *aabbs, uint32_t s_first, uint32_t nb, uint64_t N, uint64_t *mcodes, cudaStream_t stream)

@@ -96,15 +96,16 @@ __device__ __forceinline__ void queue_pair(const pair_queue &Q, uint32_t slot0, 
 // of one another.  Appended one by one from inside the divergent walk, every
 // partner cost its warp two dependent L2 round trips, and dense catalogues
 // serialised on the counter.  Broad phase of 48 steps of a 60,000-object
-// catalogue at 20 km (24 M pairs) 16.9 -> 4.6 ms, 192 steps of 20,000 objects
-// with shells at 10 km (9.8 M) 5.4 -> 2.3 ms, of which the second, full walk
+// catalogue at 20 km (24 M pairs) 16.9 -> 4.3 ms, 192 steps of 20,000 objects
+// with shells at 10 km (9.8 M) 5.4 -> 2.2 ms, of which the second, full walk
 // that the older spill list took on overflow was 11.7 and 2.9 ms; the
-// 20,000-object day (4.5 M) is unchanged (2.55 / 2.60 ms): bound by the latency
-// of its dependent node loads.  HITS 8 keeps the buffer at 4 KB per CTA, so
-// that the walk nodes keep the L1.  Ten CTAs an SM (48 registers): at 72
+// 20,000-object day (4.5 M) is unchanged (2.55 ms): bound by the latency of its
+// dependent node loads.  HITS 16 keeps the buffer at 8 KB per CTA, so that the
+// walk nodes keep the L1 (the same broad phases with 8, 16 and 24: 4.67, 4.34,
+// 4.46; 2.30, 2.19, 2.32; day 2.54, 2.55, 2.70 ms).  Ten CTAs an SM (48 registers): at 72
 // registers the day took 3.2 ms, at 40 with spills 3.3 ms.
 constexpr int WALK_T = 128;
-constexpr int HITS = 8;
+constexpr int HITS = 16;
 
 __global__ void __launch_bounds__(WALK_T, 10) k_broad_half(const float *__restrict__ srt_aabbs,
                                                        const bvh_node *__restrict__ trees, uint64_t cap,

@@ -2141,7 +2141,7 @@ static int conjunctions_call(const mzb_pj *pj, double conj_thresh, double conj_d
                                   + ": expected 0 (automatic), 256 or 512");
             run_detection(*pj, conj_thresh, conj_det_interval, otypes, skip_cd, spb, mixed,
                           int(bvh_threads), int(broad_walk),
-                          sort_threads ? int(sort_threads) : 512, dst, *R);
+                          int(sort_threads), dst, *R);
         } catch (...) {
             delete R;
             throw;
