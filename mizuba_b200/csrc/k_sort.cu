@@ -8,18 +8,26 @@
 // stable LSD radix sort on the code; boxes without data carry the code
 // 2^64 - 1, so they stay behind every finite box.  Bits that are equal in
 // every code of the step do not affect the order, so the codes are first
-// compacted to their varying bits (passes whose digit is constant over the
-// step are skipped; the 20,000-object catalogue varies in all 64 bits).  The
-// prologue counts the finite boxes, finds the varying bits, stores every
-// compacted key by original index and builds the histograms of every pass;
-// each pass then moves original indices only, reading each one's digit from
-// the stored keys, and ranks tiles of 4,096 (8 per thread, warp-striped so a
-// warp's are consecutive) with bit ballots and per-warp digit counters in
-// shared memory.  Scratch: the compacted keys (8 bytes per object and step)
-// and the index ping-pong (2 x 4 bytes).  Moving indices alone keeps a step's
-// working set at 320 KB, so under a full grid the resident steps' buffers fit
-// the L2 (the key + index ping-pong took 480 KB and 1.62 against 1.34 ms for
-// the day's sorts).
+// compacted to their varying bits, V of them (the 20,000-object catalogue
+// varies in all 64).  Of those the passes sort by the top SORT_BITS only: that
+// is fine enough that few objects share them, and a last pass over the
+// positions orders every run of equal top bits by the whole code, in place
+// and stably (one thread per run; runs are two or three long in a catalogue).
+// A step with a run above RUN_MAX (dense clusters) takes the passes over all
+// bits instead, from the order it has.  The prologue counts the finite boxes,
+// finds the varying bits, stores every compacted key by original index and
+// builds the histograms of the passes (a pass whose digit is constant over the
+// step is skipped); each pass then moves original indices only, reading each
+// one's digit from the stored keys, and ranks tiles of 4,096 (8 per thread,
+// warp-striped so a warp's are consecutive) with bit ballots and per-warp digit
+// counters in shared memory.  Scratch: the compacted keys (8 bytes per object
+// and step) and the index ping-pong (2 x 4 bytes).  Moving indices alone keeps
+// a step's working set at 320 KB, so under a full grid the resident steps'
+// buffers fit the L2 (the key + index ping-pong took 480 KB and 1.62 against
+// 1.34 ms for the day's sorts, all bits).
+// Morton and sort with all 64 bits, the top 48, 40 and 32 (ms): 480 steps of
+// 20,000 objects 1.35, 1.15, 1.05, 0.99; 48 of 60,000 with dense shells 0.96,
+// 0.79, 0.72, 0.73; 40 leaves the longer runs of larger catalogues room.
 #include <mutex>
 
 #include "block.cuh"
@@ -30,6 +38,8 @@ namespace mzb
 {
 
 constexpr int SORT_KPT = 8;
+constexpr int SORT_BITS = 40;
+constexpr uint32_t RUN_MAX = 64;
 
 // SORT_T: 256, 512 or 1,024 threads (the per-digit sections need at least 256).
 template <int SORT_T>
@@ -94,7 +104,9 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
     __syncthreads();
     const uint64_t mask = vmask;
     const uint32_t n_fin = nfin_s;
-    const int npass = (__popcll(mask) + 7) / 8;
+    const int vbits = __popcll(mask);
+    const int low = vbits > SORT_BITS ? vbits - SORT_BITS : 0; // bits left to the runs
+    const int npass = (vbits - low + 7) / 8;
     for (unsigned z = tid; z < 8u * 256u; z += SORT_T) {
         const unsigned j = z >> 8, v = z & 255u;
         const unsigned mb = unsigned(mask >> (8 * j)) & 255u;
@@ -130,7 +142,7 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         c |= uint64_t(ctab[j][unsigned(code >> (8 * j)) & 255u]) << cshift[j];
-                    for (int ps = 0; ps < npass; ++ps) atomicAdd(&hist[ps][unsigned(c >> (8 * ps)) & 255u], 1u);
+                    for (int ps = 0; ps < npass; ++ps) atomicAdd(&hist[ps][unsigned(c >> (low + 8 * ps)) & 255u], 1u);
                 }
                 ck[k] = c;
             }
@@ -161,10 +173,9 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
         if ((&hist[0][0])[z] == N) atomicOr(&skipmask, 1u << (z >> 8));
     __syncthreads();
 
-    // ---- LSD radix passes over the compacted keys.
-    for (int ps = 0; ps < npass; ++ps) {
-        if ((skipmask >> ps) & 1u) continue; // digit constant: the pass is the identity
-        const int shift = 8 * ps;
+    // ---- One LSD radix pass over the compacted keys' digit at `shift`, whose
+    // histogram is hist[ps].
+    auto radix_pass = [&](int ps, int shift) {
         if (tid < 256) {
             const uint32_t v = hist[ps][tid];
             uint32_t x = v;
@@ -255,13 +266,61 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
         uint32_t *vt = vin;
         vin = vout;
         vout = vt;
+    };
+    for (int ps = 0; ps < npass; ++ps)
+        if (!((skipmask >> ps) & 1u)) radix_pass(ps, low + 8 * ps); // else the digit is constant
+
+    uint64_t *sc = srt_mcodes + s * N;
+    for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
+    if (low > 0) {
+        // Runs of equal top bits.  Only the thread at a run's start writes in
+        // it, and what the others read there to find out that they are not at
+        // a start differs from its neighbours in the low bits only, whatever
+        // has been moved.
+        uint64_t top = mask;
+        for (int k = 0; k < low; ++k) top &= top - 1;
+        if (tid == 0) nfin_s = 0; // from here on: a run is too long
+        __syncthreads();
+        for (uint64_t p = tid; p + 1 < N; p += SORT_T) {
+            const uint64_t c = sc[p];
+            if (((c ^ sc[p + 1]) & top) != 0 || (p > 0 && ((c ^ sc[p - 1]) & top) == 0)) continue;
+            uint64_t e = p + 2;
+            while (e < N && e - p <= RUN_MAX && ((c ^ sc[e]) & top) == 0) ++e;
+            if (e - p > RUN_MAX) {
+                nfin_s = 1;
+                continue;
+            }
+            for (uint64_t x = p + 1; x < e; ++x) {
+                const uint64_t cx = sc[x];
+                const uint32_t vx = vin[x];
+                uint64_t y = x;
+                for (; y > p && sc[y - 1] > cx; --y) {
+                    sc[y] = sc[y - 1];
+                    vin[y] = vin[y - 1];
+                }
+                sc[y] = cx;
+                vin[y] = vx;
+            }
+        }
+        __syncthreads();
+        if (nfin_s) {
+            // All bits, from the order so far: equal codes are in theirs.
+            for (unsigned z = tid; z < 8u * 256u; z += SORT_T) (&hist[0][0])[z] = 0;
+            __syncthreads();
+            for (uint64_t i = tid; i < N; i += SORT_T) {
+                const uint64_t c = ckey[i];
+                for (int ps = 0; ps < (vbits + 7) / 8; ++ps) atomicAdd(&hist[ps][unsigned(c >> (8 * ps)) & 255u], 1u);
+            }
+            __syncthreads();
+            for (int ps = 0; ps < (vbits + 7) / 8; ++ps) radix_pass(ps, 8 * ps);
+            for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
+        }
     }
 
-    // Outputs: sorted indices and codes, gathered boxes, global box row.
+    // Outputs: sorted indices, gathered boxes, global box row.
     for (uint64_t p = tid; p < N; p += SORT_T) {
         const uint32_t o = vin[p];
         srt_idx[s * N + p] = o;
-        srt_mcodes[s * N + p] = mc[o];
         const float4 *src = reinterpret_cast<const float4 *>(ab + uint64_t(o) * 8);
         float4 *dst = reinterpret_cast<float4 *>(srt_aabbs + (s * (N + 1) + p) * 8);
         dst[0] = src[0];
