@@ -698,18 +698,22 @@ def main():
         # Narrow phase, per item (one pair of overlapping segments).  Plain
         # form: the reference's formulation (translation of 3 + 3
         # coordinates, Horner at m nodes for 6 polynomials, dist^2,
-        # Bjorck-Pereyra, Cargo-Shisha).  Mixed form: FMA Horner of 6
-        # polynomials at m shifted nodes, dist^2, Bjorck-Pereyra with
-        # reciprocals, Cargo-Shisha on [0, 1].
+        # Bjorck-Pereyra, Cargo-Shisha).  Filter (both forms): per coordinate
+        # both polynomials' magnitude bounds and shifts, their scaled
+        # difference and its even and odd parts at the nodes' mirror pairs;
+        # then Bjorck-Pereyra with reciprocals and Cargo-Shisha with the
+        # differences of its coefficients.
         ops_plain = (2 * 3 * (3 * m * (m + 1) // 2 + n) + 2 * 6 * m * n + 8 * m
                      + (3 * n * (n + 1) // 2 + n * (n + 1)) + (3 * n + m + n * (n + 1) // 2 + 2 * m))
-        ops_mixed = 6 * m * n + 3 * m + 3 * m + 3 * n * (n + 1) // 2 + m + n * (n + 1) // 2 + 2 * n
-        # Mixed narrow stage: the distance screen on every item (about 65
-        # FP64 operations from the two stored linear models), the FMA
-        # prefilter on the items that pass it, the reference formulation on
-        # the prefilter's survivors.
+        ops_filter = (3 * (n * (n + 1) + 2 * n + 3 * m - 1 + (m // 2) * (n + 1) + m)
+                      + 3 * n * (n + 1) // 2 + m + n * (n + 1) // 2 + 4 * n)
+        # Narrow stage: in the mixed form the distance screen on every item
+        # (about 65 FP64 operations from the two stored linear models), then
+        # the filter on the items that pass it (in the plain form: on all).
+        # The reference formulation runs on the few items the filter leaves
+        # (about 1 in 100) and is not counted.
         ops_screen = 65
-        mixed_narrow_ops = np_rep[0] * ops_screen + np_split[0] * ops_mixed + np_split[1] * ops_plain
+        mixed_narrow_ops = np_rep[0] * ops_screen + np_split[0] * ops_filter
 
         def fp64_roof(stage, kernel, units, ops, t_ms, extra=None, kernels=None):
             ach = units * ops / (t_ms / 1e3) / 1e12
@@ -721,24 +725,31 @@ def main():
             return r
 
         n_seg_items = step_items(pj, srange[0], srange[1])
-        ops_seg_plain = 4 * (m * (m + 1) + (m * (m + 1) // 2 - m) + 2 * (n - 1) + 2 * m + n * (n + 1) // 2 + 2)
-        # Mixed enclosure per variable, plus the screen model of x, y, z
-        # (value and derivative by Horner, the curvature bound: 3 n each).
-        ops_seg_mixed = 4 * (n + n * (n + 1) // 2 + 3 * m + n * (n + 1) // 2 + 2 * n + 4) + 3 * 3 * n
+        # Enclosure per variable (magnitude bound, shift, scaling, difference
+        # table with its minimum and maximum, error bound); segments that
+        # start inside a step are not shifted.  Mixed form: plus the screen
+        # model of x, y, z (value and derivative by Horner, the curvature
+        # bound: 3 n each).
+        unshifted = max(n_seg_items - pj.n_objs * S_day, 0) / max(n_seg_items, 1)
+        ops_seg_plain = 4 * (n + (1 - unshifted) * n * (n + 1) // 2 + 3 * m + n * (n + 1) // 2 + 2 * n + 8)
+        ops_seg_mixed = ops_seg_plain - 16 + 3 * 3 * n
         seg_bytes = {"algorithmic_bytes_per_unit": 4 * m * 8 + 16}
         stages = {
-            "narrow": fp64_roof("narrow", "k_items_screen + k_narrow_mixed + k_narrow", np_rep[0],
+            "narrow": fp64_roof("narrow", "k_items_screen + k_narrow_filter + k_narrow", np_rep[0],
                                 mixed_narrow_ops / max(np_rep[0], 1), stage_avg["narrow"],
-                                {"items_screened": np_rep[0], "items_prefiltered": np_split[0],
-                                 "items_exact": np_split[1],
-                                 "ops_per_item": {"screen": ops_screen, "prefilter": ops_mixed,
-                                                  "exact": ops_plain}},
-                                kernels=["k_items_screen", "k_narrow_mixed", "k_narrow_survivors"]),
-            "aabb": fp64_roof("aabb", "k_aabb_mixed", n_seg_items, ops_seg_mixed, stage_avg["aabb"], seg_bytes,
-                              kernels=["k_aabb_mixed", "k_aabb_mixed_more"]),
-            "narrow_plain_form": fp64_roof("narrow", "k_narrow", np_rep_plain[0], ops_plain, stage_plain["narrow"]),
-            "aabb_plain_form": fp64_roof("aabb", "k_aabb", n_seg_items, ops_seg_plain, stage_plain["aabb"],
-                                         seg_bytes),
+                                {"items_screened": np_rep[0], "items_filtered": np_split[0],
+                                 "items_reaching_threshold": np_split[1],
+                                 "ops_per_item": {"screen": ops_screen, "filter": ops_filter,
+                                                  "reference": ops_plain}},
+                                kernels=["k_items_screen", "k_narrow_filter", "k_narrow"]),
+            "aabb": fp64_roof("aabb", "k_aabb + k_aabb_more", n_seg_items, ops_seg_mixed, stage_avg["aabb"], seg_bytes,
+                              kernels=["k_aabb", "k_aabb_more"]),
+            "narrow_plain_form": fp64_roof("narrow", "k_items + k_narrow_filter + k_narrow", np_rep_plain[0],
+                                           ops_filter, stage_plain["narrow"],
+                                           kernels=["k_items", "k_narrow_filter_plain", "k_narrow_plain"]),
+            "aabb_plain_form": fp64_roof("aabb", "k_aabb + k_aabb_more", n_seg_items, ops_seg_plain,
+                                         stage_plain["aabb"], seg_bytes,
+                                         kernels=["k_aabb_plain", "k_aabb_more_plain"]),
         }
         # BVH: the trees written (48 B per node) and the sorted codes and
         # boxes read (40 B per object and step).  Broad phase: one 32-byte
@@ -752,7 +763,7 @@ def main():
                          "algorithmic_bytes": bvh_bytes, "peak_source": "MEASURED_PEAKS.json hbm_gbs"}
         broad_bytes = broad_visits * 32 + ident["pairs_mixed"] * 8
         broad_ach = broad_bytes / (stage_avg["broad"] / 1e3) / 1e9
-        stages["broad"] = {"stage": "broad", "kernel": "k_broad_half + scan + copy", "bound": "hbm",
+        stages["broad"] = {"stage": "broad", "kernel": "k_broad_half + offsets + lists", "bound": "hbm",
                            "achieved": broad_ach, "peak": hbm_peak, "unit": "GB/s", "frac": broad_ach / hbm_peak,
                            "traffic": traffic_of("k_broad_half"), "node_visits": broad_visits,
                            "node_visits_per_s": broad_visits / (stage_avg["broad"] / 1e3),

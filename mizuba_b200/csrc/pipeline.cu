@@ -4,10 +4,10 @@
 // stages per conjunction step on CPU threads, chunked by 128 steps, and
 // streams variable-size outputs to files through a writer thread.  Here the
 // steps are processed in batches (all of a batch's steps in every launch):
-//   aabb -> global box -> morton -> sort/gather -> bvh -> broad count ->
-//   scan -> broad write -> narrow -> roots -> per-step conj order
-// on one CUDA stream, with three host synchronisations per batch (to size the
-// pair list, the root queue and the conjunction list).  All outputs stay in
+//   aabb -> global box -> morton -> sort/gather -> bvh -> broad walk ->
+//   offsets -> pair lists -> items -> filter -> narrow -> roots -> conj order
+// on one CUDA stream, with two host synchronisations inside a batch (to size
+// the pair list, and to check the queues and the status).  All outputs stay in
 // HBM until the caller copies them out.
 #include <fcntl.h>
 #include <sys/stat.h>
@@ -2117,7 +2117,7 @@ static int conjunctions_call(const mzb_pj *pj, double conj_thresh, double conj_d
             R->n_objs = pj->n_objs;
             uint32_t spb = (opts && opts->steps_per_batch) ? opts->steps_per_batch : 0;
             if (spb == 0) {
-                // Batch scratch is ~184 bytes per object and step (248 in the
+                // Batch scratch is ~190 bytes per object and step (254 in the
                 // mixed form); stay near 3 GB.
                 const uint64_t per_step = 248ull * pj->n_objs + 4096;
                 spb = uint32_t(std::clamp<uint64_t>((3ull << 30) / per_step, 16, 1024));
