@@ -442,27 +442,47 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 //   c_m by Bjorck-Pereyra with precomputed reciprocals 1 / (c_j - c_{j-k-1}),
 //   and their Bernstein coefficients b_i over [0, 1] come from the difference
 //   table of Cargo-Shisha;
-// * both formulations interpolate the same values on the same nodes.  Their
-//   Bernstein coefficients differ by the rounding of the values (of order
-//   u P sqrt(max f) + u max f, with P = sum |c_k| (delta + rf_int)^k over both
-//   objects and the three coordinates), which interpolation amplifies by at
-//   most the largest Bernstein coefficient of the Chebyshev polynomial,
-//   A_n = C(2n, n) / C(n, n / 2), for a single value.  Over random pairs of
-//   catalogue segments (orders 2 to 32, sub-intervals from 1e-6 of a segment
-//   to a whole one, distances from 1 m to 2,000 km) the largest difference was
-//   1.3 u A_n (P sqrt(max f) + max f) at order 2 and at most 0.33 of that from
-//   order 12 on; the margin M takes 32 (and a P^2 term for vanishing f);
+// * both formulations interpolate the same polynomial's values on the same
+//   nodes, and M bounds how far their Bernstein coefficients can differ by
+//   rounding, u = 2^-53 (filter_margins):
+//   - an object's coordinate at a node: the reference formulation (powers,
+//     binomial sums, Horner) is within sum (3k + 8) u |c_k| e^k of its exact
+//     value, this one (shift, scaling, even and odd Horner) within sum (4k + 5)
+//     u |c_k| e^k, e = delta + rf_int, and 7k + 14 <= 18 (5/4)^k.  With P_c the
+//     sum of |c_k| (5e/4)^k over both objects' coordinate c and P^2 = sum P_c^2,
+//     the squared distance at node m differs by at most 36 u P sqrt(f_m) +
+//     324 u^2 P^2 + 10 u f_m, and a Bernstein coefficient by node_w[m] times
+//     that.  Their sum over the nodes is bounded with F = sum node_w[m] f_m
+//     (Cauchy-Schwarz); the weights, 1.3 times the largest Bernstein coefficient
+//     of the Chebyshev polynomial together, are largest in the middle, where an
+//     encounter is close;
+//   - each divided difference has a relative rounding of 4 u here, 3 u there and
+//     u (c_j + c_i) / (c_j - c_i) for the nodes c rf_int there; each step from
+//     Newton form to monomials four roundings of what it adds up.  All of them
+//     are at most linear in the magnitudes of the Newton coefficients; newton[l]
+//     is what the l-th one's can do to a Bernstein coefficient;
+//   - scaling by 1 / C(n, i) and the difference table: (3n + 5) u sum |f_k|, f_k
+//     the monomials' coefficients on [0, 1]; Ms = (6n + 24) u sum |f_k|, part of
+//     M, also covers the derivative in root finding: its coefficients (n (n + 12)
+//     u sum |f_k|), values (n (3n + 2)) and slope (3 n^3).
+//   On segments of a catalogue the first term is nearly all of M, where the
+//   coefficients do not fall off the other two are.  A margin measured on the
+//   former, 32 u A_n (P sqrt(max f) + max f), lost conjunctions of the latter at
+//   orders from 20 on;
 // * min b >= threshold^2 + M: the reference prunes the item (counter 1);
-// * b_1 - b_0 < -2M, b_n - b_{n-1} > 2M, every second difference > 4M and
-//   min b < threshold^2 - M: the reference keeps the item and finds exactly
-//   one root of the derivative, a minimum.  The polynomial is convex with
-//   p'' / 2 >= kappa = n (n - 1) / 2 min (second difference), so p is at least
-//   p(s) - p'(s)^2 / (4 kappa) for any s; after a Newton step from the secant
-//   of p' that bound is the minimum itself for all purposes.  If it is
-//   at least threshold^2 + 2M, the minimum is discarded (counters 2, 5 and 6)
-//   and no trajectory boundary in the item can be below the threshold either;
+// * b_1 - b_0 < -2M - Ms, b_n - b_{n-1} > 2M + Ms, every second difference >
+//   4M + 2Ms and min b < threshold^2 - M: the reference keeps the item.  The
+//   Bernstein coefficients of its derivative ascend from negative to positive,
+//   by steps and with ends that exceed their roundings, so it finds exactly one
+//   root, a minimum.  The polynomial is convex with p'' / 2 >= kappa =
+//   n (n - 1) / 2 (min second difference - 4M), so p is at least
+//   p(s) - p'(s)^2 / (4 kappa) for any s; after a Newton step from the secant of
+//   p' that bound is the minimum itself for all purposes.  If it is at least
+//   threshold^2 + 2M (with n Ms more for p'), the minimum is discarded
+//   (counters 2, 5 and 6) and no trajectory boundary in the item can be below
+//   the threshold either;
 // * everything else (also values outside the range in which neither
-//   formulation can overflow: see filter_limits) goes to k_narrow.
+//   formulation can overflow: see filter_range) goes to k_narrow.
 //
 // So the records and all counters are those of the reference formulation.
 //
@@ -485,7 +505,136 @@ struct filter_tables {
     double x[MAX_OP1 / 2], y[MAX_OP1 / 2]; // nodes in (0, 1] of [-1, 1], descending, and their squares
     double node[MAX_OP1];                  // nodes of [0, 1], ascending
     double inv_binom[MAX_OP1];
+    double node_w[MAX_OP1];                // F = sum node_w[m] f_m
+    double newton[MAX_OP1];                // margin per Newton coefficient
+    double value, square, norm, mono;      // and per sqrt(F) P, F, P^2 and sum |f_k|
+    double rf_lo, rf_hi;                   // range of sub-interval lengths
 };
+// Where the filter's argument holds for order n: the reference formulation
+// divides differences of f by node distances c rf_int, so its k-th divided
+// differences are at most 2^k max f / (G_k rf_int^k), G_k the product of the
+// smallest node distances at lags 1 to k; with max f <= 1e30 they stay below
+// 1e280 for rf_int >= rf_lo, and neither rf_int^n nor its inverse leaves the
+// exponent range for rf_int in [rf_lo, rf_hi].
+static void filter_range(filter_tables &t, int n)
+{
+    t.rf_lo = std::pow(10.0, -250.0 / n);
+    t.rf_hi = std::pow(10.0, 200.0 / n);
+    double log_g = 0;
+    for (int k = 1; k <= n; ++k) {
+        double gap = 1.0;
+        for (int j = k; j <= n; ++j) gap = std::min(gap, t.node[j] - t.node[j - k]);
+        log_g += std::log10(gap);
+        t.rf_lo = std::max(t.rf_lo, std::pow(10.0, (k * std::log10(2.0) + 30.0 - log_g - 280.0) / k));
+    }
+}
+
+// The weights of the margin M (above) for order n.  Everything here is a
+// linear map of the few dozen numbers of an item; the maps are applied to unit
+// vectors in long double and the results' largest Bernstein coefficients taken.
+static void filter_margins(filter_tables &t, int n)
+{
+    using real = long double;
+    using vec = std::vector<real>;
+    const double *c = t.node;
+    const size_t m = size_t(n) + 1;
+    // p (s - r) and the degree elevation of p, in Bernstein form over [0, 1].
+    auto times_root = [](const vec &p, real r) {
+        const int d = int(p.size()) - 1;
+        vec q(size_t(d) + 2, 0);
+        for (int i = 0; i <= d + 1; ++i) {
+            if (i <= d) q[i] -= r * (d + 1 - i) * p[i] / (d + 1);
+            if (i > 0) q[i] += (1 - r) * i * p[i - 1] / (d + 1);
+        }
+        return q;
+    };
+    auto elevated = [n](vec p) {
+        while (int(p.size()) <= n) {
+            const int d = int(p.size()) - 1;
+            vec q(size_t(d) + 2, 0);
+            for (int i = 0; i <= d + 1; ++i)
+                q[i] = ((i ? i * p[i - 1] : 0) + (i <= d ? (d + 1 - i) * p[i] : 0)) / (d + 1);
+            p = std::move(q);
+        }
+        return p;
+    };
+    auto largest = [](const vec &p) {
+        real a = 0;
+        for (const real v : p) a = std::max(a, std::fabs(v));
+        return a;
+    };
+    // Newton basis w_l = prod_{i < l} (s - c_i), also at degree n.
+    std::vector<vec> w(m), wn(m);
+    for (int l = 0; l <= n; ++l) {
+        w[l] = l ? times_root(w[l - 1], c[l - 1]) : vec{1};
+        wn[l] = elevated(w[l]);
+    }
+    // Bernstein coefficients from the divided differences of level k (entries
+    // from k on; the ones before are zero).
+    auto bernstein = [&](vec f, int k) {
+        for (int q = k; q < n; ++q)
+            for (int j = n; j > q; --j) f[j] = (f[j] - f[j - 1]) / (real(c[j]) - c[j - q - 1]);
+        vec b(m, 0);
+        for (int l = k; l <= n; ++l)
+            for (int i = 0; i <= n; ++i) b[i] += f[l] * wn[l][i];
+        return b;
+    };
+    // What a node's value can do to a Bernstein coefficient.
+    real L = 0;
+    for (int j = 0; j <= n; ++j) {
+        vec e(m, 0);
+        e[j] = 1;
+        const real a = largest(bernstein(std::move(e), 0));
+        t.node_w[j] = double(a);
+        L += a;
+    }
+    // Divided difference j of level k: its relative rounding in both
+    // formulations, and what an error of it does to the coefficients.
+    std::vector<vec> dd(m, vec(m, 0));
+    for (int k = 1; k <= n; ++k)
+        for (int j = k; j <= n; ++j) {
+            vec e(m, 0);
+            e[j] = 1;
+            dd[k][j] = (7 + (real(c[j]) + c[j - k]) / (real(c[j]) - c[j - k])) * largest(bernstein(std::move(e), k));
+        }
+    // Step k of Newton form -> monomials writes the coefficients of
+    // s^(j - k) w_k: four roundings of at most the sum of magnitudes there.
+    std::vector<vec> nm(m, vec(m, 0));
+    for (int k = 0; k < n; ++k) {
+        vec p = w[k];
+        for (int j = k; j < n; ++j) {
+            nm[k][j] = 4 * largest(elevated(p));
+            p = times_root(p, 0);
+        }
+    }
+    const real u = 1.1102230246251565e-16L, slack = 1.05L; // slack: second order and this function's own rounding
+    for (int l = 0; l <= n; ++l) {
+        real g = 0;
+        vec f(m); // w_l at the nodes, then its divided differences level by level (none beyond l)
+        for (int j = 0; j <= n; ++j) {
+            f[j] = 1;
+            for (int i = 0; i < l; ++i) f[j] *= real(c[j]) - c[i];
+        }
+        for (int k = 1; k <= l; ++k)
+            for (int j = n; j >= k; --j) {
+                f[j] = (f[j] - f[j - 1]) / (real(c[j]) - c[j - k]);
+                g += dd[k][j] * std::fabs(f[j]);
+            }
+        vec a(m, 0); // magnitudes of the coefficients that w_l contributes to
+        a[l] = 1;
+        for (int k = n - 1; k >= 0; --k)
+            for (int j = k; j < n; ++j) {
+                a[j] += c[k] * a[j + 1];
+                g += nm[k][j] * a[j];
+            }
+        t.newton[l] = double(slack * u * g);
+    }
+    t.value = double(slack * u * std::sqrt(L) * 36);
+    t.square = double(slack * u * 10);
+    t.norm = double(slack * u * u * L * 324);
+    t.mono = double(slack * u * (6 * n + 24));
+}
+
 // Reciprocal node differences, row k: 1 / (c_j - c_{j-k-1}), j = k + 1 .. n.
 template <int OP1>
 struct filter_consts {
@@ -511,6 +660,8 @@ static filter_consts<OP1> make_filter_consts()
         f.t.x[m] = 2.0 * c.v[n - m] - 1.0;
         f.t.y[m] = f.t.x[m] * f.t.x[m];
     }
+    filter_range(f.t, n);
+    filter_margins(f.t, n);
     return f;
 }
 __host__ __device__ constexpr int filter_row(int op1, int k) { return k * (op1 - 1) - k * (k - 1) / 2; } // start of row k
@@ -526,7 +677,7 @@ struct filter_shape {
 
 template <int OP1>
 __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
-    k_narrow_filter(dev_pj pj, const filter_consts<OP1> K, filter_limits lim, const double2 *__restrict__ cd_bounds,
+    k_narrow_filter(dev_pj pj, const filter_consts<OP1> K, const double2 *__restrict__ cd_bounds,
                     uint32_t s_first, const np_item *__restrict__ items, const unsigned long long *item_count,
                     uint64_t item_cap, double thresh2, np_item *__restrict__ surv, uint64_t surv_cap,
                     unsigned long long *surv_count, unsigned long long *counters)
@@ -572,8 +723,9 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
         if (OP1 & 1) c[OP1 - 1] = r[OP1 / 2].x;
         __syncwarp();
     };
-    // Shift to the origin a; returns sum |c_k| e^k first.
+    // Shift to the origin a; returns sum |c_k| (5/4 e)^k first.
     auto shifted = [](double(&c)[OP1], double a, double e) {
+        e *= 1.25;
         double p = fabs(c[n]);
 #pragma unroll
         for (int k = n - 1; k >= 0; --k) p = fma(p, e, fabs(c[k]));
@@ -604,7 +756,7 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             di = lb_rf - si;
             dj = lb_rf - sj;
             rf_int = ub_rf - lb_rf;
-            usable = di >= 0 && dj >= 0 && rf_int >= lim.rf_lo && rf_int <= lim.rf_hi;
+            usable = di >= 0 && dj >= 0 && rf_int >= K.t.rf_lo && rf_int <= K.t.rf_hi;
             gsi = pj.seg_off[it.i] + it.it_i - 1;
             gsj = pj.seg_off[it.j] + it.it_j - 1;
         }
@@ -613,17 +765,18 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
         base[1][lane] = reinterpret_cast<const double2 *>(coef_row<OP1>(pj, gsj, 0));
         __syncwarp();
         fetch(0, 0);
-        double P = 0;
+        double P2 = 0;
         const double h = 0.5 * rf_int;
 #pragma unroll 1
         for (int c = 0; c < 3; ++c) {
             double g[OP1], t[OP1];
             row_in(g);
             fetch(1, c);
-            P += shifted(g, di + h, di + rf_int);
+            double pc = shifted(g, di + h, di + rf_int);
             row_in(t);
             if (c < 2) fetch(0, c + 1);
-            P += shifted(t, dj + h, dj + rf_int);
+            pc += shifted(t, dj + h, dj + rf_int);
+            P2 = fma(pc, pc, P2);
             double hp = h;
             g[0] = g[0] - t[0];
 #pragma unroll
@@ -646,21 +799,28 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             }
             if (OP1 & 1) add(n / 2, g[0]);
         }
-        double f[OP1];
+        double f[OP1], F_s = 0;
 #pragma unroll
-        for (int m = 0; m < OP1; ++m) f[m] = fs[m][lane];
-        double fmax_s = f[0];
-#pragma unroll
-        for (int m = 1; m < OP1; ++m) fmax_s = f[m] > fmax_s ? f[m] : fmax_s;
+        for (int m = 0; m < OP1; ++m) {
+            f[m] = fs[m][lane];
+            F_s = fma(K.t.node_w[m], f[m], F_s);
+        }
         // Bjorck-Pereyra on the normalised nodes.
 #pragma unroll
         for (int k = 0; k < n; ++k)
 #pragma unroll
             for (int jj = n; jj > k; --jj) f[jj] = (f[jj] - f[jj - 1]) * K.inv_dd[filter_row(OP1, k) + jj - k - 1];
+        double M = 1e-250;
+#pragma unroll
+        for (int k = 0; k < OP1; ++k) M = fma(K.t.newton[k], fabs(f[k]), M);
 #pragma unroll
         for (int k = n - 1; k >= 0; --k)
 #pragma unroll
             for (int jj = k; jj < n; ++jj) f[jj] = fma(-K.t.node[k], f[jj + 1], f[jj]);
+        double Ms = 0;
+#pragma unroll
+        for (int k = 0; k < OP1; ++k) Ms += fabs(f[k]);
+        Ms *= K.t.mono;
         // Bernstein coefficients over s in [0, 1], each one's first and
         // second differences as it appears.
         double e[OP1];
@@ -682,15 +842,16 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
             d_prev = d;
             b1 = e[0];
         }
-        const double root_f = double(__fsqrt_ru(__double2float_ru(fmax_s)));
-        const double M = lim.margin * (root_f * P + fmax_s + 1e-14 * P * P);
-        // P is NaN or too large for non-finite values (the comparisons above
-        // would drop a NaN).
-        usable = usable && fmax_s <= 1e30 && P <= 1e15;
+        auto root_up = [](double x) { return double(__fsqrt_ru(__double2float_ru(x))); };
+        M += Ms + fma(K.t.value * root_up(F_s), root_up(P2), fma(K.t.square, F_s, K.t.norm * P2));
+        // F is NaN or too large for non-finite values (the comparisons above
+        // would drop a NaN); every node_w is above 1.
+        usable = usable && F_s <= 1e30 && P2 <= 1e30;
         const bool pruned = usable && emin >= thresh2 + M;
         bool single = false;
-        if (usable && !pruned && emin < thresh2 - M && d_first < -2 * M && d_prev > 2 * M && dd_min > 4 * M) {
-            const double kappa = 0.5 * (double(n) * (n - 1)) * dd_min;
+        if (usable && !pruned && emin < thresh2 - M && d_first < -2 * M - Ms && d_prev > 2 * M + Ms
+            && dd_min > 4 * M + 2 * Ms) {
+            const double kappa = 0.5 * (double(n) * (n - 1)) * (dd_min - 4 * M);
             double s = d_first / (d_first - d_prev);
             double p = 0, p1 = 0;
 #pragma unroll 1
@@ -705,6 +866,7 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
                 }
                 if (r == 0) s = fmin(fmax(s - p1 / (2 * p2), 0.0), 1.0);
             }
+            p1 = fabs(p1) + n * Ms;
             single = p - p1 * p1 / (4 * kappa) >= thresh2 + 2 * M;
         }
         n_pruned += pruned;
@@ -1991,26 +2153,24 @@ void launch_narrow(const dev_pj &pj, const double *shift, const double2 *cdb, ui
 }
 
 template <int OP1>
-static void filter_t(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
-                     uint32_t s_first, const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
+static void filter_t(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
                      double thresh2, np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
                      unsigned long long *counters, cudaStream_t stream)
 {
     using F = filter_shape<OP1>;
     static const filter_consts<OP1> consts = make_filter_consts<OP1>();
-    k_narrow_filter<OP1><<<148 * F::CTAS, 32, 0, stream>>>(pj, consts, lim, cdb, s_first, items, item_count, item_cap,
+    k_narrow_filter<OP1><<<148 * F::CTAS, 32, 0, stream>>>(pj, consts, cdb, s_first, items, item_count, item_cap,
                                                              thresh2, surv, surv_cap, surv_count, counters);
 }
 
-void launch_narrow_filter(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
-                          uint32_t s_first, const np_item *items, const unsigned long long *item_count,
+void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count,
                           uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
                           unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream)
 {
     switch (pj.op1) {
 #define X(K)                                                                                                         \
     case K:                                                                                                            \
-        filter_t<K>(pj, lim, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,     \
+        filter_t<K>(pj, cdb, s_first, items, item_count, item_cap, thresh2, surv, surv_cap, surv_count,     \
                     counters, stream);                                                                                 \
         break;
         MZB_FOR_EACH_OP1(X)
@@ -2018,33 +2178,6 @@ void launch_narrow_filter(const dev_pj &pj, const filter_limits &lim, const doub
     default:
         break;
     }
-}
-
-// Where the filter's argument holds for order op1 - 1: the reference
-// formulation divides differences of f by node distances c rf_int, so its
-// k-th divided differences are at most 2^k max f / (G_k rf_int^k), G_k the
-// product of the smallest node distances at lags 1 to k; with max f <= 1e30
-// they stay below 1e280 for rf_int >= rf_lo, and neither rf_int^n nor its
-// inverse leaves the exponent range for rf_int in [rf_lo, rf_hi].
-filter_limits make_filter_limits(int op1)
-{
-    const int n = op1 - 1;
-    const cheb_nodes c = make_cheb_nodes(op1);
-    filter_limits lim{};
-    lim.rf_lo = std::pow(10.0, -250.0 / n);
-    lim.rf_hi = std::pow(10.0, 200.0 / n);
-    double log_g = 0;
-    for (int k = 1; k <= n; ++k) {
-        double gap = 1.0;
-        for (int j = k; j <= n; ++j) gap = std::min(gap, c.v[j] - c.v[j - k]);
-        log_g += std::log10(gap);
-        lim.rf_lo = std::max(lim.rf_lo, std::pow(10.0, (k * std::log10(2.0) + 30.0 - log_g - 280.0) / k));
-    }
-    double a = 1.0; // C(2n, n) / C(n, n / 2)
-    for (int k = 1; k <= n; ++k) a = a * (n + k) / k;
-    for (int k = 1; k <= n / 2; ++k) a = a * k / (n - n / 2 + k);
-    lim.margin = 32.0 * 1.1102230246251565e-16 * a;
-    return lim;
 }
 
 template <int OP1>

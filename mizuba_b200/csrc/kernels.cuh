@@ -98,13 +98,7 @@ void launch_items_screen(const dev_pj &pj, const double2 *cdb, uint32_t s_first,
                          const float4 *scr, np_item *cand, uint64_t cand_cap, unsigned long long *cand_count,
                          unsigned long long *item_count, unsigned long long *counters, dev_status *st,
                          cudaStream_t stream);
-// Range of sub-interval lengths and the error margin of k_narrow_filter.
-struct filter_limits {
-    double rf_lo, rf_hi, margin;
-};
-filter_limits make_filter_limits(int op1);
-void launch_narrow_filter(const dev_pj &pj, const filter_limits &lim, const double2 *cdb,
-                          uint32_t s_first, const np_item *items, const unsigned long long *item_count,
+void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count,
                           uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
                           unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream);
 constexpr int ROOTS_WL_SMALL = 24;  // working-list entries per thread, first pass

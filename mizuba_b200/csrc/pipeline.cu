@@ -1053,7 +1053,6 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     const double2 *d_cdb = reinterpret_cast<const double2 *>(d_in.p);
     const double *shift = reinterpret_cast<const double *>(d_in.p + at_shift);
     const int32_t *d_ot = reinterpret_cast<const int32_t *>(d_in.p + at_ot);
-    const filter_limits filter_lim = make_filter_limits(pj.order + 1);
 
     tr.mark("inputs on the device", std::to_string(N) + " objects, " + std::to_string(S) + " steps, "
                                         + std::to_string(spb) + " per batch");
@@ -1333,7 +1332,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 // The FMA filter, then the reference formulation on the items
                 // it leaves.
                 const dbuf<np_item> &src = mixed ? cand : items;
-                launch_narrow_filter(P, filter_lim, d_cdb, sf, src.p,
+                launch_narrow_filter(P, d_cdb, sf, src.p,
                                      mixed ? &C->narrow.cand.v : &C->narrow.items.v, src.n, thresh2, surv.p, surv.n,
                                      &C->narrow.surv.v, C->narrow.np, st);
                 launch_narrow(P, shift, d_cdb, sf, surv.p, &C->narrow.surv.v, surv.n, thresh2, rq.p, rq.n,
