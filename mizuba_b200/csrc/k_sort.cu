@@ -11,10 +11,11 @@
 // compacted to their varying bits, V of them (the 20,000-object catalogue
 // varies in all 64).  Of those the passes sort by the top SORT_BITS only: that
 // is fine enough that few objects share them, and a last pass over the
-// positions orders every run of equal top bits by the whole code, in place
-// and stably (one thread per run; runs are two or three long in a catalogue).
-// A step with a run above RUN_MAX (dense clusters) takes the passes over all
-// bits instead, from the order it has.  The prologue counts the finite boxes,
+// positions orders every run of equal top bits by the whole code, stably (runs
+// are two or three long in a catalogue).
+// A step with a run above RUN_MAX (dense clusters; far outliers, which leave
+// few of the top bits to the others) takes the passes over all bits instead;
+// the prologue sees most of these coming.  The prologue counts the finite boxes,
 // finds the varying bits, stores every compacted key by original index and
 // builds the histograms of the passes (a pass whose digit is constant over the
 // step is skipped); each pass then moves original indices only, reading each
@@ -39,7 +40,7 @@ namespace mzb
 
 constexpr int SORT_KPT = 8;
 constexpr int SORT_BITS = 40;
-constexpr uint32_t RUN_MAX = 64;
+constexpr uint32_t RUN_MAX = 64, RUN_SHORT = 8;
 
 // SORT_T: 256, 512 or 1,024 threads (the per-digit sections need at least 256).
 template <int SORT_T>
@@ -62,7 +63,7 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
     __shared__ uint32_t cshift[8];   // where each byte's packed bits go
     __shared__ uint32_t base[256], tilecnt[256], bscan[8], wtot[SORT_W];
     __shared__ unsigned long long vmask;
-    __shared__ uint32_t nfin_s, skipmask;
+    __shared__ uint32_t nfin_s, skipmask, n_list;
 
     const uint32_t b = blockIdx.x;
     const uint64_t s = uint64_t(s_first) + b;
@@ -116,7 +117,14 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
         ctab[j][v] = uint8_t(out);
     }
     if (tid < 8) cshift[tid] = __popcll(mask & ((1ull << (8 * tid)) - 1ull));
+    // Whether the top bits will do: the objects per hash of their top bits, in
+    // the counters that the passes use later.  A run of more than RUN_MAX shows
+    // as a bin that far above the mean.
+    constexpr uint32_t BINS = 256 * (SORT_W + 1);
+    uint32_t *bins = &wcnt[0][0];
+    for (unsigned z = tid; z < BINS; z += SORT_T) bins[z] = 0;
     __syncthreads();
+    if (tid == 0) nfin_s = 0; // from here on: a run is too long
 
     // ---- Prologue 2: stable partition (finite first), compacted keys, and
     // the digit histograms of every pass.
@@ -143,6 +151,8 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
                     for (int j = 0; j < 8; ++j)
                         c |= uint64_t(ctab[j][unsigned(code >> (8 * j)) & 255u]) << cshift[j];
                     for (int ps = 0; ps < npass; ++ps) atomicAdd(&hist[ps][unsigned(c >> (low + 8 * ps)) & 255u], 1u);
+                    if (low > 0 && f)
+                        atomicAdd(bins + __umulhi(uint32_t((c >> low) * 0x9E3779B97F4A7C15ull >> 32), BINS), 1u);
                 }
                 ck[k] = c;
             }
@@ -171,7 +181,11 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
     }
     for (unsigned z = tid; z < 8u * 256u; z += SORT_T)
         if ((&hist[0][0])[z] == N) atomicOr(&skipmask, 1u << (z >> 8));
+    if (low > 0)
+        for (unsigned z = tid; z < BINS; z += SORT_T)
+            if (bins[z] > RUN_MAX + n_fin / BINS) nfin_s = 1;
     __syncthreads();
+    bool long_runs = nfin_s != 0;
 
     // ---- One LSD radix pass over the compacted keys' digit at `shift`, whose
     // histogram is hist[ps].
@@ -267,30 +281,43 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
         vin = vout;
         vout = vt;
     };
-    for (int ps = 0; ps < npass; ++ps)
-        if (!((skipmask >> ps) & 1u)) radix_pass(ps, low + 8 * ps); // else the digit is constant
+    if (!long_runs)
+        for (int ps = 0; ps < npass; ++ps)
+            if (!((skipmask >> ps) & 1u)) radix_pass(ps, low + 8 * ps); // else the digit is constant
 
     uint64_t *sc = srt_mcodes + s * N;
-    for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
-    if (low > 0) {
+    if (!long_runs)
+        for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
+    if (low > 0 && !long_runs) {
         // Runs of equal top bits among the objects with data (the others stand
         // behind them in index order since the partition, and are one run of
         // any length: 192 steps of 20,000 objects, 100 of them without data,
-        // 0.93 ms with a pass over that run, 0.50 without).  Only the thread at a run's start writes in
-        // it, and what the others read there to find out that they are not at
-        // a start differs from its neighbours in the low bits only, whatever
-        // has been moved.
+        // 0.93 ms with a pass over that run, 0.50 without).  The thread at a
+        // short run's start orders it; only it writes there, and what the
+        // others read there to find out that they are not at a start differs
+        // from its neighbours in the low bits only, whatever has been moved.
+        // Longer runs are listed and ordered by a warp each, by counting: one
+        // thread was a chain of up to RUN_MAX^2 / 4 dependent moves (192 steps
+        // of 20,000 objects of which 20 are 800,000 km away, runs of up to 64:
+        // 2.21 ms, the same steps' passes over all bits 0.61).
         uint64_t top = mask;
         for (int k = 0; k < low; ++k) top &= top - 1;
-        if (tid == 0) nfin_s = 0; // from here on: a run is too long
+        uint32_t *list = bins; // (start, length) pairs
+        if (tid == 0) n_list = 0;
         __syncthreads();
         for (uint64_t p = tid; p + 1 < n_fin; p += SORT_T) {
             const uint64_t c = sc[p];
             if (((c ^ sc[p + 1]) & top) != 0 || (p > 0 && ((c ^ sc[p - 1]) & top) == 0)) continue;
             uint64_t e = p + 2;
             while (e < n_fin && e - p <= RUN_MAX && ((c ^ sc[e]) & top) == 0) ++e;
-            if (e - p > RUN_MAX) {
-                nfin_s = 1;
+            if (e - p > RUN_SHORT) {
+                const uint32_t at = e - p > RUN_MAX ? BINS : atomicAdd(&n_list, 1u);
+                if (at < BINS / 2) {
+                    list[2 * at] = uint32_t(p);
+                    list[2 * at + 1] = uint32_t(e - p);
+                } else {
+                    nfin_s = 1;
+                }
                 continue;
             }
             for (uint64_t x = p + 1; x < e; ++x) {
@@ -306,18 +333,39 @@ __global__ void __launch_bounds__(SORT_T, 1024 / SORT_T) k_sort_step(const float
             }
         }
         __syncthreads();
-        if (nfin_s) {
-            // All bits, from the order so far: equal codes are in theirs.
-            for (unsigned z = tid; z < 8u * 256u; z += SORT_T) (&hist[0][0])[z] = 0;
-            __syncthreads();
-            for (uint64_t i = tid; i < N; i += SORT_T) {
-                const uint64_t c = ckey[i];
-                for (int ps = 0; ps < (vbits + 7) / 8; ++ps) atomicAdd(&hist[ps][unsigned(c >> (8 * ps)) & 255u], 1u);
+        if (!nfin_s)
+            for (uint32_t r = warp; r < n_list; r += SORT_W) {
+                static_assert(RUN_MAX <= 64, "two entries a lane");
+                uint64_t *rc = sc + list[2 * r];
+                uint32_t *rv = vin + list[2 * r];
+                const uint32_t len = list[2 * r + 1];
+                const bool one = lane < len, two = lane + 32 < len;
+                const uint64_t c0 = one ? rc[lane] : 0, c1 = two ? rc[lane + 32] : 0;
+                const uint32_t v0 = one ? rv[lane] : 0, v1 = two ? rv[lane + 32] : 0;
+                uint32_t p0 = 0, p1 = 0;
+                for (uint32_t k = 0; k < len; ++k) {
+                    const uint64_t x = rc[k];
+                    p0 += x < c0 || (x == c0 && k < lane);
+                    p1 += x < c1 || (x == c1 && k < lane + 32);
+                }
+                __syncwarp();
+                if (one) rc[p0] = c0, rv[p0] = v0;
+                if (two) rc[p1] = c1, rv[p1] = v1;
             }
-            __syncthreads();
-            for (int ps = 0; ps < (vbits + 7) / 8; ++ps) radix_pass(ps, 8 * ps);
-            for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
+        __syncthreads();
+        long_runs = nfin_s != 0; // shorter than they look in the bins
+    }
+    if (long_runs) {
+        // All bits, from the order so far: equal codes are in theirs.
+        for (unsigned z = tid; z < 8u * 256u; z += SORT_T) (&hist[0][0])[z] = 0;
+        __syncthreads();
+        for (uint64_t i = tid; i < N; i += SORT_T) {
+            const uint64_t c = ckey[i];
+            for (int ps = 0; ps < (vbits + 7) / 8; ++ps) atomicAdd(&hist[ps][unsigned(c >> (8 * ps)) & 255u], 1u);
         }
+        __syncthreads();
+        for (int ps = 0; ps < (vbits + 7) / 8; ++ps) radix_pass(ps, 8 * ps);
+        for (uint64_t p = tid; p < N; p += SORT_T) sc[p] = mc[vin[p]];
     }
 
     // Outputs: sorted indices, gathered boxes, global box row.
