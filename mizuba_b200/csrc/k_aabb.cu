@@ -287,7 +287,9 @@ struct aabb_smem {
 
 // The boxes of one segment per lane, folded into (lb, ub), by the whole warp:
 // `first` is lane's segment (its first coefficient row), lanes with !act do no
-// folding.  SHIFT false: every h_lb is zero, the shift is the identity.
+// folding and have none: nothing is copied for them (copying one row in place
+// of all of theirs, 192 steps of 5,000 objects of which 1,000 had no data took
+// 0.49 ms instead of 0.24, every warp reading the same lines of the L2).  SHIFT false: every h_lb is zero, the shift is the identity.
 // `unsure` (plain form) is set where the float bounds are not proven.
 //
 // With scr != nullptr (mixed form) the pass also writes the distance screen's
@@ -310,7 +312,7 @@ __device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_bi
 #pragma unroll
         for (int k = 0; k < (32 + F::GROUPS - 1) / F::GROUPS; ++k) {
             const unsigned r = grp + unsigned(k * F::GROUPS);
-            if (grp < F::GROUPS && r < 32) {
+            if (grp < F::GROUPS && r < 32 && S.base[r]) {
                 const double2 *src = S.base[r] + v * F::UNITS + part;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                                  dst0 + unsigned(k * F::GROUPS * F::STRIDE * 16)),
@@ -467,7 +469,7 @@ __global__ void __launch_bounds__(AABB_T, aabb_shape<OP1>::CTAS)
     const uint32_t i = active ? uint32_t(gid % N) : 0;
     bool seg = false, queue = false;
     double h_lb = 0, h_ub = 0;
-    const double *first = pj.coef; // lanes without a segment copy the first one's rows
+    const double *first = nullptr;
     uint2 rng = make_uint2(0, 0);  // empty: no segment overlaps the step
     const uint32_t ns = active ? pj.nseg[i] : 0;
     if (ns > 0) {
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(AABB_T, OP1 <= 20 ? 4 : 3)
             const bool act = active && it < rng.y && !unsure;
             if (!__any_sync(0xffffffffu, act)) break;
             double h_ub = 0;
-            const double *first = pj.coef;
+            const double *first = nullptr;
             if (act) {
                 const double s0 = t[it - 1], s1 = t[it];
                 const double ev_ub = (s1 < ce) ? s1 : ce;
