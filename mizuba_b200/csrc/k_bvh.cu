@@ -695,8 +695,11 @@ void launch_bvh(const float *srt_aabbs, const uint64_t *srt_mcodes, uint32_t s_f
                                          st, csm, dsm);
     };
     // Small steps leave most of a 1,024-thread CTA idle between its barriers:
-    // smaller CTAs, several an SM, where there are steps enough for that.
-    if (N <= 1024) launch(k_bvh_flat<256>, 256);
+    // smaller CTAs, several an SM, where there are steps enough for that.  With
+    // one step an SM or fewer the larger CTA is ahead above 256 objects (BVH
+    // stage of 60 steps of 500 and 1,000 objects: 256 threads 34 and 44 us,
+    // 1,024 threads 32 and 38; of 150 objects 26 and 27).
+    if (N <= 256 || (N <= 1024 && nb > 148)) launch(k_bvh_flat<256>, 256);
     else if (N <= 4096 && nb > 148) launch(k_bvh_flat<512>, 512);
     else launch(k_bvh_flat<1024>, 1024);
     k_walk_nodes<<<dim3(unsigned((cap + 255) / 256), nb), 256, 0, stream>>>(srt_aabbs, trees, cap, ropes, tree_size,
