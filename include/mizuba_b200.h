@@ -53,7 +53,7 @@ typedef struct mzb_opts {
     uint64_t step_end;        /* 0, 0 = all steps (a shard of the time axis) */
     uint32_t bvh_threads;     /* BVH build: 0 = one-pass build; 256, 512, 1024 = level-by-level build with that CTA size */
     uint32_t broad_walk;      /* broad phase: 0 = one position per thread, 1 = warp-coherent, 2 = walks with work refill */
-    uint32_t sort_threads;    /* CTA size of the step sort above 2,048 objects: 256, 512 (0 = automatic) */
+    uint32_t sort_threads;    /* CTA size of the step sort above 2,048 objects: 256, or 512 (0 = 512), which a batch of no more steps than SMs takes as 1,024 */
     uint32_t reserved;        /* must be 0 */
 } mzb_opts;
 

@@ -27,7 +27,7 @@ from .conjunctions import device_conjunctions
 # (broad_walk 2) lost everywhere and is not timed by default.
 BVH_CANDIDATES = (0,)
 BROAD_WALKS = (0, 1)  # one position per thread, warp-coherent
-SORT_CANDIDATES = (256, 512)
+SORT_CANDIDATES = (256, 512)  # 512: the default, 1,024 where a batch has no more steps than SMs
 
 
 def autotune(pj, conj_thresh, conj_det_interval, form="mixed", step_range=None, repeats=2,
