@@ -24,6 +24,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "block.cuh"
@@ -978,11 +979,12 @@ void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_
     for (uint64_t k = 0; k < n_t; ++k)
         if (!std::isfinite(ht[k]))
             throw std::invalid_argument("A non-finite propagation time was passed to mzb_sgp4_propagate()");
-    // Arrays in this device's memory are read and written in place; others
-    // through buffers.
+    // Arrays in this device's memory are read and written in place if they are
+    // aligned as the kernels' loads and stores need; others go through buffers.
     int dev = 0;
     SK(cudaGetDevice(&dev));
-    auto here = [dev](const void *p) {
+    auto here = [dev](const auto *p) {
+        if (reinterpret_cast<uintptr_t>(p) % alignof(std::remove_pointer_t<decltype(p)>) != 0) return false;
         cudaPointerAttributes pa{};
         const bool ok = cudaPointerGetAttributes(&pa, p) == cudaSuccess;
         if (!ok) cudaGetLastError();
