@@ -58,3 +58,22 @@ def test_unaligned_device_arrays(lib, offsets):
     for x, o, a in zip(d[2:], offsets[2:], (out, err)):  # nothing beside them
         rest = x.cpu().numpy()
         assert not rest[:o].any() and not rest[o + a.nbytes:].any()
+
+
+@pytest.mark.parametrize("device", [False, True])
+def test_no_state_is_nan(lib, device):
+    import torch
+
+    g, ts = inputs(24)
+    g["e0"][::3] = 0.999  # below the surface: an error at every time
+    g["bstar"][1::3] = 0.5  # decays within the day
+    out, err = host_result(lib, g, ts, fill=3.0)
+    if device:
+        d = [torch.from_numpy(a.view(np.uint8).reshape(-1).copy()).cuda() for a in (g, ts, np.full_like(out, 3.0), err)]
+        assert lib.mzb_sgp4_propagate(d[0].data_ptr(), len(g), d[1].data_ptr(), len(ts), d[2].data_ptr(),
+                                      d[3].data_ptr()) == 0, lib.mzb_last_error()
+        out = d[2].cpu().numpy().view(np.float64).reshape(out.shape)
+        err = d[3].cpu().numpy().view(np.int32).reshape(err.shape)
+    state = (err == 0) | (err == 6)
+    assert state.any() and (~state).any()
+    assert np.isfinite(out[state]).all() and np.isnan(out[~state]).all()
