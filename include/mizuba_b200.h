@@ -249,14 +249,16 @@ uint64_t mzb_result_n_launches(const mzb_result *r);
  * size, sized by the largest call so far) on the device between calls, so
  * that repeated calls allocate nothing; a freed result's block of per-step
  * outputs is also kept, as the spare the next call of the same size takes.
+ * SGP4 production and propagation keep up to 2 GiB of their memory.
  * This returns the current device's cached blocks and spare to the
- * stream-ordered pool, and frees the pinned buffers (32 MB at most) that
- * copies to pageable memory and files keep; it waits for a screening call in
- * progress on the device to finish.  No counterpart in the reference (its buffers are host
+ * stream-ordered pool and the SGP4 memory that is not in use to the device,
+ * and frees the pinned buffers (32 MB at most) that copies to pageable memory
+ * and files keep; it waits for a screening call in progress on the device to
+ * finish.  No counterpart in the reference (its buffers are host
  * memory owned by each call). */
 int mzb_scratch_release(void);
 /* Bytes of batch scratch and spare output block cached on the current
- * device. */
+ * device, and of its SGP4 memory. */
 uint64_t mzb_scratch_bytes(void);
 
 /* Measures the current device's FP64 FMA issue rate (instructions per

@@ -79,7 +79,8 @@ class device_polyjectory:
 def release_scratch() -> None:
     """Returns the batch scratch that screening calls keep cached on the
     current CUDA device (sized by the largest call so far) to the driver's
-    stream-ordered pool.  Waits for a call in progress on the device."""
+    stream-ordered pool, and the memory that SGP4 production and propagation
+    keep to the device.  Waits for a call in progress on the device."""
     L = _native.core()
     rc = L.mzb_scratch_release()
     if rc:
@@ -87,7 +88,8 @@ def release_scratch() -> None:
 
 
 def scratch_bytes() -> int:
-    """Bytes of batch scratch cached on the current CUDA device."""
+    """Bytes of batch scratch and SGP4 memory cached on the current CUDA
+    device."""
     return int(_native.core().mzb_scratch_bytes())
 
 

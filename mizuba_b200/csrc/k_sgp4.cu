@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -593,8 +594,35 @@ namespace
         if (e_ != cudaSuccess) sgp4_cuda_fail(e_, #x);                                                                 \
     } while (0)
 
-// A device buffer from the stream-ordered pool, on the legacy default stream
-// (all of this file's work is on it).
+// A device's pool for this file's buffers and the produced coefficients, apart
+// from the default one, whose blocks stay with the process: up to KEEP bytes
+// stay between calls (production of 3,000 element sets over a day takes half of
+// that), more goes back to the device at the next synchronisation, and
+// mzb_scratch_release gives back all that is not in use.
+constexpr uint64_t KEEP = uint64_t(2) << 30;
+
+cudaMemPool_t g_pools[64];
+std::once_flag g_pool_flags[64];
+cudaMemPool_t device_pool()
+{
+    int dev = 0;
+    SK(cudaGetDevice(&dev));
+    std::call_once(g_pool_flags[dev & 63], [dev]() {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        SK(cudaMemPoolCreate(&pool, &props));
+        uint64_t keep = KEEP;
+        SK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        g_pools[dev & 63] = pool;
+    });
+    return g_pools[dev & 63];
+}
+
+// A device buffer from it, on the legacy default stream (all of this file's
+// work is on it).
 template <typename T>
 struct devbuf {
     T *p = nullptr;
@@ -613,8 +641,7 @@ struct devbuf {
     void alloc(size_t count)
     {
         release();
-        ensure_device_pool();
-        if (count) SK(cudaMallocAsync(reinterpret_cast<void **>(&p), count * sizeof(T), 0));
+        if (count) SK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), device_pool(), 0));
         n = count;
     }
 };
@@ -924,7 +951,8 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
     out->n_traj = seg_cursor * OP1 * 7;
     out->dev = dev;
     if (out->n_traj)
-        SK(cudaMallocAsync(reinterpret_cast<void **>(&out->d_traj), out->n_traj * sizeof(double), 0));
+        SK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&out->d_traj), out->n_traj * sizeof(double), device_pool(),
+                                   0));
     devbuf<double> d_time(time_cursor);
     devbuf<unsigned long long> d_bad(1);
     SK(cudaMemset(d_bad.p, 0xff, sizeof(unsigned long long)));
@@ -958,6 +986,20 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
 }
 
 void free_sgp4_pj(sgp4_pj_out *p) { delete p; }
+
+void release_scratch()
+{
+    const cudaMemPool_t pool = device_pool();
+    SK(cudaStreamSynchronize(0)); // the frees queued so far
+    SK(cudaMemPoolTrimTo(pool, 0));
+}
+
+uint64_t scratch_bytes()
+{
+    uint64_t b = 0;
+    SK(cudaMemPoolGetAttribute(device_pool(), cudaMemPoolAttrReservedMemCurrent, &b));
+    return b;
+}
 
 void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_t n_t, double *out, int32_t *err)
 {

@@ -34,9 +34,6 @@ struct conj_out {
     uint32_t pad;
 };
 
-// Raises the release threshold of the current device's default memory pool
-// once (pipeline.cu).
-void ensure_device_pool();
 cudaError_t init_aabb_consts();
 cudaError_t measure_dfma_rate(double *per_second);
 cudaError_t init_narrow_consts();
@@ -147,6 +144,10 @@ void gpe_check(const gpe_host *g, uint64_t n, double jd_begin, double jd_end, do
 sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double jd_end, double reentry,
                           double exit_r);
 void free_sgp4_pj(sgp4_pj_out *p);
+// The current device's memory of production and propagation: what is not in use
+// given back, all of it counted.
+void release_scratch();
+uint64_t scratch_bytes();
 void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_t n_t, double *out, int32_t *err);
 } // namespace sgp4pj
 

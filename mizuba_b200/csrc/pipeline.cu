@@ -78,16 +78,6 @@ void ensure_pool()
     });
 }
 
-} // namespace
-
-namespace mzb
-{
-void ensure_device_pool() { ensure_pool(); }
-} // namespace mzb
-
-namespace
-{
-
 // Batch scratch kept between screening calls, one set of blocks per device.
 // Every call allocates the same few dozen scratch buffers of a few GB in
 // total; drawn from the stream-ordered pool afresh each time, their changing
@@ -2480,6 +2470,7 @@ int mzb_scratch_release(void)
         int dev = 0;
         CK(cudaGetDevice(&dev));
         out_lanes().drop(dev);
+        sgp4pj::release_scratch();
     });
 }
 
@@ -2491,7 +2482,7 @@ uint64_t mzb_scratch_bytes(void)
         std::lock_guard<std::mutex> lk(c.m);
         for (const scratch_slot &sl : c.slots) b += sl.bytes;
         std::lock_guard<std::mutex> lk2(c.spare_m);
-        b += c.spare_bytes;
+        b += c.spare_bytes + sgp4pj::scratch_bytes();
     } catch (...) {
     }
     return b;
