@@ -106,6 +106,7 @@ struct scratch_cache {
     std::mutex spare_m;
     void *spare = nullptr;
     size_t spare_bytes = 0;
+    cudaEvent_t spare_free = nullptr; // the default stream when the block became the spare
     // The call's screening and copy streams and its events, created once:
     // creating them per call goes through the driver, where a concurrent
     // query of the GPU (a clock monitor, say) can hold it up.
@@ -143,12 +144,19 @@ struct scratch_lease {
     scratch_slot *next() { return (slots && used < SCRATCH_SLOTS) ? &slots[used++] : nullptr; }
 };
 
-// The spare output block of device dev: taken when it holds at least bytes.
-void *take_spare(int dev, size_t bytes, size_t &got)
+// The spare output block of the current device, dev, for use on stream st:
+// taken when it holds at least bytes.  Copies of the freed result to device
+// memory may still be queued on the default stream, which st does not wait for
+// by itself: it waits for the event of the block's release.
+void *take_spare(int dev, size_t bytes, size_t &got, cudaStream_t st)
 {
     scratch_cache &c = device_scratch_of(dev);
     std::lock_guard<std::mutex> lk(c.spare_m);
     if (!c.spare || c.spare_bytes < bytes) return nullptr;
+    if (cudaStreamWaitEvent(st, c.spare_free, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
     void *p = c.spare;
     got = c.spare_bytes;
     c.spare = nullptr;
@@ -160,24 +168,24 @@ void *take_spare(int dev, size_t bytes, size_t &got)
 void give_spare(int dev, void *p, size_t bytes)
 {
     scratch_cache &c = device_scratch_of(dev);
-    void *drop = nullptr;
+    int cur = 0;
+    cudaGetDevice(&cur);
+    cudaSetDevice(dev);
+    void *drop = p;
     {
         std::lock_guard<std::mutex> lk(c.spare_m);
-        if (c.spare && c.spare_bytes >= bytes) {
-            drop = p;
-        } else {
-            drop = c.spare;
-            c.spare = p;
-            c.spare_bytes = bytes;
+        if (!c.spare || c.spare_bytes < bytes) {
+            if (!c.spare_free && cudaEventCreateWithFlags(&c.spare_free, cudaEventDisableTiming) != cudaSuccess)
+                c.spare_free = nullptr;
+            if (c.spare_free && cudaEventRecord(c.spare_free, 0) == cudaSuccess) {
+                drop = c.spare;
+                c.spare = p;
+                c.spare_bytes = bytes;
+            }
         }
     }
-    if (drop) {
-        int cur = 0;
-        cudaGetDevice(&cur);
-        cudaSetDevice(dev);
-        cudaFreeAsync(drop, 0);
-        cudaSetDevice(cur);
-    }
+    if (drop) cudaFreeAsync(drop, 0);
+    cudaSetDevice(cur);
 }
 
 template <typename T>
@@ -1060,7 +1068,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
         const uint64_t o_tsz = place(S * 4), o_tr = place(S * R.cap * sizeof(bvh_node));
         CK(cudaGetDevice(&R.dev));
         size_t got = 0;
-        if (void *sp = off ? take_spare(R.dev, off, got) : nullptr) {
+        if (void *sp = off ? take_spare(R.dev, off, got, st) : nullptr) {
             R.block = sp;
             R.block_bytes = got;
         } else if (off) {
@@ -1630,8 +1638,9 @@ void stream_out(const std::vector<out_piece> &pieces, F put)
     if (error) std::rethrow_exception(error);
 }
 
-// Device memory to a caller's array, complete on return: pageable memory of a
-// few megabytes or more through the lanes, anything else as one copy.
+// Device memory to a caller's array: pageable memory of a few megabytes or more
+// through the lanes, anything else as one copy.  Complete on return for host
+// memory; a copy to device memory is queued on the default stream.
 void copy_to_caller(void *dst, const void *src, size_t bytes)
 {
     if (bytes >= 2 * OUT_PIECE) {
