@@ -1406,6 +1406,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             n_conj_launches =
                 launch_conj_sort(cq.p, h_cq, nb, cc_cnt.p, cc_off.p, cc_ch.p, cc_cur.p, ckey.p, cidx.p,
                                  R.conj.p + R.n_conj, st);
+            CK(cudaGetLastError()); // the status word has been read before these launches
             CK(cudaEventRecord(ev[6].b, st));
             R.n_conj += h_cq;
             t_bp = ev[3].ms();
