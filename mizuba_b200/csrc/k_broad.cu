@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_steps(const uint32_t *__restric
     __shared__ uint32_t sm[33];
     const uint64_t row = uint64_t(blockIdx.x) * N;
     // 32-bit sums: a batch of 2^32 pairs or more is refused by the host, which
-    // reads the 64-bit totals.
+    // reads the queue's 64-bit count (a tile's sum alone can wrap).
     uint64_t carry = 0;
     for (uint64_t t0 = 0; t0 < N; t0 += SCAN_T * SCAN_K) {
         const uint64_t i0 = t0 + uint64_t(threadIdx.x) * SCAN_K;
@@ -565,10 +565,12 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_steps(const uint32_t *__restric
     if (threadIdx.x == 0) step_tot[blockIdx.x] = carry;
 }
 
-// step_off[b], b <= nb: the pairs of the batch before step b.  host_off and
-// host_visits: device addresses of mapped host memory.
+// step_off[b], b <= nb: the pairs of the batch before step b.  host_off,
+// host_count and host_visits: device addresses of mapped host memory.
 __global__ void __launch_bounds__(SCAN_T) k_step_offsets(const uint64_t *__restrict__ step_tot, uint32_t nb,
                                                          uint64_t *__restrict__ step_off, uint64_t *host_off,
+                                                         const unsigned long long *qcount,
+                                                         unsigned long long *host_count,
                                                          const unsigned long long *visits,
                                                          unsigned long long *host_visits)
 {
@@ -597,16 +599,19 @@ __global__ void __launch_bounds__(SCAN_T) k_step_offsets(const uint64_t *__restr
     }
     if (threadIdx.x == 0) {
         step_off[nb] = host_off[nb] = carry;
+        *host_count = *qcount;
         *host_visits = *visits;
     }
 }
 
 void launch_pair_offsets(const uint32_t *counts, uint64_t N, uint32_t nb, uint32_t *offs, uint64_t *step_tot,
-                         uint64_t *step_off, uint64_t *host_off, const unsigned long long *visits,
+                         uint64_t *step_off, uint64_t *host_off, const unsigned long long *qcount,
+                         unsigned long long *host_count, const unsigned long long *visits,
                          unsigned long long *host_visits, cudaStream_t stream)
 {
     k_scan_steps<<<nb, SCAN_T, 0, stream>>>(counts, N, offs, step_tot);
-    k_step_offsets<<<1, SCAN_T, 0, stream>>>(step_tot, nb, step_off, host_off, visits, host_visits);
+    k_step_offsets<<<1, SCAN_T, 0, stream>>>(step_tot, nb, step_off, host_off, qcount, host_count, visits,
+                                             host_visits);
 }
 
 // counts, *qcount, *walk_next and *visits start at zero.

@@ -78,7 +78,8 @@ void launch_broad_half(const float *srt_aabbs, const bvh_node *trees, uint64_t c
                        uint32_t *counts, uint2 *qpair, uint32_t *qrank, uint64_t qcap, unsigned long long *qcount,
                        unsigned long long *walk_next, int walk, unsigned long long *visits, cudaStream_t stream);
 void launch_pair_offsets(const uint32_t *counts, uint64_t N, uint32_t nb, uint32_t *offs, uint64_t *step_tot,
-                         uint64_t *step_off, uint64_t *host_off, const unsigned long long *visits,
+                         uint64_t *step_off, uint64_t *host_off, const unsigned long long *qcount,
+                         unsigned long long *host_count, const unsigned long long *visits,
                          unsigned long long *host_visits, cudaStream_t stream);
 void launch_broad_lists(uint32_t nb, uint64_t N, const uint32_t *counts, const uint32_t *offs,
                         const uint64_t *step_off, const uint2 *qpair, const uint32_t *qrank, uint64_t n_pairs,

@@ -996,6 +996,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     dev_status *h_status = mbox.take<dev_status>(1);
     unsigned long long *h_bad = mbox.take<unsigned long long>(1);
     unsigned long long *h_visits = mbox.take<unsigned long long>(1);
+    unsigned long long *h_pairs = mbox.take<unsigned long long>(1);
     // Copies of this batch's per-step rows [s0, s0 + nb) of a [S][row] array.
     auto stream_rows = [&](void *host, const void *dev, uint64_t row_bytes, uint64_t s0, uint32_t nb) {
         if (host && row_bytes && nb)
@@ -1251,12 +1252,12 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 launch_broad_half(R.srt_aabbs.p, R.trees.p, R.cap, ropes.p, walks.p, leaf_of.p, R.srt_idx.p,
                                   R.tree_size.p, d_ot, sf, nb, N, counts, qpair.p, qrank.p, qcap, &C->qcount.v,
                                   &C->walk_next.v, broad_walk, &C->visits.v, st);
-                launch_pair_offsets(counts, N, nb, offs.p, step_tot.p, step_off.p, mbox.device(h_so), &C->visits.v,
-                                    mbox.device(h_visits), st);
+                launch_pair_offsets(counts, N, nb, offs.p, step_tot.p, step_off.p, mbox.device(h_so), &C->qcount.v,
+                                    mbox.device(h_pairs), &C->visits.v, mbox.device(h_visits), st);
                 CK(cudaGetLastError());
                 n_broad_launches += 3;
                 CK(cudaStreamSynchronize(st));
-                np_batch = h_so[nb];
+                np_batch = *h_pairs;
                 if (np_batch >= (1ull << 32)) throw std::runtime_error("too many broad-phase pairs in one batch");
                 again = np_batch > qcap;
                 if (again) {
