@@ -59,3 +59,18 @@ def test_copies_queued_behind_other_work():
         torch.cuda.synchronize()
         for name, a in out.items():
             assert np.array_equal(a.cpu().numpy(), want[name]), name
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1, 2])
+def test_copies_around_the_size_that_takes_the_lanes(extra):
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+    pj = synth.build_polyjectory(synth.base_elements(3, np.random.default_rng(1), 0.0), 0.05, order=18)
+    t = np.random.default_rng(2).uniform(0.0, 0.05, (16 << 20) // (3 * 56) + extra)
+    got = pj.state_meval(t)
+    for k in range(0, len(t), 10000):  # 1.7 MB at a time: one copy
+        part = pj.state_meval(t[k:k + 10000])
+        assert np.array_equal(got[:, k:k + 10000].view(np.uint64), part.view(np.uint64))
