@@ -1499,12 +1499,19 @@ struct out_lane {
     cudaStream_t s = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     int dev = 0;
-    out_lane()
+    out_lane() = default;
+    // On the current device; false when there is no pinned memory for it.
+    bool init()
     {
         CK(cudaGetDevice(&dev));
-        CK(cudaMallocHost(reinterpret_cast<void **>(&buf), 2 * OUT_PIECE));
+        if (cudaMallocHost(reinterpret_cast<void **>(&buf), 2 * OUT_PIECE) != cudaSuccess) {
+            buf = nullptr;
+            cudaGetLastError();
+            return false;
+        }
         CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         for (cudaEvent_t &e : ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        return true;
     }
     ~out_lane()
     {
@@ -1523,6 +1530,7 @@ struct out_lane {
 struct out_lane_cache {
     std::mutex m;
     std::vector<std::unique_ptr<out_lane>> idle;
+    // Nothing when a new lane cannot be had.
     std::unique_ptr<out_lane> take(int dev)
     {
         {
@@ -1535,7 +1543,8 @@ struct out_lane_cache {
                     return r;
                 }
         }
-        return std::make_unique<out_lane>();
+        auto r = std::make_unique<out_lane>();
+        return r->init() ? std::move(r) : nullptr;
     }
     void give(std::unique_ptr<out_lane> l)
     {
@@ -1579,6 +1588,8 @@ void cut_pieces(std::vector<out_piece> &v, const void *src, size_t bytes, int to
 // Hands every piece's bytes in host memory to put(piece, host), from several
 // threads at once.  The copies wait for the work on the default stream so far.
 // The first exception of a put or a copy is rethrown once all threads are done.
+// Threads without a lane leave the work to the others, the caller's own copies
+// piece by piece into a pageable buffer then.
 template <typename F>
 void stream_out(const std::vector<out_piece> &pieces, F put)
 {
@@ -1595,11 +1606,20 @@ void stream_out(const std::vector<out_piece> &pieces, F put)
     std::atomic<bool> stop{false};
     std::mutex em;
     std::exception_ptr error;
-    auto work = [&]() {
+    auto work = [&](bool own) {
         std::unique_ptr<out_lane> lane;
         try {
             CK(cudaSetDevice(dev));
             lane = out_lanes().take(dev);
+            if (!lane) {
+                if (!own) return;
+                std::vector<char> buf(OUT_PIECE);
+                for (size_t k; !stop.load() && (k = next.fetch_add(1)) < pieces.size();) {
+                    CK(cudaMemcpy(buf.data(), pieces[k].src, pieces[k].bytes, cudaMemcpyDeviceToHost));
+                    put(pieces[k], buf.data());
+                }
+                return;
+            }
             CK(cudaStreamWaitEvent(lane->s, ready.e, 0));
             auto fetch = [&](int half) {
                 const size_t k = next.fetch_add(1);
@@ -1630,12 +1650,12 @@ void stream_out(const std::vector<out_piece> &pieces, F put)
     std::vector<std::thread> th;
     for (size_t w = 1; w < W; ++w) {
         try {
-            th.emplace_back(work);
+            th.emplace_back(work, false);
         } catch (const std::system_error &) {
             break; // fewer threads do the same
         }
     }
-    work();
+    work(true);
     for (std::thread &t : th) t.join();
     if (error) std::rethrow_exception(error);
 }
