@@ -287,9 +287,11 @@ struct aabb_smem {
 
 // The boxes of one segment per lane, folded into (lb, ub), by the whole warp:
 // `first` is lane's segment (its first coefficient row), lanes with !act do no
-// folding and have none: nothing is copied for them (copying one row in place
-// of all of theirs, 192 steps of 5,000 objects of which 1,000 had no data took
-// 0.49 ms instead of 0.24, every warp reading the same lines of the L2).  SHIFT false: every h_lb is zero, the shift is the identity.
+// folding and have none: they copy the rows of the warp's first lane that has one
+// (there is one).  When all of them copied segment 0's, every warp read the same
+// lines of the L2, and 192 steps of 5,000 objects of which 1,000 had no data took
+// 0.49 ms instead of 0.24; a test for them at every copy cost the other
+// catalogues 2 %.  SHIFT false: every h_lb is zero, the shift is the identity.
 // `unsure` (plain form) is set where the float bounds are not proven.
 //
 // With scr != nullptr (mixed form) the pass also writes the distance screen's
@@ -312,7 +314,7 @@ __device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_bi
 #pragma unroll
         for (int k = 0; k < (32 + F::GROUPS - 1) / F::GROUPS; ++k) {
             const unsigned r = grp + unsigned(k * F::GROUPS);
-            if (grp < F::GROUPS && r < 32 && S.base[r]) {
+            if (grp < F::GROUPS && r < 32) {
                 const double2 *src = S.base[r] + v * F::UNITS + part;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                                  dst0 + unsigned(k * F::GROUPS * F::STRIDE * 16)),
@@ -322,7 +324,9 @@ __device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_bi
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    S.base[lane] = reinterpret_cast<const double2 *>(first);
+    const unsigned has = __ballot_sync(0xffffffffu, act);
+    const unsigned long long other = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(first), __ffs(has) - 1);
+    S.base[lane] = act ? reinterpret_cast<const double2 *>(first) : reinterpret_cast<const double2 *>(other);
     __syncwarp();
     fetch(0);
     const double delta = h_ub - h_lb;
