@@ -1160,11 +1160,14 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
     for (const auto &e : {std::pair(0, 1), std::pair(1, 2), std::pair(2, 3), std::pair(3, 4), std::pair(5, 6),
                           std::pair(6, 7), std::pair(8, 9)})
         ev.emplace_back(cst.ev[e.first], cst.ev[e.second]);
-    // Queue entries per broad-phase pair seen so far in this call (items,
-    // root items, conjunctions): the next batch's queues are sized from
+    // Queue entries per broad-phase pair seen so far in this call (items, root
+    // items, conjunctions, items left by the filter): the next batch's queues are sized from
     // them, since an overflow reruns the batch's narrow phase and root
     // finding.
     double items_per_pair = 2.0, roots_per_pair = 0.5, conj_per_pair = 0.125;
+    // Items that the filter leaves: as many as could go on to the root queue;
+    // at orders where its margin can be too wide to settle anything, all.
+    double surv_per_pair = pj.order <= 28 ? roots_per_pair : items_per_pair;
     const double thresh2 = thresh * thresh;
     const double radius = thresh / 2;
 
@@ -1304,12 +1307,13 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             // stage reruns with grown queues on overflow.
             auto sized = [np_batch](double per_pair) { return uint64_t(double(np_batch) * per_pair * 1.1) + 1024; };
             // The mixed form screens items as they are found: no item queue,
-            // the screen's queue (cand) is sized for every item instead, as
-            // is the queue of the items that the filter leaves (surv).
+            // the screen's queue (cand) is sized for every item instead.  The
+            // filter leaves a few percent of them (surv).
             const uint64_t item_cap0 = std::max<uint64_t>(mixed ? cand.n : items.n, sized(items_per_pair));
             if (!mixed && items.n < item_cap0) items.alloc_queue(item_cap0, st);
             if (mixed && cand.n < item_cap0) cand.alloc_queue(item_cap0, st);
-            if (surv.n < (mixed ? cand.n : items.n)) surv.alloc_queue(mixed ? cand.n : items.n, st);
+            const uint64_t surv_cap0 = std::max<uint64_t>(surv.n, sized(surv_per_pair));
+            if (surv.n < surv_cap0) surv.alloc_queue(surv_cap0, st);
             const uint64_t rq_cap0 = std::max<uint64_t>(rq.n, sized(roots_per_pair));
             if (rq.n < rq_cap0) rq.alloc_queue(rq_cap0, st);
             if (retry.n < rq.n) retry.alloc_queue(rq.n, st);
@@ -1370,7 +1374,10 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
                 if (h_items > (mixed ? cand.n : items.n)) {
                     dbuf<np_item> &q = mixed ? cand : items;
                     q.alloc_queue(h_items + h_items / 4, st);
-                    surv.alloc_queue(q.n, st);
+                    again = true;
+                }
+                if (h_surv > surv.n) {
+                    surv.alloc_queue(h_surv + h_surv / 4, st);
                     again = true;
                 }
                 if (h_rq > rq.n) {
@@ -1388,6 +1395,7 @@ void run_detection(const mzb_pj &pj, double thresh, double interval, const int32
             check_status(); // the ordering below sets no error
             if (np_batch) {
                 items_per_pair = std::max(items_per_pair, double(h_items) / double(np_batch));
+                surv_per_pair = std::max(surv_per_pair, double(h_surv) / double(np_batch));
                 roots_per_pair = std::max(roots_per_pair, double(h_rq) / double(np_batch));
                 conj_per_pair = std::max(conj_per_pair, double(h_cq) / double(np_batch));
             }

@@ -108,3 +108,23 @@ def test_threshold_at_the_minimum(mzb, order):
         for d in dca:
             for e in (0.0, 1e-15, -1e-15, 1e-12, -1e-12, 1e-8, -1e-8, -1e-3):
                 same(mzb, pair_pj(ci, cj), d * (1 + e), ("plain", "mixed"))
+
+
+def test_more_left_than_the_queue_expects(mzb):
+    """A first call whose filter leaves nearly every item: its queue is grown
+    and the narrow phase run again."""
+    from mizuba_b200 import synth
+
+    pj = synth.build_polyjectory(synth.base_elements(400, np.random.default_rng(9), 0.0), 0.1, order=18)
+    thresh, interval = 3000.0, 3.0 / 1440.0
+    r = oracle.run(pj, thresh, interval)
+    mzb.release_scratch()
+    for _ in range(2):
+        for form in ("plain", "mixed"):
+            g = mzb.device_conjunctions(pj, thresh, interval, form=form)
+            a, b = g.conjunctions, r["conjunctions"]
+            assert g.np_report[0] >= r["np_report"][0] and len(a) == len(b) > 10000
+            for f in ("i", "j", "tca", "dca", "ri", "vi", "rj", "vj"):
+                assert np.array_equal(a[f], b[f]), f
+            if form == "plain":
+                assert g.np_report == r["np_report"]
