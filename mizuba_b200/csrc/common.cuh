@@ -337,16 +337,6 @@ __device__ __forceinline__ uint32_t lower_bound_t(const double *t, uint32_t lo, 
     return lo;
 }
 
-// Range [tb, te) of time indices `it` whose step [t[it-1], t[it]) overlaps
-// [cb, ce) (detect_conjunctions_aabbs.cpp:130-142).
-__device__ __forceinline__ void step_range(const double *t, uint32_t ns, double cb, double ce, uint32_t &tb,
-                                           uint32_t &te)
-{
-    tb = upper_bound_t(t, 1, ns + 1, cb);
-    te = lower_bound_t(t, tb, ns + 1, ce);
-    te += (te != ns + 1);
-}
-
 // Order-preserving map of a float's bits to uint32 (for atomic min/max).
 __device__ __forceinline__ uint32_t f2ord(float f)
 {

@@ -421,12 +421,13 @@ __device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_bi
     }
 }
 
-// step_range for an object whose data overlap [cb, ce): the first segment end
-// after cb is looked for around the place it would have if the segments were
-// equally long (most objects' are), so that it usually takes two dependent
-// loads instead of a binary search's seven.
-__device__ __forceinline__ void step_range_near(const double *t, uint32_t ns, double t0, double tn, double cb,
-                                                double ce, uint32_t &tb, uint32_t &te)
+// Range [tb, te) of time indices `it` whose step [t[it-1], t[it]) overlaps
+// [cb, ce) (detect_conjunctions_aabbs.cpp:130-142), for an object whose data do.
+// The first segment end after cb is looked for around the place it would have
+// if the segments were equally long (most objects' are), so that it usually
+// takes two dependent loads instead of a binary search's seven.
+__device__ __forceinline__ void step_range(const double *t, uint32_t ns, double t0, double tn, double cb,
+                                           double ce, uint32_t &tb, uint32_t &te)
 {
     const double x = (cb - t0) / (tn - t0) * double(ns);
     uint32_t lo = 1, hi = ns; // t[ns] > cb: the answer is in [lo, hi]
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(AABB_T, aabb_shape<OP1>::CTAS)
         const double t0 = t[0], tn = t[ns];
         if (!(t0 >= ce || tn <= cb)) {
             uint32_t tb, te;
-            step_range_near(t, ns, t0, tn, cb, ce, tb, te);
+            step_range(t, ns, t0, tn, cb, ce, tb, te);
             rng = make_uint2(tb, te);
             if (tb != te) {
                 seg = true;

@@ -62,8 +62,6 @@ constexpr double X2O3 = 2.0 / 3.0;
 // velocity unit RE * XKE / 60 in km/s.
 MZB_HD inline double xke() { return 60.0 / std::sqrt(RE * RE * RE / MU); }
 
-// One element set after set-up: the mean elements at epoch (un-Kozai mean
-// motion no) and the secular and drag terms SGP4 derives from them.
 // Sine and cosine of one argument: one call on the device, where the two
 // share the argument reduction (the same values as apart).
 MZB_HD inline void sc(double x, double &s, double &c)
@@ -76,6 +74,8 @@ MZB_HD inline void sc(double x, double &s, double &c)
 #endif
 }
 
+// One element set after set-up: the mean elements at epoch (un-Kozai mean
+// motion no) and the secular and drag terms SGP4 derives from them.
 struct sat {
     double no, ecco, inclo, nodeo, argpo, mo, bstar;
     double mdot, argpdot, nodedot, nodecf, omgcof, xmcof, xlcof, aycof;
