@@ -448,11 +448,12 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 //   - an object's coordinate at a node: the reference formulation (powers,
 //     binomial sums, Horner) is within sum (3k + 8) u |c_k| e^k of its exact
 //     value, this one (shift, scaling, even and odd Horner) within sum (4k + 5)
-//     u |c_k| e^k, e = delta + rf_int, and 7k + 14 <= 18 (5/4)^k.  With P_c the
-//     sum of |c_k| (5e/4)^k over both objects' coordinate c and P^2 = sum P_c^2,
-//     the squared distance at node m differs by at most 36 u P sqrt(f_m) +
-//     324 u^2 P^2 + 10 u f_m, and a Bernstein coefficient by node_w[m] times
-//     that.  Their sum over the nodes is bounded with F = sum node_w[m] f_m
+//     u |c_k| e^k, e = delta + rf_int, and 7k + 14 <= 39.2 1.08^k (no base is
+//     closer over coefficients that fall off, k about 3, and ones that do not).
+//     With P_c the sum of |c_k| (1.08 e)^k over both objects' coordinate c and
+//     P^2 = sum P_c^2, the squared distance at node m differs by at most 78.4 u P
+//     sqrt(f_m) + 1537 u^2 P^2 + 10 u f_m, and a Bernstein coefficient by
+//     node_w[m] times that.  Their sum over the nodes is bounded with F = sum node_w[m] f_m
 //     (Cauchy-Schwarz); the weights, 1.3 times the largest Bernstein coefficient
 //     of the Chebyshev polynomial together, are largest in the middle, where an
 //     encounter is close;
@@ -629,9 +630,9 @@ static void filter_margins(filter_tables &t, int n)
             }
         t.newton[l] = double(slack * u * g);
     }
-    t.value = double(slack * u * std::sqrt(L) * 36);
+    t.value = double(slack * u * std::sqrt(L) * 78.4);
     t.square = double(slack * u * 10);
-    t.norm = double(slack * u * u * L * 324);
+    t.norm = double(slack * u * u * L * 1537);
     t.mono = double(slack * u * (6 * n + 24));
 }
 
@@ -723,9 +724,9 @@ __global__ void __launch_bounds__(32, filter_shape<OP1>::CTAS)
         if (OP1 & 1) c[OP1 - 1] = r[OP1 / 2].x;
         __syncwarp();
     };
-    // Shift to the origin a; returns sum |c_k| (5/4 e)^k first.
+    // Shift to the origin a; returns sum |c_k| (1.08 e)^k first.
     auto shifted = [](double(&c)[OP1], double a, double e) {
-        e *= 1.25;
+        e *= 1.08;
         double p = fabs(c[n]);
 #pragma unroll
         for (int k = n - 1; k >= 0; --k) p = fma(p, e, fabs(c[k]));

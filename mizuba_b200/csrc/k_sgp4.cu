@@ -565,15 +565,21 @@ __global__ void __launch_bounds__(128) k_sgp4_propagate(const sgp4::sat *sats, c
     if (g >= n * n_t) return;
     const uint64_t i = g / n_t, t = g % n_t;
     int e = init[i];
-    double r[3], v[3];
-    if (e == 0) e = sgp4::propagate(sats[i], tsince[t], r, v);
-    // Decay (6) has a state; the other errors come before there is one.
-    const bool state = e == 0 || e == 6;
     double *o = out + g * 6;
-    for (int k = 0; k < 3; ++k) {
-        o[k] = state ? r[k] : NAN;
-        o[3 + k] = state ? v[k] : NAN;
+    bool state = false;
+    if (e == 0) {
+        double r[3], v[3];
+        e = sgp4::propagate(sats[i], tsince[t], r, v);
+        // Decay (6) has a state; the other errors come before there is one.
+        state = e == 0 || e == 6;
+        if (state)
+            for (int k = 0; k < 3; ++k) {
+                o[k] = r[k];
+                o[3 + k] = v[k];
+            }
     }
+    if (!state)
+        for (int k = 0; k < 6; ++k) o[k] = NAN;
     err[g] = e;
 }
 
