@@ -1037,16 +1037,17 @@ void sgp4_propagate(const gpe_host *g, uint64_t n, const double *tsince, uint64_
     };
     const bool g_here = here(g), t_here = here(tsince), out_here = here(out), err_here = here(err);
     devbuf<gpe_host> d_g(g_here ? 0 : n);
-    devbuf<sgp4::sat> d_sats(n);
+    devbuf<char> d_set(n * (sizeof(sgp4::sat) + sizeof(int))); // set-ups, then their error codes
+    sgp4::sat *const sats = reinterpret_cast<sgp4::sat *>(d_set.p);
+    int *const init = reinterpret_cast<int *>(sats + n);
     devbuf<double> d_t(t_here ? 0 : n_t), d_out(out_here ? 0 : n * n_t * 6);
-    devbuf<int> d_init(n), d_err(err_here ? 0 : n * n_t);
+    devbuf<int> d_err(err_here ? 0 : n * n_t);
     double *po = out_here ? out : d_out.p;
     int *pe = err_here ? err : d_err.p;
     if (!g_here) SK(cudaMemcpyAsync(d_g.p, g, n * sizeof(gpe_host), cudaMemcpyDefault, 0));
     if (!t_here) SK(cudaMemcpyAsync(d_t.p, tsince, n_t * 8, cudaMemcpyDefault, 0));
-    k_sgp4_setup_gpes<<<unsigned((n + 63) / 64), 64>>>(g_here ? g : d_g.p, n, d_sats.p, d_init.p);
-    k_sgp4_propagate<<<unsigned((n * n_t + 127) / 128), 128>>>(d_sats.p, d_init.p, n, t_here ? tsince : d_t.p, n_t,
-                                                                po, pe);
+    k_sgp4_setup_gpes<<<unsigned((n + 63) / 64), 64>>>(g_here ? g : d_g.p, n, sats, init);
+    k_sgp4_propagate<<<unsigned((n * n_t + 127) / 128), 128>>>(sats, init, n, t_here ? tsince : d_t.p, n_t, po, pe);
     SK(cudaGetLastError());
     if (!out_here) SK(cudaMemcpy(out, po, n * n_t * 6 * 8, cudaMemcpyDefault));
     if (!err_here) SK(cudaMemcpy(err, pe, n * n_t * 4, cudaMemcpyDefault));
