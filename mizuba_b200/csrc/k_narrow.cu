@@ -1385,10 +1385,11 @@ __device__ void states_at_t(const dev_pj &pj, uint64_t gseg, double delta, doubl
 // shift, lanes 0 to 11 one state variable each, and all lanes run the scalar
 // part (fast exclusion, TOMS 748) on coefficients in shared memory; every
 // value comes from the same operations in the same order.  52 items 46 -> 23
-// us, 2,500 sub-intervals' left-overs of the 1,000-object day 73 -> 28 us;
-// beyond one item a resident warp (2,368 of them) the thread per item is as
-// fast and keeps all lanes busy (11,000 items: 79 against 95 us).
-constexpr uint64_t ROOTS_WARP_ITEMS = 2048;
+// us, 2,700 items 83 -> 46, 5,000 items 89 -> 68; at order 25 2,200 items 133 ->
+// 58 us, 6,400 items 136 -> 141.  Beyond two items a resident warp (4,736 of
+// them) the thread per item is as fast and keeps all lanes busy (11,000 items:
+// 79 against 95 us).
+constexpr uint64_t ROOTS_WARP_ITEMS = 4096;
 constexpr int ROOTS_T = 128;
 
 template <int OP1>

@@ -128,3 +128,18 @@ def test_more_left_than_the_queue_expects(mzb):
                 assert np.array_equal(a[f], b[f]), f
             if form == "plain":
                 assert g.np_report == r["np_report"]
+
+
+@pytest.mark.parametrize("thresh", [900.0, 1100.0, 1300.0, 1600.0])
+def test_root_items_around_two_a_warp(mzb, thresh):
+    from mizuba_b200 import synth
+
+    pj = synth.build_polyjectory(synth.base_elements(150, np.random.default_rng(9), 0.0), 0.1, order=18)
+    r = oracle.run(pj, thresh, 3.0 / 1440.0)
+    assert 1200 < len(r["conjunctions"]) < 3000  # root items: these and some more
+    g = mzb.device_conjunctions(pj, thresh, 3.0 / 1440.0)
+    assert g.np_report == r["np_report"]
+    a, b = g.conjunctions, r["conjunctions"]
+    assert len(a) == len(b)
+    for f in ("i", "j", "tca", "dca", "ri", "vi", "rj", "vj"):
+        assert np.array_equal(a[f], b[f]), f
