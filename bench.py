@@ -701,12 +701,12 @@ def main():
         # Bjorck-Pereyra, Cargo-Shisha).  Filter (both forms): per coordinate
         # both polynomials' magnitude bounds and shifts, their scaled
         # difference and its even and odd parts at the nodes' mirror pairs;
-        # then Bjorck-Pereyra with reciprocals and Cargo-Shisha with the
-        # differences of its coefficients.
+        # then Bjorck-Pereyra with reciprocals, Cargo-Shisha with the
+        # differences of its coefficients and the margin's three sums.
         ops_plain = (2 * 3 * (3 * m * (m + 1) // 2 + n) + 2 * 6 * m * n + 8 * m
                      + (3 * n * (n + 1) // 2 + n * (n + 1)) + (3 * n + m + n * (n + 1) // 2 + 2 * m))
         ops_filter = (3 * (n * (n + 1) + 2 * n + 3 * m - 1 + (m // 2) * (n + 1) + m)
-                      + 3 * n * (n + 1) // 2 + m + n * (n + 1) // 2 + 4 * n)
+                      + 3 * n * (n + 1) // 2 + m + n * (n + 1) // 2 + 4 * n + 3 * m)
         # Narrow stage: in the mixed form the distance screen on every item
         # (about 65 FP64 operations from the two stored linear models), then
         # the filter on the items that pass it (in the plain form: on all).

@@ -604,8 +604,13 @@ namespace
 // from the default one, whose blocks stay with the process: up to KEEP bytes
 // stay between calls (production of 3,000 element sets over a day takes half of
 // that), more goes back to the device at the next synchronisation, and
-// mzb_scratch_release gives back all that is not in use.
+// mzb_scratch_release gives back all that is not in use.  Blocks of LARGE bytes
+// or more (whole catalogues over days) are the device's own allocations instead,
+// which cost 1.2 ms for 4 GB and go back when freed: from the pool, past KEEP,
+// every synchronisation of a call unmapped what its next buffers mapped again (7
+// ms a gigabyte; one day of 26,389 element sets 57 -> 350 ms).
 constexpr uint64_t KEEP = uint64_t(2) << 30;
+constexpr size_t LARGE = size_t(512) << 20;
 
 cudaMemPool_t g_pools[64];
 std::once_flag g_pool_flags[64];
@@ -627,8 +632,21 @@ cudaMemPool_t device_pool()
     return g_pools[dev & 63];
 }
 
-// A device buffer from it, on the legacy default stream (all of this file's
-// work is on it).
+void *device_alloc(size_t bytes)
+{
+    void *p = nullptr;
+    if (bytes >= LARGE) SK(cudaMalloc(&p, bytes));
+    else if (bytes) SK(cudaMallocFromPoolAsync(&p, bytes, device_pool(), 0));
+    return p;
+}
+void device_free(void *p, size_t bytes)
+{
+    if (bytes >= LARGE) cudaFree(p);
+    else if (p) cudaFreeAsync(p, 0);
+}
+
+// A device buffer, on the legacy default stream (all of this file's work is on
+// it).
 template <typename T>
 struct devbuf {
     T *p = nullptr;
@@ -640,14 +658,14 @@ struct devbuf {
     ~devbuf() { release(); }
     void release()
     {
-        if (p) cudaFreeAsync(p, 0);
+        device_free(p, n * sizeof(T));
         p = nullptr;
         n = 0;
     }
     void alloc(size_t count)
     {
         release();
-        if (count) SK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), device_pool(), 0));
+        p = static_cast<T *>(device_alloc(count * sizeof(T)));
         n = count;
     }
 };
@@ -956,9 +974,7 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
     SK(cudaMemcpy(d_sat_time_off.p, sat_time_off.data(), n_sats * 8, cudaMemcpyHostToDevice));
     out->n_traj = seg_cursor * OP1 * 7;
     out->dev = dev;
-    if (out->n_traj)
-        SK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&out->d_traj), out->n_traj * sizeof(double), device_pool(),
-                                   0));
+    out->d_traj = static_cast<double *>(device_alloc(out->n_traj * sizeof(double)));
     devbuf<double> d_time(time_cursor);
     devbuf<unsigned long long> d_bad(1);
     SK(cudaMemset(d_bad.p, 0xff, sizeof(unsigned long long)));
@@ -992,6 +1008,16 @@ sgp4_pj_out *make_sgp4_pj(const gpe_host *g, uint64_t n, double jd_begin, double
 }
 
 void free_sgp4_pj(sgp4_pj_out *p) { delete p; }
+
+sgp4_pj_out::~sgp4_pj_out()
+{
+    if (!d_traj) return;
+    int cur = 0;
+    cudaGetDevice(&cur);
+    cudaSetDevice(dev);
+    device_free(d_traj, n_traj * sizeof(double));
+    cudaSetDevice(cur);
+}
 
 void release_scratch()
 {

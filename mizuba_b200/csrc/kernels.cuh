@@ -130,15 +130,7 @@ struct sgp4_pj_out {
     sgp4_pj_out(const sgp4_pj_out &) = delete;
     sgp4_pj_out &operator=(const sgp4_pj_out &) = delete;
     int dev = 0; // the device of d_traj
-    ~sgp4_pj_out()
-    {
-        if (!d_traj) return;
-        int cur = 0;
-        cudaGetDevice(&cur);
-        cudaSetDevice(dev);
-        cudaFreeAsync(d_traj, 0);
-        cudaSetDevice(cur);
-    }
+    ~sgp4_pj_out();
 };
 dfl utc_to_tai(dfl utc);
 void gpe_check(const gpe_host *g, uint64_t n, double jd_begin, double jd_end, double reentry, double exit_r);
