@@ -32,16 +32,17 @@ typedef struct mzb_pj mzb_pj;         /* a polyjectory resident in HBM */
 typedef struct mzb_result mzb_result; /* a conjunctions result resident in HBM */
 
 /* Screening forms.
- * MZB_FORM_PLAIN: the reference's FP64 formulation operation for operation
- *   (boxes, codes, order, trees and pairs bit-exact with the oracle).
+ * MZB_FORM_PLAIN: the results of the reference's FP64 formulation (boxes, codes,
+ *   order, trees and pairs bit-exact with the oracle, records and narrow-phase
+ *   counters its own): FMA evaluations settle what their error bounds prove,
+ *   the rest is computed operation for operation.
  * MZB_FORM_MIXED: FMA-native FP64 enclosures widened by an a-posteriori
  *   rounding bound (boxes provably contain the plain form's, so overlapping
- *   pairs are a superset), FP32 broad phase as in the plain form, a
- *   rigorous distance screen (linear model with a Taylor remainder bound),
- *   and an FMA-native FP64 prefilter of the narrow phase (shifted-node
- *   evaluation, conservative prune) whose survivors are recomputed with the
- *   reference formulation: the conjunction records are the plain form's
- *   (the narrow-phase counters are not: fewer items reach root finding). */
+ *   pairs are a superset), FP32 broad phase as in the plain form, and a
+ *   rigorous distance screen (linear model with a Taylor remainder bound) ahead
+ *   of the plain form's narrow phase: the conjunction records are the plain
+ *   form's (the narrow-phase counters are not: fewer items reach root
+ *   finding). */
 #define MZB_FORM_PLAIN 0u
 #define MZB_FORM_MIXED 1u
 

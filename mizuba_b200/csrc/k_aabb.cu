@@ -204,7 +204,7 @@ void launch_relayout_runs(const char *piece, uint64_t n_runs, double *coef, int 
 // at an odd stride of 16-byte units (conflict-free), and has the next
 // variable's copies in flight while it computes.
 // 20,000-object day (11.4 M boxes of four variables at order 18): plain form
-// 3.8 -> 2.1 ms (the reference formulation for every box took 1,018 FP64
+// 3.8 -> 1.9 ms (the reference formulation for every box took 1,018 FP64
 // operations a variable, this one 455), mixed form 2.5 -> 2.0 ms; 60 % of the
 // FP64 rate, the rest is latency at the start of a warp's work (segment
 // search, first rows).
@@ -276,7 +276,7 @@ struct aabb_shape {
     static constexpr int STRIDE = UNITS | 1;      // odd: conflict-free 16-byte reads
     static constexpr int GROUPS = 32 / UNITS;     // rows copied per instruction
     // CTAs an SM: 80 registers a thread hold an order-18 table without
-    // spilling (day 2.12 ms; 2.18 at four CTAs, 118 registers).
+    // spilling (day 2.12 ms when measured; 2.18 at four CTAs, 118 registers).
     static constexpr int CTAS = OP1 <= 20 ? 6 : OP1 <= 26 ? 4 : 3;
 };
 template <int OP1>
@@ -325,8 +325,9 @@ __device__ __forceinline__ void warp_segment_box(aabb_smem<OP1> &S, const inv_bi
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const unsigned has = __ballot_sync(0xffffffffu, act);
-    const unsigned long long other = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(first), __ffs(has) - 1);
-    S.base[lane] = act ? reinterpret_cast<const double2 *>(first) : reinterpret_cast<const double2 *>(other);
+    const unsigned long long row = reinterpret_cast<unsigned long long>(first);
+    const unsigned long long other = __shfl_sync(0xffffffffu, row, __ffs(has) - 1);
+    S.base[lane] = reinterpret_cast<const double2 *>(act ? row : other);
     __syncwarp();
     fetch(0);
     const double delta = h_ub - h_lb;

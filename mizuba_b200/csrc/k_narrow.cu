@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 // where all but 1 % turn out to have one minimum, above the threshold.  The
 // reference formulation takes 8,921 FP64 operations and 190 divisions for an
 // item, and root finding as much again; which of the two outcomes it will
-// have can be proven from an FMA-native evaluation of 2,500 operations:
+// have can be proven from an FMA-native evaluation of 2,700 operations:
 //
 // * both objects' segment polynomials are shifted to the sub-interval's
 //   midpoint (synthetic division) and subtracted, and the difference is
@@ -453,10 +453,10 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 //     With P_c the sum of |c_k| (1.08 e)^k over both objects' coordinate c and
 //     P^2 = sum P_c^2, the squared distance at node m differs by at most 78.4 u P
 //     sqrt(f_m) + 1537 u^2 P^2 + 10 u f_m, and a Bernstein coefficient by
-//     node_w[m] times that.  Their sum over the nodes is bounded with F = sum node_w[m] f_m
-//     (Cauchy-Schwarz); the weights, 1.3 times the largest Bernstein coefficient
-//     of the Chebyshev polynomial together, are largest in the middle, where an
-//     encounter is close;
+//     node_w[m] times that.  Their sum over the nodes is bounded with
+//     F = sum node_w[m] f_m (Cauchy-Schwarz); the weights, together 1.3 times the
+//     largest Bernstein coefficient of the Chebyshev polynomial, are largest in
+//     the middle, where an encounter is close;
 //   - each divided difference has a relative rounding of 4 u here, 3 u there and
 //     u (c_j + c_i) / (c_j - c_i) for the nodes c rf_int there; each step from
 //     Newton form to monomials four roundings of what it adds up.  All of them
@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 // constants as kernel parameters (operands of the instructions instead of
 // loads) leave room for 16 warps an SM at order 18 (124 registers; 12 warps
 // are 4 % slower, 18 with spills 14 %).  6.38 M items of the 20,000-object day:
-// 1.7 ms (2.6 with Horner at every node and both objects' rows, 168
-// registers and 12 warps).  With the merge walk and root finding, the plain
+// 1.8 ms (2.6 with Horner at every node and both objects' rows, 168
+// registers and 12 warps; 0.04 of it are the margin's sums).  With the merge walk and root finding, the plain
 // form's narrow phase took 10.4 ms with the reference formulation for every
 // item and takes 2.2; 60,000 objects x 48 steps at 20 km, mixed, 11.9 and 4.2.
 struct filter_tables {
@@ -2155,9 +2155,10 @@ void launch_narrow(const dev_pj &pj, const double *shift, const double2 *cdb, ui
 }
 
 template <int OP1>
-static void filter_t(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count, uint64_t item_cap,
-                     double thresh2, np_item *surv, uint64_t surv_cap, unsigned long long *surv_count,
-                     unsigned long long *counters, cudaStream_t stream)
+static void filter_t(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items,
+                     const unsigned long long *item_count, uint64_t item_cap, double thresh2, np_item *surv,
+                     uint64_t surv_cap, unsigned long long *surv_count, unsigned long long *counters,
+                     cudaStream_t stream)
 {
     using F = filter_shape<OP1>;
     static const filter_consts<OP1> consts = make_filter_consts<OP1>();
@@ -2165,9 +2166,10 @@ static void filter_t(const dev_pj &pj, const double2 *cdb, uint32_t s_first, con
                                                              thresh2, surv, surv_cap, surv_count, counters);
 }
 
-void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count,
-                          uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
-                          unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream)
+void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items,
+                          const unsigned long long *item_count, uint64_t item_cap, double thresh2, np_item *surv,
+                          uint64_t surv_cap, unsigned long long *surv_count, unsigned long long *counters,
+                          cudaStream_t stream)
 {
     switch (pj.op1) {
 #define X(K)                                                                                                         \

@@ -96,9 +96,10 @@ void launch_items_screen(const dev_pj &pj, const double2 *cdb, uint32_t s_first,
                          const float4 *scr, np_item *cand, uint64_t cand_cap, unsigned long long *cand_count,
                          unsigned long long *item_count, unsigned long long *counters, dev_status *st,
                          cudaStream_t stream);
-void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items, const unsigned long long *item_count,
-                          uint64_t item_cap, double thresh2, np_item *surv, uint64_t surv_cap,
-                          unsigned long long *surv_count, unsigned long long *counters, cudaStream_t stream);
+void launch_narrow_filter(const dev_pj &pj, const double2 *cdb, uint32_t s_first, const np_item *items,
+                          const unsigned long long *item_count, uint64_t item_cap, double thresh2, np_item *surv,
+                          uint64_t surv_cap, unsigned long long *surv_count, unsigned long long *counters,
+                          cudaStream_t stream);
 constexpr int ROOTS_WL_SMALL = 24;  // working-list entries per thread, first pass
 constexpr int ROOTS_WL_FULL = 251;  // the reference's bound (list size > 250 fails)
 void launch_roots(const dev_pj &pj, const double *shift, const root_item *rq, const unsigned long long *rq_count, uint64_t rq_cap,
