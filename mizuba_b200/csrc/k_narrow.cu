@@ -30,6 +30,7 @@
 
 #include "block.cuh"
 #include "common.cuh"
+#include "filter_margin.cuh"
 #include "kernels.cuh"
 
 namespace mzb
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 //   table of Cargo-Shisha;
 // * both formulations interpolate the same polynomial's values on the same
 //   nodes, and M bounds how far their Bernstein coefficients can differ by
-//   rounding, u = 2^-53 (filter_margins):
+//   rounding, u = 2^-53 (filter_margins, in filter_margin.cuh):
 //   - an object's coordinate at a node: the reference formulation (powers,
 //     binomial sums, Horner) is within sum (3k + 8) u |c_k| e^k of its exact
 //     value, this one (shift, scaling, even and odd Horner) within sum (4k + 5)
@@ -502,140 +503,7 @@ __global__ void __launch_bounds__(NARROW_T) k_narrow(dev_pj pj, cheb_nodes cheb,
 // registers and 12 warps; 0.04 of it are the margin's sums).  With the merge walk and root finding, the plain
 // form's narrow phase took 10.4 ms with the reference formulation for every
 // item and takes 2.2; 60,000 objects x 48 steps at 20 km, mixed, 11.9 and 4.2.
-struct filter_tables {
-    double x[MAX_OP1 / 2], y[MAX_OP1 / 2]; // nodes in (0, 1] of [-1, 1], descending, and their squares
-    double node[MAX_OP1];                  // nodes of [0, 1], ascending
-    double inv_binom[MAX_OP1];
-    double node_w[MAX_OP1];                // F = sum node_w[m] f_m
-    double newton[MAX_OP1];                // margin per Newton coefficient
-    double value, square, norm, mono;      // and per sqrt(F) P, F, P^2 and sum |f_k|
-    double rf_lo, rf_hi;                   // range of sub-interval lengths
-};
-// Where the filter's argument holds for order n: the reference formulation
-// divides differences of f by node distances c rf_int, so its k-th divided
-// differences are at most 2^k max f / (G_k rf_int^k), G_k the product of the
-// smallest node distances at lags 1 to k; with max f <= 1e30 they stay below
-// 1e280 for rf_int >= rf_lo, and neither rf_int^n nor its inverse leaves the
-// exponent range for rf_int in [rf_lo, rf_hi].
-static void filter_range(filter_tables &t, int n)
-{
-    t.rf_lo = std::pow(10.0, -250.0 / n);
-    t.rf_hi = std::pow(10.0, 200.0 / n);
-    double log_g = 0;
-    for (int k = 1; k <= n; ++k) {
-        double gap = 1.0;
-        for (int j = k; j <= n; ++j) gap = std::min(gap, t.node[j] - t.node[j - k]);
-        log_g += std::log10(gap);
-        t.rf_lo = std::max(t.rf_lo, std::pow(10.0, (k * std::log10(2.0) + 30.0 - log_g - 280.0) / k));
-    }
-}
-
-// The weights of the margin M (above) for order n.  Everything here is a
-// linear map of the few dozen numbers of an item; the maps are applied to unit
-// vectors in long double and the results' largest Bernstein coefficients taken.
-static void filter_margins(filter_tables &t, int n)
-{
-    using real = long double;
-    using vec = std::vector<real>;
-    const double *c = t.node;
-    const size_t m = size_t(n) + 1;
-    // p (s - r) and the degree elevation of p, in Bernstein form over [0, 1].
-    auto times_root = [](const vec &p, real r) {
-        const int d = int(p.size()) - 1;
-        vec q(size_t(d) + 2, 0);
-        for (int i = 0; i <= d + 1; ++i) {
-            if (i <= d) q[i] -= r * (d + 1 - i) * p[i] / (d + 1);
-            if (i > 0) q[i] += (1 - r) * i * p[i - 1] / (d + 1);
-        }
-        return q;
-    };
-    auto elevated = [n](vec p) {
-        while (int(p.size()) <= n) {
-            const int d = int(p.size()) - 1;
-            vec q(size_t(d) + 2, 0);
-            for (int i = 0; i <= d + 1; ++i)
-                q[i] = ((i ? i * p[i - 1] : 0) + (i <= d ? (d + 1 - i) * p[i] : 0)) / (d + 1);
-            p = std::move(q);
-        }
-        return p;
-    };
-    auto largest = [](const vec &p) {
-        real a = 0;
-        for (const real v : p) a = std::max(a, std::fabs(v));
-        return a;
-    };
-    // Newton basis w_l = prod_{i < l} (s - c_i), also at degree n.
-    std::vector<vec> w(m), wn(m);
-    for (int l = 0; l <= n; ++l) {
-        w[l] = l ? times_root(w[l - 1], c[l - 1]) : vec{1};
-        wn[l] = elevated(w[l]);
-    }
-    // Bernstein coefficients from the divided differences of level k (entries
-    // from k on; the ones before are zero).
-    auto bernstein = [&](vec f, int k) {
-        for (int q = k; q < n; ++q)
-            for (int j = n; j > q; --j) f[j] = (f[j] - f[j - 1]) / (real(c[j]) - c[j - q - 1]);
-        vec b(m, 0);
-        for (int l = k; l <= n; ++l)
-            for (int i = 0; i <= n; ++i) b[i] += f[l] * wn[l][i];
-        return b;
-    };
-    // What a node's value can do to a Bernstein coefficient.
-    real L = 0;
-    for (int j = 0; j <= n; ++j) {
-        vec e(m, 0);
-        e[j] = 1;
-        const real a = largest(bernstein(std::move(e), 0));
-        t.node_w[j] = double(a);
-        L += a;
-    }
-    // Divided difference j of level k: its relative rounding in both
-    // formulations, and what an error of it does to the coefficients.
-    std::vector<vec> dd(m, vec(m, 0));
-    for (int k = 1; k <= n; ++k)
-        for (int j = k; j <= n; ++j) {
-            vec e(m, 0);
-            e[j] = 1;
-            dd[k][j] = (7 + (real(c[j]) + c[j - k]) / (real(c[j]) - c[j - k])) * largest(bernstein(std::move(e), k));
-        }
-    // Step k of Newton form -> monomials writes the coefficients of
-    // s^(j - k) w_k: four roundings of at most the sum of magnitudes there.
-    std::vector<vec> nm(m, vec(m, 0));
-    for (int k = 0; k < n; ++k) {
-        vec p = w[k];
-        for (int j = k; j < n; ++j) {
-            nm[k][j] = 4 * largest(elevated(p));
-            p = times_root(p, 0);
-        }
-    }
-    const real u = 1.1102230246251565e-16L, slack = 1.05L; // slack: second order and this function's own rounding
-    for (int l = 0; l <= n; ++l) {
-        real g = 0;
-        vec f(m); // w_l at the nodes, then its divided differences level by level (none beyond l)
-        for (int j = 0; j <= n; ++j) {
-            f[j] = 1;
-            for (int i = 0; i < l; ++i) f[j] *= real(c[j]) - c[i];
-        }
-        for (int k = 1; k <= l; ++k)
-            for (int j = n; j >= k; --j) {
-                f[j] = (f[j] - f[j - 1]) / (real(c[j]) - c[j - k]);
-                g += dd[k][j] * std::fabs(f[j]);
-            }
-        vec a(m, 0); // magnitudes of the coefficients that w_l contributes to
-        a[l] = 1;
-        for (int k = n - 1; k >= 0; --k)
-            for (int j = k; j < n; ++j) {
-                a[j] += c[k] * a[j + 1];
-                g += nm[k][j] * a[j];
-            }
-        t.newton[l] = double(slack * u * g);
-    }
-    t.value = double(slack * u * std::sqrt(L) * 78.4);
-    t.square = double(slack * u * 10);
-    t.norm = double(slack * u * u * L * 1537);
-    t.mono = double(slack * u * (6 * n + 24));
-}
-
+static_assert(FILTER_MAX_OP1 == MAX_OP1, "tables for every order");
 // Reciprocal node differences, row k: 1 / (c_j - c_{j-k-1}), j = k + 1 .. n.
 template <int OP1>
 struct filter_consts {
@@ -646,23 +514,11 @@ template <int OP1>
 static filter_consts<OP1> make_filter_consts()
 {
     filter_consts<OP1> f{};
-    const int n = OP1 - 1;
     const cheb_nodes c = make_cheb_nodes(OP1);
+    f.t = make_filter_tables(c.v, OP1);
     int at = 0;
-    for (int k = 0; k < n; ++k)
-        for (int j = k + 1; j <= n; ++j) f.inv_dd[at++] = 1.0 / (c.v[j] - c.v[j - k - 1]);
-    double b = 1.0;
-    for (int i = 0; i <= n; ++i) {
-        f.t.node[i] = c.v[i];
-        f.t.inv_binom[i] = 1.0 / b;
-        b = b * (n - i) / (i + 1);
-    }
-    for (int m = 0; m < OP1 / 2; ++m) {
-        f.t.x[m] = 2.0 * c.v[n - m] - 1.0;
-        f.t.y[m] = f.t.x[m] * f.t.x[m];
-    }
-    filter_range(f.t, n);
-    filter_margins(f.t, n);
+    for (int k = 0; k < OP1 - 1; ++k)
+        for (int j = k + 1; j < OP1; ++j) f.inv_dd[at++] = 1.0 / (c.v[j] - c.v[j - k - 1]);
     return f;
 }
 __host__ __device__ constexpr int filter_row(int op1, int k) { return k * (op1 - 1) - k * (k - 1) / 2; } // start of row k
